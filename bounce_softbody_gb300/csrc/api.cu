@@ -240,10 +240,8 @@ int ensure_precision(b3g_body* b, int prec)
 	bytes += align_up(alo);
 	const size_t xff = prec == kP64 ? 0 : 8 * np * sizeof(float);  // float-float solution for refinement
 	bytes += align_up(xff);
-	// BF16: the flexible outer CG's workspace (7 vectors, inner scalars, outer scalars, partials)
-	const size_t fcg = prec == kPBF ? align_up(7 * 4 * np * vs) + align_up(sizeof(Scalars)) +
-	                                      align_up(sizeof(FcgScalars)) + align_up(2 * kMaxPartials * sizeof(double))
-	                                : 0;
+	// BF16: the inner solve's vectors z, r, d, q
+	const size_t fcg = prec == kPBF ? align_up(4 * 4 * np * vs) : 0;
 	bytes += fcg;
 	char* mem = nullptr;
 	cudaError_t e = cudaMalloc(&mem, bytes);
@@ -271,13 +269,7 @@ int ensure_precision(b3g_body* b, int prec)
 	p += align_up(xff);
 	if (fcg)
 	{
-		for (int k = 0; k < 7; ++k) pb.fcg_vec[k] = p + k * 4 * np * vs;
-		p += align_up(7 * 4 * np * vs);
-		pb.fcg_inner = (Scalars*)p;
-		p += align_up(sizeof(Scalars));
-		pb.fcg = (FcgScalars*)p;
-		p += align_up(sizeof(FcgScalars));
-		pb.fcg_part = (double*)p;
+		for (int k = 0; k < 4; ++k) pb.fcg_vec[k] = p + k * 4 * np * vs;
 	}
 	return B3G_OK;
 }
@@ -648,8 +640,7 @@ int b3g_body_create(b3g_context* ctx, const b3g_body_desc* d, b3g_body** out)
 		D.shapes = C.take<DevShape>(b->nw);
 		shape_dev = C.take<float>(b->nw ? shape_data.size() : 0);
 		D.sc = C.take<Scalars>(1);
-		D.partials = C.take<double>(kMaxPartials);
-		D.team_partials = C.take<double>(kMaxPartials);
+		D.team = C.take<TeamMemory>(1);
 		b->staging = C.take<float>(3 * (size_t)n);
 	};
 	DevBody D{};
@@ -783,10 +774,6 @@ static void release_body_memory(b3g_body* b)
 	if (b->arena) cudaFree(b->arena);
 	if (b->ray_buf) cudaFree(b->ray_buf);
 	if (b->filt) cudaFree(b->filt);
-	for (auto& g : b->chunk_graphs) cudaGraphExecDestroy(g.exec);
-	b->chunk_graphs.clear();
-	for (auto& g : b->fcg_graphs) cudaGraphExecDestroy(g.exec);
-	b->fcg_graphs.clear();
 	for (int k = 0; k < 3; ++k) b->prec[k] = PrecBuffers();
 	b->arena = nullptr;
 	b->ray_buf = nullptr;
@@ -836,43 +823,6 @@ int b3g_body_device_bytes(const b3g_body* b, uint64_t* bytes)
 	return B3G_OK;
 }
 
-// kPcgChunk iterations of the per-op PCG from iteration j0 (a multiple of kPcgChunk, so even):
-// one replay of the chunk's CUDA graph, captured on first use. The kernels decide on the device
-// whether the solve already finished; the host only checks between chunks. A chunk's launches
-// depend on j0 only through which iterations refresh, so a handful of graphs serve every chunk.
-static cudaError_t pcg_chunk(b3g_body* b, const DevBody& D, int prec, int precond, int j0, int refresh,
-                             cudaStream_t st)
-{
-	const unsigned mask = pcg_resid_mask(prec, j0, kPcgChunk, refresh);
-	for (const auto& g : b->chunk_graphs)
-		if (g.prec == prec && g.precond == precond && g.refresh == refresh && g.resid_mask == mask)
-			return cudaGraphLaunch(g.exec, st);
-	op_pcg_prime(D, prec);
-	cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-	cudaError_t e = cudaStreamIsCapturing(st, &cs);
-	if (e == cudaSuccess && cs == cudaStreamCaptureStatusNone) e = cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal);
-	else e = cudaErrorStreamCaptureUnsupported;
-	if (e != cudaSuccess)
-	{
-		// no graph (the stream is captured by someone else, or capture is unavailable): launch
-		// the chunk's kernels one by one
-		cudaGetLastError();
-		e = cudaSuccess;
-		for (int k = 0; k < kPcgChunk && e == cudaSuccess; ++k) e = op_pcg_iteration(D, prec, j0 + k, refresh, st);
-		return e;
-	}
-	for (int k = 0; k < kPcgChunk && e == cudaSuccess; ++k) e = op_pcg_iteration(D, prec, j0 + k, refresh, st);
-	cudaGraph_t graph = nullptr;
-	const cudaError_t ec = cudaStreamEndCapture(st, &graph);
-	if (e == cudaSuccess) e = ec;
-	cudaGraphExec_t exec = nullptr;
-	if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-	if (graph) cudaGraphDestroy(graph);
-	if (e != cudaSuccess) return e;
-	b->chunk_graphs.push_back({prec, precond, refresh, mask, exec});
-	return cudaGraphLaunch(exec, st);
-}
-
 // Inner BF16 PCG iterations per outer iteration of the BF16 mode (B3G_BF16_INNER overrides).
 static int bf16_inner_iterations()
 {
@@ -882,79 +832,6 @@ static int bf16_inner_iterations()
 		return v > 0 ? v : 20;
 	}();
 	return m;
-}
-
-// The BF16 mode's solve: a flexible CG on the FP32 blocks (float-float solution, the true residual
-// refreshed every refresh_period outer iterations) preconditioned by a fixed number of Jacobi-PCG
-// iterations with the BF16 blocks (from z = 0). The matrix is read mostly as BF16: per outer
-// iteration one FP32 product and bf16_inner_iterations() BF16 products. Unlike refining a BF16
-// PCG, this converges when the BF16 rounding of the matrix times its condition number exceeds
-// one: the outer iteration only needs the inner solve to be a fair approximation of A^-1.
-// max_pcg_iterations bounds the outer iterations; the step's PCG statistics count them.
-static cudaError_t run_bf16_fcg(b3g_body* b, const DevBody& D, const b3g_solver_config& cfg, cudaStream_t st)
-{
-	const PrecBuffers& pb = b->prec[kPBF];
-	DevBody Bin = D;
-	Bin.pb = D.r;  // the inner solve's right-hand side is the outer residual
-	Bin.py = pb.fcg_vec[0];
-	Bin.r = pb.fcg_vec[1];
-	Bin.s = pb.fcg_vec[2];
-	Bin.d = pb.fcg_vec[3];
-	Bin.d2 = pb.fcg_vec[4];
-	Bin.q = pb.fcg_vec[5];
-	Bin.xff = nullptr;
-	Bin.sc = pb.fcg_inner;
-	const int m = bf16_inner_iterations();
-	Scalars* hs = b->ctx->h_scalars;
-	// one outer iteration's launches: the inner solve, then the outer direction, product and update
-	auto launch = [&](int k) -> cudaError_t {
-		cudaError_t e = op_fcg_inner_begin(Bin, D.sc, m, 0.0, st);
-		for (int j = 0; j < m && e == cudaSuccess; ++j) e = op_fcg_inner_iteration(Bin, j, st);
-		// p and p_prev alternate between d and d2, q and q_prev between q and the workspace's
-		DevBody Bo = D;
-		if (k & 1) std::swap(Bo.d, Bo.d2);
-		float* qa = (float*)D.q;
-		float* qb = (float*)pb.fcg_vec[6];
-		Bo.q = (k & 1) ? qb : qa;
-		if (e == cudaSuccess) e = op_fcg_outer(Bo, (const float*)Bin.py, (k & 1) ? qa : qb, pb.fcg, pb.fcg_part, k, st);
-		return e;
-	};
-	// ... replayed as a CUDA graph per variant (first, odd, even), captured on first use; launched
-	// directly when the stream is being captured by the caller
-	auto run = [&](int k) -> cudaError_t {
-		const int variant = k == 0 ? 0 : ((k & 1) ? 1 : 2);
-		for (const auto& g : b->fcg_graphs)
-			if (g.variant == variant && g.inner == m && g.precond == D.precond) return cudaGraphLaunch(g.exec, st);
-		op_pcg_prime(Bin, kPBF);
-		op_pcg_prime(D, kP32);
-		cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-		cudaError_t e = cudaStreamIsCapturing(st, &cs);
-		if (e != cudaSuccess || cs != cudaStreamCaptureStatusNone ||
-		    cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal) != cudaSuccess)
-		{
-			cudaGetLastError();
-			return launch(k);
-		}
-		e = launch(k);
-		cudaGraph_t graph = nullptr;
-		const cudaError_t ec = cudaStreamEndCapture(st, &graph);
-		if (e == cudaSuccess) e = ec;
-		cudaGraphExec_t exec = nullptr;
-		if (e == cudaSuccess) e = cudaGraphInstantiate(&exec, graph, 0);
-		if (graph) cudaGraphDestroy(graph);
-		if (e != cudaSuccess) return e;
-		b->fcg_graphs.push_back({variant, m, D.precond, exec});
-		return cudaGraphLaunch(exec, st);
-	};
-	cudaError_t e = cudaSuccess;
-	for (int k = 0; k < (int)cfg.max_pcg_iterations && e == cudaSuccess; ++k)
-	{
-		e = run(k);
-		if (e == cudaSuccess) e = cudaMemcpyAsync(&hs->done, &D.sc->done, sizeof(int), cudaMemcpyDeviceToHost, st);
-		if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-		if (e == cudaSuccess && hs->done) break;
-	}
-	return e;
 }
 
 int b3g_body_step(b3g_body* b, float dt, const b3g_solver_config* cfg_in, b3g_step_stats* stats)
@@ -992,48 +869,41 @@ int b3g_body_step(b3g_body* b, float dt, const b3g_solver_config* cfg_in, b3g_st
 		D.filt = b->filt;
 	}
 	const int newton = (int)std::max<uint32_t>(1u, cfg.force_iterations);
-	e = op_begin(D, st, (int)cfg.max_pcg_iterations, cfg.pcg_tolerance * cfg.pcg_tolerance, (int)cfg.refresh_period,
-	             cfg.newton_tolerance * cfg.newton_tolerance);
-	const int chunk = kPcgChunk;
+	e = cudaSuccess;
 	Scalars* hs = b->ctx->h_scalars;
 	for (int k = 0; k < newton && e == cudaSuccess; ++k)
 	{
 		StepParamsHost P{dt, k == 0 ? 1 : 0};
-		if (k > 0) e = op_newton_begin(D, st);
-		else if (D.filt && e == cudaSuccess) e = op_contact_filter(D, dt, st);
+		if (k == 0 && D.filt) e = op_contact_filter(D, dt, st);
 		if (e == cudaSuccess) e = op_elements(D, P, st);
-		if (e == cudaSuccess) e = op_assemble(D, P, prec, k == 0, st);
-		if (e == cudaSuccess && k > 0) e = op_pcg_init(D, prec, st);
-		// the host first asks whether the solve ended one chunk before the previous step's solve
-		// did: the chunks before that queue back to back (a chunk launched after the end returns
-		// at once from every kernel)
-		const int quiet = std::max(0, b->pcg_chunks_hint - 1);
-		int chunks = 0;
-		if (prec == kPBF && e == cudaSuccess) e = run_bf16_fcg(b, D, cfg, st);
-		for (int it = 0; prec != kPBF && it < (int)cfg.max_pcg_iterations && e == cudaSuccess; it += chunk)
-		{
-			if (it + chunk <= (int)cfg.max_pcg_iterations)
-				e = pcg_chunk(b, D, prec, (int)cfg.preconditioner, it, (int)cfg.refresh_period, st);
-			else
-				for (int j = 0; it + j < (int)cfg.max_pcg_iterations && e == cudaSuccess; ++j)
-					e = op_pcg_iteration(D, prec, it + j, (int)cfg.refresh_period, st);
-			if (e != cudaSuccess) break;
-			if (++chunks <= quiet) continue;
-			e = cudaMemcpyAsync(&hs->done, &D.sc->done, sizeof(int), cudaMemcpyDeviceToHost, st);
-			if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-			if (e == cudaSuccess && hs->done) break;
-		}
-		if (k == 0) b->pcg_chunks_hint = chunks;
+		if (e == cudaSuccess) e = op_assemble(D, P, prec, k > 0 ? kInitNone : kInitTeam, st);
 		if (e != cudaSuccess) break;
-		const bool single = newton == 1;
-		e = op_final(D, P, prec, single ? 1 : 0, st);
-		if (e != cudaSuccess || single) break;
-		e = cudaMemcpyAsync(&hs->newton_done, &D.sc->newton_done, sizeof(int), cudaMemcpyDeviceToHost, st);
-		if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-		if (e == cudaSuccess && (hs->newton_done || k == newton - 1))
+		SolveArgs A;
+		A.tol2 = cfg.pcg_tolerance * cfg.pcg_tolerance;
+		A.newton_tol2 = cfg.newton_tolerance * cfg.newton_tolerance;
+		A.max_iter = (int)cfg.max_pcg_iterations;
+		A.refresh = (int)cfg.refresh_period;
+		A.h = dt;
+		A.newton = k;
+		A.newton_max = newton;
+		A.forces_left = k + 1 < newton ? 1 : 0;
+		A.warm = k > 0 ? 1 : 0;
+		A.smem = 0;
+		if (prec == kPBF)
 		{
-			e = op_post(D, dt, st);
-			break;
+			const PrecBuffers& pb = b->prec[kPBF];
+			const FcgVecs W = {(float*)pb.fcg_vec[0], (float*)pb.fcg_vec[1], (float*)pb.fcg_vec[2], (float*)pb.fcg_vec[3]};
+			e = op_solve_fcg(D, W, A, bf16_inner_iterations(), st);
+		}
+		else
+			e = op_solve(D, A, prec, st);
+		// the launches of Newton iterations past the loop's end do nothing; the host asks now and
+		// then whether it has ended
+		if (e == cudaSuccess && A.forces_left && k % 8 == 7)
+		{
+			e = cudaMemcpyAsync(&hs->newton_done, &D.sc->newton_done, sizeof(int), cudaMemcpyDeviceToHost, st);
+			if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+			if (e == cudaSuccess && hs->newton_done) break;
 		}
 	}
 	if (e != cudaSuccess) return cuda_fail(e, "step");

@@ -76,13 +76,9 @@ struct PrecBuffers
 	void* minv = nullptr;
 	void* alo = nullptr;
 	float* xff = nullptr;  // float-float solution (FP32 and BF16 modes), 8 floats per vertex
-	// BF16 mode of the per-op step (flexible outer CG around inner BF16 PCG solves): the inner
-	// solution z, the inner r s d d2 q, the outer q of the previous iteration (7 vectors, 4-wide),
-	// the inner solve's scalars, the outer's extra scalars and their reduction partials
-	void* fcg_vec[7] = {};
-	Scalars* fcg_inner = nullptr;
-	FcgScalars* fcg = nullptr;
-	double* fcg_part = nullptr;
+	// BF16 mode of the per-op step: the inner solve's z, r, d, q (4-wide), used where the solve's
+	// shared memory has no room for them
+	void* fcg_vec[4] = {};
 };
 
 } // namespace b3g
@@ -110,24 +106,6 @@ struct b3g_body
 	uint32_t ray_cap = 0;
 	// per-vertex constraints of filtered contacts, made on the first step in that mode
 	float4* filt = nullptr;
-	// the per-op PCG's chunks of kPcgChunk iterations, captured into CUDA graphs once per kind:
-	// precision, preconditioner, refresh period and which iterations of the chunk refresh
-	struct ChunkGraph
-	{
-		int prec, precond, refresh;
-		unsigned resid_mask;
-		cudaGraphExec_t exec;
-	};
-	std::vector<ChunkGraph> chunk_graphs;
-	// the BF16 mode's outer iterations captured into CUDA graphs: variant 0 = the first outer
-	// iteration, 1 / 2 = later odd / even ones (buffers alternate), for `inner` inner iterations
-	struct FcgGraph
-	{
-		int variant, inner, precond;
-		cudaGraphExec_t exec;
-	};
-	std::vector<FcgGraph> fcg_graphs;
-	int pcg_chunks_hint = 0;  // chunks the previous step's first solve launched
 };
 
 namespace b3g {

@@ -3,6 +3,7 @@
 #pragma once
 
 #include "internal.h"
+#include "ops.h"
 
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
@@ -1204,10 +1205,10 @@ __device__ __forceinline__ void contact_filter_vertex(const DevBody& B, int i, f
 __device__ __forceinline__ bool filt_on(float4 f) { return f.x != 0.0f || f.y != 0.0f || f.z != 0.0f; }
 
 // The end of row i's assembly once its right-hand side bi and diagonal block are final: pb,
-// the Jacobi preconditioner and, when init_pcg is set, r = pb, s = d = M^-1 r and the zero
-// initial guess; returns r.s (0 without init_pcg).
+// the Jacobi preconditioner and, for init_pcg = kInitAll, r = pb, s = d = M^-1 r and the zero
+// initial guess; returns r.s (0 otherwise). kInitTeam: only s = M^-1 pb.
 template <class TV>
-__device__ __forceinline__ double row_finish(const DevBody& B, int i, float3 bi, const float diag[9], bool init_pcg)
+__device__ __forceinline__ double row_finish(const DevBody& B, int i, float3 bi, const float diag[9], int init_pcg)
 {
 	TV* pb = vp<TV>(B.pb);
 	const TV bv[3] = {(TV)bi.x, (TV)bi.y, (TV)bi.z};
@@ -1256,9 +1257,10 @@ __device__ __forceinline__ double row_finish(const DevBody& B, int i, float3 bi,
 		sv[1] = m3[4] * r1;
 		sv[2] = m3[8] * r2;
 	}
+	vst(vp<TV>(B.s), i, sv);
+	if (init_pcg == kInitTeam) return 0.0;
 	const TV zero[3] = {0, 0, 0};
 	vst(vp<TV>(B.r), i, bv);
-	vst(vp<TV>(B.s), i, sv);
 	vst(vp<TV>(B.d), i, sv);
 	vst(vp<TV>(B.py), i, zero);
 	if (B.xff)
@@ -1280,7 +1282,7 @@ __device__ __forceinline__ double row_finish(const DevBody& B, int i, float3 bi,
 // contact terms), so those parts are compiled out: fewer registers, the same arithmetic.
 template <class TA, class TV, class L = LdPlain, bool FILTER = false, bool TETS = false>
 __device__ __forceinline__ double assemble_row(const DevBody& B, int slice, int lane, const StepParams& P,
-                                               bool init_pcg)
+                                               int init_pcg)
 {
 	const int i = slice * kSlice + lane;
 	if (i >= B.n) return 0.0;
@@ -1903,22 +1905,10 @@ __device__ __forceinline__ void find_new_contacts(const DevBody& B, int i, float
 // v = v + dv, x = x0 + h v + y (sparse_force_solver.cpp:194-200); returns |dv|^2 of the vertex.
 // finish != 0 also ends the step: friction, clearing of external forces and translations, new
 // contacts (body.cpp:572-603), and writes the state instead of the Newton iterate.
-template <class TV, class L = LdPlain, bool FILTER = false>
-__device__ __forceinline__ double final_vertex(const DevBody& B, int i, float h, bool first_newton, bool finish)
+template <class L = LdPlain, bool FILTER = false>
+__device__ __forceinline__ double final_vertex_dv(const DevBody& B, int i, float h, bool first_newton, bool finish,
+                                                  float3 dv)
 {
-	float3 dv;
-	if (B.xff)
-	{
-		float yh[3], yl[3];
-		ff_ld(B.xff, i, yh, yl);
-		dv = f3(yh[0] + yl[0], yh[1] + yl[1], yh[2] + yl[2]);
-	}
-	else
-	{
-		TV y3[3];
-		vld<TV, L>((const TV*)B.py, i, y3);
-		dv = f3((float)y3[0], (float)y3[1], (float)y3[2]);
-	}
 	if (FILTER && first_newton)
 	{
 		// dv = y + z (sparse_force_solver.cpp:187)
@@ -1937,6 +1927,26 @@ __device__ __forceinline__ double final_vertex(const DevBody& B, int i, float h,
 	st3(finish ? B.x : B.xi, i, x);
 	st3(finish ? B.v : B.vi, i, v);
 	return (double)dv.x * dv.x + (double)dv.y * dv.y + (double)dv.z * dv.z;
+}
+
+// the same with dv read from the PCG solution
+template <class TV, class L = LdPlain, bool FILTER = false>
+__device__ __forceinline__ double final_vertex(const DevBody& B, int i, float h, bool first_newton, bool finish)
+{
+	float3 dv;
+	if (B.xff)
+	{
+		float yh[3], yl[3];
+		ff_ld(B.xff, i, yh, yl);
+		dv = f3(yh[0] + yl[0], yh[1] + yl[1], yh[2] + yl[2]);
+	}
+	else
+	{
+		TV y3[3];
+		vld<TV, L>((const TV*)B.py, i, y3);
+		dv = f3((float)y3[0], (float)y3[1], (float)y3[2]);
+	}
+	return final_vertex_dv<L, FILTER>(B, i, h, first_newton, finish, dv);
 }
 
 // finish a multi-Newton step for vertex i: iterate -> state, friction, clearing, new contacts

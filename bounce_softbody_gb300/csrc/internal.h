@@ -39,7 +39,6 @@
 namespace b3g {
 
 constexpr int kSlice = 32;
-constexpr int kPcgChunk = 8;     // per-op PCG iterations between host checks of convergence
 constexpr int kGroup = 4;
 
 B3G_HD size_t block_slot(size_t base, int k, int lane) { return base + 128 * (size_t)(k >> 2) + 4 * lane + (k & 3); }
@@ -69,18 +68,6 @@ struct Scalars
 	int fault;         // a bounded device wait expired (the step's results are not valid)
 	unsigned long long total_iters;  // PCG iterations of every step since creation
 	unsigned long long total_steps;
-};
-
-// Scalars of the flexible outer CG of the BF16 mode (per-op path): z.q_prev, p.r, p.q of this
-// iteration and of the previous one, and the arrival counter of its two-value reductions.
-struct FcgScalars
-{
-	double gamma;      // z . q_prev
-	double rho;        // p . r
-	double pq;         // p . q
-	double pq_prev;    // p_prev . q_prev
-	unsigned counter;
-	int pad;
 };
 
 // One static world shape (b3WorldFixture + b3Shape) on the device. Geometry is in world space
@@ -114,6 +101,19 @@ constexpr int kMeshTriFloats = 28;
 constexpr int kBwFloats = 20;
 constexpr int kMouseFloats = 6;
 constexpr uint32_t kForceStretch = 0, kForceShear = 1;
+
+constexpr int kMaxPartials = 4096;
+constexpr int kTeamMax = 160;   // CTAs of the grid team (solve.cuh), at most
+constexpr int kTeamReplicas = 16;
+
+// Reduction memory of a grid team (solve.cuh)
+struct TeamMemory
+{
+	unsigned arrived;
+	unsigned pad[31];
+	unsigned long long slots[2][kTeamMax];
+	unsigned long long tagged[2][kTeamReplicas][kTeamMax];
+};
 
 // Everything a kernel needs about one body. Passed by value to the per-op kernels and read
 // from a device array by the persistent batch kernel.
@@ -224,13 +224,10 @@ struct DevBody
 	float gravity[3];
 
 	Scalars* sc;
-	double* partials;           // reduction scratch of the per-op kernels (kMaxPartials)
-	double* team_partials;      // reduction scratch of the grid team (persistent kernel)
+	TeamMemory* team;           // reduction memory of the grid team's solve
 	int precond;                // b3g_preconditioner
 	float tet_ratio;            // lambda / mu when every tetrahedron has the same ratio, else -1
 };
-
-constexpr int kMaxPartials = 4096;
 
 // Host-side result of the pattern builder (pattern.cpp).
 struct Pattern

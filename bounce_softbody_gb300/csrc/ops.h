@@ -24,42 +24,46 @@ enum Prec
 	kPBF = 2    // bf16 blocks in the iteration, float blocks for the residual refresh, float vectors
 };
 
+// What the row assembly sets up for the PCG besides pb and the Jacobi: nothing, r = pb, s = d =
+// M^-1 r and the zero initial guess, or only s = M^-1 pb (the grid team's solve sets up its other
+// vectors itself).
+enum { kInitNone = 0, kInitAll = 1, kInitTeam = 2 };
+
 struct StepParamsHost
 {
 	float h;
 	int first_newton;
 };
 
-cudaError_t op_begin(const DevBody& B, cudaStream_t st, int max_it, double tol2, int refresh, double newton_tol2);
-cudaError_t op_newton_begin(const DevBody& B, cudaStream_t st);
 cudaError_t op_elements(const DevBody& B, const StepParamsHost& P, cudaStream_t st);
-cudaError_t op_assemble(const DevBody& B, const StepParamsHost& P, int prec, bool init, cudaStream_t st);
+cudaError_t op_assemble(const DevBody& B, const StepParamsHost& P, int prec, int init, cudaStream_t st);
 // filtered contacts: contact update and per-vertex constraints (B.filt) at the start of a step
 cudaError_t op_contact_filter(const DevBody& B, float h, cudaStream_t st);
-cudaError_t op_pcg_init(const DevBody& B, int prec, cudaStream_t st);
-// iteration j (0-based) of the current solve; refresh = the true-residual refresh period
-cudaError_t op_pcg_iteration(const DevBody& B, int prec, int j, int refresh, cudaStream_t st);
-// Iterations of j that launch the true-residual refresh kernel (bit k: iteration j0 + k) for a
-// chunk of `count` iterations from j0; and the launch geometry of the iteration kernels computed
-// once outside any stream capture.
-unsigned pcg_resid_mask(int prec, int j0, int count, int refresh);
-void op_pcg_prime(const DevBody& B, int prec);
-// BF16 mode of the per-op step: a flexible CG (Notay's FCG with one stored direction) on the FP32
-// blocks whose preconditioner is an inner Jacobi-PCG solve with the BF16 blocks.
-//   Bin: the inner solve's view (pb = the outer residual, py = z, its own r s d d2 q and scalars,
-//        no float-float solution); inner_begin starts it (max_it iterations, tolerance tol2) unless
-//        the outer solve is done (outer_sc), inner_iteration runs iteration j.
-//   Bo:  the outer view of outer iteration k (d = p_prev, d2 = p, q = q of this iteration), z the
-//        inner solution, q_prev the previous iteration's q: p = z - (z.q_prev / p_prev.q_prev)
-//        p_prev, q = A p, alpha = p.r / p.q, then the body step's update and true-residual refresh.
-cudaError_t op_fcg_inner_begin(const DevBody& Bin, const Scalars* outer_sc, int max_it, double tol2, cudaStream_t st);
-cudaError_t op_fcg_inner_iteration(const DevBody& Bin, int j, cudaStream_t st);
-cudaError_t op_fcg_outer(const DevBody& Bo, const float* z, const float* q_prev, FcgScalars* f, double* part, int k,
-                         cudaStream_t st);
-// mode 0: write the Newton iterate (xi, vi); mode 1: write the state and finish the step
-cudaError_t op_final(const DevBody& B, const StepParamsHost& P, int prec, int mode, cudaStream_t st);
-// finish a multi-Newton step: iterate -> state, friction, clear, new contacts
-cudaError_t op_post(const DevBody& B, float h, cudaStream_t st);
+// One PCG solve by the grid team (solve.cuh) and, for newton >= 0, what follows it in Newton
+// iteration `newton` of a step: the final update, or the new iterate and the step's end once the
+// Newton loop is done.
+struct SolveArgs
+{
+	double tol2, newton_tol2;
+	int max_iter, refresh;
+	float h;
+	int newton;        // Newton iteration of a body step; -1: only solve, the solution stays in py
+	int newton_max;    // Newton iterations the step may take
+	int forces_left;   // another Newton iteration may follow this one
+	int warm;          // start from the solution at hand (r = b - A x) instead of zero
+	int smem;          // bytes of shared memory of a CTA (set by op_solve)
+};
+cudaError_t op_solve(const DevBody& B, const SolveArgs& P, int prec, cudaStream_t st);
+// the team's reduction slots cleared before a solve (op_assemble does it for a body step)
+cudaError_t op_solve_clear(const DevBody& B, cudaStream_t st);
+// The BF16 mode's solve (flexible CG on the FP32 blocks around `inner` PCG iterations with the BF16
+// blocks) and what follows it. W: the inner solve's vectors, 4-wide, where shared memory has no
+// room for them.
+struct FcgVecs
+{
+	float *z, *r, *d, *q;
+};
+cudaError_t op_solve_fcg(const DevBody& B, const FcgVecs& W, const SolveArgs& P, int inner, cudaStream_t st);
 // dt <= 0: no solve, only contact bookkeeping and clearing (body.cpp:552-604)
 cudaError_t op_nostep(const DevBody& B, cudaStream_t st);
 // clear a float array on the device

@@ -256,7 +256,7 @@ __device__ __forceinline__ double spmv_lin_rows(const DevBody& B, const TA* A, c
 // default forms inlined in the team kernels keep their register allocation.
 template <class TA, class TV, class LD>
 __device__ __noinline__ double assemble_row_filtered(const DevBody& B, int sl, int lane, const StepParams& sp,
-                                                     bool init)
+                                                     int init)
 {
 	return assemble_row<TA, TV, LD, true>(B, sl, lane, sp, init);
 }
@@ -409,8 +409,8 @@ __device__ double team_assemble(Team<CL>& T, const DevBody& B, const BatchParams
 	pc.tick(kPhElem);
 	double part = 0.0;
 	for (int sl = T.warp(); sl < B.nslices; sl += T.nwarps())
-		part += B.filt ? assemble_row_filtered<TA, TV, LD>(B, sl, lane, sp, k == 0)
-		               : assemble_row<TA, TV, LD>(B, sl, lane, sp, k == 0);
+		part += B.filt ? assemble_row_filtered<TA, TV, LD>(B, sl, lane, sp, k == 0 ? kInitAll : kInitNone)
+		               : assemble_row<TA, TV, LD>(B, sl, lane, sp, k == 0 ? kInitAll : kInitNone);
 	if (k > 0)
 	{
 		const TA* Asp = (sizeof(TA) == sizeof(float) && !bf16) ? (const TA*)B.A32 : (const TA*)B.Alo;
@@ -775,8 +775,8 @@ k_batch_rows(BatchParams P)
 		}
 		__syncwarp();
 		const int sl = (int)(g - __ldg(P.slice_off + b));
-		if (FILT && B.filt) assemble_row_filtered<TA, TV, LdPlain>(B, sl, lane, sp, true);
-		else assemble_row<TA, TV, LdPlain, false, TETS>(B, sl, lane, sp, true);
+		if (FILT && B.filt) assemble_row_filtered<TA, TV, LdPlain>(B, sl, lane, sp, kInitAll);
+		else assemble_row<TA, TV, LdPlain, false, TETS>(B, sl, lane, sp, kInitAll);
 	}
 }
 

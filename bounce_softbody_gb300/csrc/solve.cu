@@ -1,0 +1,111 @@
+// Launch of the grid team's PCG (solve.cuh).
+#include "solve.cuh"
+
+#include <algorithm>
+
+namespace b3g {
+
+namespace {
+
+struct Device
+{
+	int sms = 1, room = 0;  // SMs a team may use, dynamic shared memory of a CTA
+};
+
+const Device& device()
+{
+	static const Device d = [] {
+		Device v;
+		int dev = 0;
+		cudaGetDevice(&dev);
+		cudaDeviceGetAttribute(&v.sms, cudaDevAttrMultiProcessorCount, dev);
+		int smem = 0;
+		cudaDeviceGetAttribute(&smem, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+		v.room = (smem - (int)sizeof(SolveSh) - 128) & ~127;
+		v.sms = std::max(1, std::min(v.sms, kTeamMax));
+		return v;
+	}();
+	return d;
+}
+
+// A CTA takes consecutive slices, one warp each up to 32 warps. At least four slices a CTA: on
+// small bodies fewer CTAs make the sums cheaper than more CTAs make the sweeps (10^3 block, 32
+// slices: 32 / 16 / 8 / 4 CTAs 263 / 265 / 256 / 300 us a step).
+struct Geometry
+{
+	int ctas, threads, smem;
+};
+
+Geometry geometry(const DevBody& B, size_t vec_bytes, size_t slot_bytes)
+{
+	const Device& dv = device();
+	const int per = std::max(4, (B.nslices + dv.sms - 1) / dv.sms);
+	Geometry g;
+	g.ctas = std::max(1, (B.nslices + per - 1) / per);
+	const int slices = (B.nslices + g.ctas - 1) / g.ctas;
+	g.threads = 32 * std::max(1, std::min(slices, kSolveMaxThreads / 32));
+	const size_t want = (size_t)slices * (vec_bytes + (size_t)B.maxw * kSlice * slot_bytes);
+	g.smem = (int)(std::min(want, (size_t)dv.room) & ~(size_t)127);
+	return g;
+}
+
+// A cooperative launch: the CTAs of the team wait for one another, so all have to be resident.
+template <class... Args>
+cudaError_t launch_team(void (*kernel)(Args...), const Geometry& g, cudaStream_t st, Args... args)
+{
+	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, device().room);
+	if (e != cudaSuccess) return e;
+	cudaLaunchConfig_t cfg = {};
+	cfg.gridDim = dim3((unsigned)g.ctas, 1, 1);
+	cfg.blockDim = dim3((unsigned)g.threads, 1, 1);
+	cfg.dynamicSmemBytes = (size_t)g.smem;
+	cfg.stream = st;
+	cudaLaunchAttribute attr[1];
+	attr[0].id = cudaLaunchAttributeCooperative;
+	attr[0].val.cooperative = 1;
+	cfg.attrs = attr;
+	cfg.numAttrs = 1;
+	return cudaLaunchKernelEx(&cfg, kernel, args...);
+}
+
+template <class TA, class TV, bool FF, bool FILTER>
+cudaError_t launch_solve(const DevBody& B, SolveArgs P, cudaStream_t st)
+{
+	const Geometry g = geometry(B, solve_vec_bytes<TV, FF>(), solve_slot_bytes<TA>());
+	P.smem = g.smem;
+	if (g.threads <= 256) return launch_team(k_solve<TA, TV, FF, FILTER, 256>, g, st, B, P);
+	if (g.threads <= 512) return launch_team(k_solve<TA, TV, FF, FILTER, 512>, g, st, B, P);
+	return launch_team(k_solve<TA, TV, FF, FILTER, 1024>, g, st, B, P);
+}
+
+template <bool FILTER>
+cudaError_t launch_fcg(const DevBody& B, const FcgVecs& W, SolveArgs P, int inner, cudaStream_t st)
+{
+	const Geometry g = geometry(B, kFcgVecBytes, solve_slot_bytes<__nv_bfloat16>());
+	P.smem = g.smem;
+	if (g.threads <= 256) return launch_team(k_solve_fcg<FILTER, 256>, g, st, B, W, P, inner);
+	if (g.threads <= 512) return launch_team(k_solve_fcg<FILTER, 512>, g, st, B, W, P, inner);
+	return launch_team(k_solve_fcg<FILTER, 1024>, g, st, B, W, P, inner);
+}
+
+} // namespace
+
+cudaError_t op_solve(const DevBody& B, const SolveArgs& P, int prec, cudaStream_t st)
+{
+	if (prec == kP64)
+		return B.filt ? launch_solve<double, double, false, true>(B, P, st) : launch_solve<double, double, false, false>(B, P, st);
+	if (!B.xff) return launch_solve<float, float, false, false>(B, P, st);
+	return B.filt ? launch_solve<float, float, true, true>(B, P, st) : launch_solve<float, float, true, false>(B, P, st);
+}
+
+cudaError_t op_solve_fcg(const DevBody& B, const FcgVecs& W, const SolveArgs& P, int inner, cudaStream_t st)
+{
+	return B.filt ? launch_fcg<true>(B, W, P, inner, st) : launch_fcg<false>(B, W, P, inner, st);
+}
+
+cudaError_t op_solve_clear(const DevBody& B, cudaStream_t st)
+{
+	return cudaMemsetAsync(B.team, 0, sizeof(TeamMemory), st);
+}
+
+} // namespace b3g

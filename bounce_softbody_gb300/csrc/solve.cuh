@@ -1,0 +1,1152 @@
+// The PCG of one body as one cooperative launch over the whole GPU (the grid team).
+//
+// What bounds it: a body's matrix is a few MB, so an iteration moves it in microseconds; what the
+// earlier launches per iteration paid for was launch latency, a reduction through one counter, and
+// the solver vectors' round trips. Here the whole solve is one launch. A CTA owns a contiguous run
+// of 32-row slices for the launch: their vectors (r, d, q, x, and the scalar Jacobi) stay in shared
+// memory, and so does as much of their matrix as fits; only s, which neighbours gather, goes
+// through global memory (L2). Two team-wide sums per iteration are all that is exchanged:
+//   d.q     after q = A s + beta q, d = s + beta d  (nothing is written that others read: no fence)
+//   r.s     after r -= alpha q, s = M^-1 r          (release / acquire: s becomes visible)
+// and x += alpha d runs while the second sum is on its way.
+//
+// Team sums. One warp of every CTA adds the CTAs' partials up in CTA order, so every thread holds
+// the same bits and takes the same decisions. Measured on one GB300 (us a sum, 4 / 32 / 152 CTAs):
+// * r.s, which publishes s: partials in slots, arrivals counted by one release atomic that one lane
+//   of every CTA polls, then the slots are read: 1.2 / 1.4 / 1.5. Polling the slots themselves
+//   behind a fence instead: 1.1 / 1.7 / 2.2 at best;
+// * d.q, which publishes nothing: the partials carry two bits of the sum's number in their lowest
+//   mantissa bits (4e-16 of the partial), and the slots are polled without any fence or atomic:
+//   0.4 / 0.95 / 1.6. Above 16 CTAs the slots exist 16 times, a replica for every 16th CTA: with
+//   one copy the pollers' traffic on the same lines costs 0.4 / 1.4 / 3.8.
+// Two slot arrays alternate in both kinds: a CTA can only overwrite its slot of sum e with that of
+// sum e + 2 after every CTA has arrived at sum e + 1, and so has read sum e. Polls are bounded; a
+// sum that never completes sets Scalars::fault and ends the launch.
+// FP64 is slow on this GPU: an FP64 instruction occupies the SM's pipe for 16 clocks a warp and its
+// result takes about 100; a division takes about 1000. Measured per iteration of a small body with
+// FP64 trees and divisions: 1500 clocks of the update and 1000 of each sum. So sums are exact integer sums of
+// aligned mantissas (Fixed, error at most that of FP64 additions), comparisons are made on the bits, and
+// alpha and beta of the FP32 modes, which are rounded to float, are divided in float-float.
+//
+// The rows' arithmetic is that of the launches it replaces, in the same order.
+#pragma once
+
+#include "device.cuh"
+#include "ops.h"
+
+namespace b3g {
+
+namespace {
+
+constexpr int kSolveMaxThreads = 1024;
+constexpr int kPollLimit = 1 << 20;           // polls before a warp gives up (about a second)
+constexpr int kTeamWarpSlots = kTeamMax / 32; // slots a lane of the polling warp reads
+
+
+__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v)
+{
+	asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+}
+__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p)
+{
+	unsigned long long v;
+	asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+	return v;
+}
+__device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
+{
+	unsigned v;
+	asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+	return v;
+}
+__device__ __forceinline__ void red_release(unsigned* p)
+{
+	asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
+}
+
+// m 2^e with |m| < 2^58: a float's or a double's value, or a sum of such values to 2^-53 of the
+// largest (the precision of FP64 additions). e >= kNotFinite: not finite.
+struct Fixed
+{
+	long long m;
+	int e;
+};
+constexpr int kNotFinite = 1 << 20, kFixedZero = -(1 << 20);
+
+__device__ __forceinline__ Fixed to_fixed(float t)
+{
+	const unsigned u = __float_as_uint(t);
+	const int e = (int)((u >> 23) & 0xffu);
+	const long long m = (long long)((u & 0x7fffffu) | (e > 0 ? 0x800000u : 0u)) << 34;
+	Fixed f;
+	f.m = (u >> 31) ? -m : m;
+	f.e = e == 0xff ? kNotFinite : (m == 0 ? kFixedZero : max(e, 1) - 184);
+	return f;
+}
+__device__ __forceinline__ Fixed to_fixed(double t)
+{
+	const unsigned long long u = (unsigned long long)__double_as_longlong(t);
+	const int e = (int)((u >> 52) & 0x7ffu);
+	const long long m = (long long)((u & 0xfffffffffffffull) | (e > 0 ? 0x10000000000000ull : 0ull)) << 5;
+	Fixed f;
+	f.m = (u >> 63) ? -m : m;
+	f.e = e == 0x7ff ? kNotFinite : (m == 0 ? kFixedZero : max(e, 1) - 1080);
+	return f;
+}
+// back below 2^58
+__device__ __forceinline__ Fixed fixed_norm(long long m, int e)
+{
+	const int sh = max(0, 6 - __clzll(m < 0 ? -m : m));
+	Fixed f;
+	f.m = m >> sh;
+	f.e = m == 0 && e < kNotFinite ? kFixedZero : e + sh;
+	return f;
+}
+__device__ __forceinline__ Fixed fixed_add(Fixed a, Fixed b)
+{
+	const int e = max(a.e, b.e);
+	return fixed_norm((a.m >> min(e - a.e, 63)) + (b.m >> min(e - b.e, 63)), e);
+}
+// the 32 lanes' sum, in all lanes: aligned to the largest exponent, in limbs of 20 bits whose sums
+// fit 32 bits
+__device__ __forceinline__ Fixed fixed_warp_sum(Fixed a)
+{
+	const int e = __reduce_max_sync(0xffffffffu, a.e);
+	const long long q = a.m >> min(e - a.e, 63);
+	const int l0 = (int)__reduce_add_sync(0xffffffffu, (unsigned)(q & 0xfffff));
+	const int l1 = (int)__reduce_add_sync(0xffffffffu, (unsigned)((q >> 20) & 0xfffff));
+	const int l2 = __reduce_add_sync(0xffffffffu, (int)(q >> 40));
+	return fixed_norm((long long)l0 + ((long long)l1 << 20) + ((long long)l2 << 40), e);
+}
+// the nearest double towards zero
+__device__ __forceinline__ double fixed_value(Fixed a)
+{
+	if (a.e >= kNotFinite) return __longlong_as_double(0x7ff8000000000000ll);
+	const unsigned long long u = (unsigned long long)(a.m < 0 ? -a.m : a.m);
+	const int lead = 63 - __clzll((long long)u);  // u = 1.xxx 2^lead
+	const int ex = a.e + lead + 1023;
+	if (u == 0 || ex <= 0) return 0.0;
+	if (ex >= 0x7ff) return __longlong_as_double(0x7ff8000000000000ll);
+	const unsigned long long frac = (lead >= 52 ? u >> (lead - 52) : u << (52 - lead)) & 0xfffffffffffffull;
+	return __longlong_as_double((long long)((a.m < 0 ? 1ull << 63 : 0ull) | ((unsigned long long)ex << 52) | frac));
+}
+
+// Comparisons on the bits of doubles (an FP64 comparison waits for the FP64 pipe)
+__device__ __forceinline__ bool bits_finite(double x) { return ((__double_as_longlong(x) >> 52) & 0x7ff) != 0x7ff; }
+__device__ __forceinline__ bool bits_positive(double x) { return __double_as_longlong(x) > 0; }
+// x <= y for finite x and y >= 0
+__device__ __forceinline__ bool bits_at_most(double x, double y) { return __double_as_longlong(x) <= __double_as_longlong(y); }
+
+// a / b rounded to the vector type. For float, the mantissas are split into two floats each and
+// divided in double-single arithmetic (Dekker, A floating-point technique for extending the
+// available precision, 1971: quotient estimate and one correction from the remainder), good to
+// about 2^-44 before the rounding to 24 bits.
+__device__ __forceinline__ double quotient(double a, double b, double) { return a / b; }
+__device__ __forceinline__ float quotient(double a, double b, float)
+{
+	const unsigned long long ua = (unsigned long long)__double_as_longlong(a), ub = (unsigned long long)__double_as_longlong(b);
+	const int ea = (int)((ua >> 52) & 0x7ff), eb = (int)((ub >> 52) & 0x7ff);
+	if (ea == 0 || eb == 0 || ea == 0x7ff || eb == 0x7ff) return (float)(a / b);
+	// mantissas in [1, 2): 23 fraction bits in the high float, 29 in the low one
+	const float ah = __uint_as_float(0x3f800000u | (unsigned)((ua >> 29) & 0x7fffffu));
+	const float bh = __uint_as_float(0x3f800000u | (unsigned)((ub >> 29) & 0x7fffffu));
+	const float al = (float)(unsigned)(ua & 0x1fffffffu) * 0x1p-52f, bl = (float)(unsigned)(ub & 0x1fffffffu) * 0x1p-52f;
+	const float inv = __fdividef(1.0f, bh);
+	const float q0 = ah * inv;
+	const float rem = fmaf(-q0, bh, ah) + fmaf(-q0, bl, al);
+	const float q = fmaf(rem, inv, q0);
+	return scalbnf(((ua ^ ub) >> 63) ? -q : q, ea - eb);
+}
+
+// One row's term of a dot product in the vector type (dot3 widens it)
+template <class TV>
+__device__ __forceinline__ TV term3(const TV a[3], const TV b[3])
+{
+	return a[0] * b[0] + a[1] * b[1] + a[2] * b[2];
+}
+
+struct SolveSh
+{
+	Fixed w[2][32];
+	double total, ratio;
+	int ok;
+};
+
+// The reduction memory of a team (cleared before the launch): an arrival counter, slots of the
+// sums that publish data, and the replicated slots of the others.
+template <class TV>
+struct GridTeam
+{
+	SolveSh* sh;
+	TeamMemory* mem;
+	int ctas, rank;
+	int replicas;
+	unsigned published, plain;  // sums of each kind so far
+	int ok;
+	TV ratio;
+
+	__device__ __forceinline__ GridTeam(SolveSh* s, TeamMemory* m)
+	    : sh(s), mem(m), ctas(gridDim.x), rank(blockIdx.x), replicas(gridDim.x > 16 ? kTeamReplicas : 1), published(0),
+	      plain(0), ok(1), ratio((TV)0)
+	{
+	}
+
+	// This warp's value v (the same in all lanes) summed over the team. `between` runs after this
+	// CTA's partial is on its way; ratio(total) is evaluated once per CTA and left in `ratio`.
+	// VISIBLE: what the team's threads wrote before the sum may be read by all of them after it.
+	template <bool VISIBLE, class F, class R>
+	__device__ __forceinline__ double sum(Fixed v, F between, R ratio_of)
+	{
+		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
+		const int buf = (published + plain) & 1;
+		if (nw > 1)
+		{
+			if (lane == 0) sh->w[buf][warp] = v;
+			__syncthreads();
+		}
+		else
+			__syncwarp();
+		unsigned long long* mine = nullptr;
+		unsigned long long tag = 0;
+		if (warp == 0)
+		{
+			if (nw > 1)
+			{
+				Fixed z;
+				z.m = 0;
+				z.e = kFixedZero;
+				v = fixed_warp_sum(lane < nw ? sh->w[buf][lane] : z);
+			}
+			const unsigned long long bits = (unsigned long long)__double_as_longlong(fixed_value(v));
+			if (VISIBLE)
+			{
+				mine = mem->slots[published & 1];
+				if (lane == 0)
+				{
+					st_relaxed(mine + rank, bits);
+					red_release(&mem->arrived);
+				}
+			}
+			else
+			{
+				tag = (unsigned long long)(((plain >> 1) + 1) & 3);
+				unsigned long long(*all)[kTeamMax] = mem->tagged[plain & 1];
+				mine = all[rank & (replicas - 1)];
+				if (lane < replicas) st_relaxed(all[lane] + rank, (bits & ~3ull) | tag);
+			}
+		}
+		between();
+		if (warp == 0)
+		{
+			unsigned long long u[kTeamWarpSlots];
+			int polls = 0;
+			bool there = true;
+			if (VISIBLE)
+			{
+				const unsigned want = (published + 1) * (unsigned)ctas;
+				// every lane polls, so that each lane's slot reads follow its own acquire
+				while (ld_acquire(&mem->arrived) < want)
+					if (++polls > kPollLimit)
+					{
+						there = false;
+						break;
+					}
+				there = __all_sync(0xffffffffu, there) != 0;
+#pragma unroll
+				for (int q = 0; q < kTeamWarpSlots; ++q) u[q] = lane + 32 * q < ctas ? ld_relaxed(mine + lane + 32 * q) : 0ull;
+			}
+			else
+				for (;;)
+				{
+					there = true;
+#pragma unroll
+					for (int q = 0; q < kTeamWarpSlots; ++q)
+					{
+						u[q] = lane + 32 * q < ctas ? ld_relaxed(mine + lane + 32 * q) : tag;
+						there = there && (u[q] & 3ull) == tag;
+					}
+					there = __all_sync(0xffffffffu, there) != 0;
+					if (there || ++polls > kPollLimit) break;
+				}
+			Fixed t = to_fixed(__longlong_as_double((long long)(VISIBLE ? u[0] : u[0] & ~3ull)));
+#pragma unroll
+			for (int q = 1; q < kTeamWarpSlots; ++q)
+				if (32 * q < ctas) t = fixed_add(t, to_fixed(__longlong_as_double((long long)(VISIBLE ? u[q] : u[q] & ~3ull))));
+			const double total = fixed_value(fixed_warp_sum(t));
+			const TV r = ratio_of(total);
+			if (lane == 0)
+			{
+				sh->total = total;
+				*(TV*)&sh->ratio = r;
+				sh->ok = there ? 1 : 0;
+			}
+		}
+		if (VISIBLE) ++published;
+		else ++plain;
+		__syncthreads();
+		ok = sh->ok;
+		ratio = *(const TV*)&sh->ratio;
+		return sh->total;
+	}
+	template <bool VISIBLE>
+	__device__ __forceinline__ double sum(Fixed v)
+	{
+		return sum<VISIBLE>(v, [] {}, [](double) { return (TV)0; });
+	}
+	// execution and visibility only
+	__device__ __forceinline__ void publish()
+	{
+		Fixed z;
+		z.m = 0;
+		z.e = kFixedZero;
+		sum<true>(z);
+	}
+};
+
+// Where a slice's matrix comes from: shared memory (a chunk of nine planes and the column ids of
+// its w x 32 slots) or global memory with an L2 policy.
+template <class TA>
+struct SmemMat
+{
+	const unsigned char* chunk;
+	int slots;
+	__device__ __forceinline__ int4 cols(int off) const { return *(const int4*)(chunk + (size_t)9 * slots * sizeof(TA) + 4 * (size_t)off); }
+	__device__ __forceinline__ void plane(int p, int off, typename Acc<TA>::type o[4]) const
+	{
+		load4<TA, LdPlain>((const TA*)chunk + (size_t)p * slots + off, o);
+	}
+};
+template <class TA>
+struct GlobalMat
+{
+	const TA* A;
+	const int* col;
+	size_t ns;
+	size_t base;
+	unsigned long long pol;
+	__device__ __forceinline__ int4 cols(int off) const { return hinted_cols<MatNC>(col + base + off, pol); }
+	__device__ __forceinline__ void plane(int p, int off, typename Acc<TA>::type o[4]) const
+	{
+		hinted_load4<MatNC>(A + p * ns + base + off, o, pol);
+	}
+};
+
+// o = (A s)_i and own = s_i (the diagonal block leads every row); the products are summed in slot
+// order, as spmv_row sums them. DEPTH groups of four blocks have their columns' s in flight at a
+// time: the gathers go to L2, and a thread that waits for them group by group pays that trip four
+// times a row.
+template <class TA, class TV, int DEPTH, class M>
+__device__ __forceinline__ void team_spmv_row(const M& m, int w, int lane, const TV* s, TV o[3], TV own[3])
+{
+	typedef typename Acc<TA>::type AT;
+	AT o0 = 0, o1 = 0, o2 = 0;
+	for (int k0 = 0; k0 < w; k0 += DEPTH * kGroup)
+	{
+		TV xv[DEPTH][4][3];
+#pragma unroll
+		for (int g = 0; g < DEPTH; ++g)
+			if (g == 0 || k0 + g * kGroup < w)
+			{
+				const int4 jj = m.cols(32 * (k0 + g * kGroup) + 4 * lane);
+				vld<TV, LdCG>(s, jj.x, xv[g][0]);
+				vld<TV, LdCG>(s, jj.y, xv[g][1]);
+				vld<TV, LdCG>(s, jj.z, xv[g][2]);
+				vld<TV, LdCG>(s, jj.w, xv[g][3]);
+			}
+		if (k0 == 0)
+		{
+#pragma unroll
+			for (int c = 0; c < 3; ++c) own[c] = xv[0][0][c];
+		}
+#pragma unroll
+		for (int g = 0; g < DEPTH; ++g)
+			if (g == 0 || k0 + g * kGroup < w)
+			{
+				AT a[9][4];
+#pragma unroll
+				for (int p = 0; p < 9; ++p) m.plane(p, 32 * (k0 + g * kGroup) + 4 * lane, a[p]);
+#pragma unroll
+				for (int u = 0; u < 4; ++u)
+				{
+					const AT x0 = (AT)xv[g][u][0], x1 = (AT)xv[g][u][1], x2 = (AT)xv[g][u][2];
+					o0 += a[0][u] * x0 + a[1][u] * x1 + a[2][u] * x2;
+					o1 += a[3][u] * x0 + a[4][u] * x1 + a[5][u] * x2;
+					o2 += a[6][u] * x0 + a[7][u] * x1 + a[8][u] * x2;
+				}
+			}
+	}
+	o[0] = (TV)o0;
+	o[1] = (TV)o1;
+	o[2] = (TV)o2;
+}
+
+// (A x)_i in float-float from the float-float x (spmv_row_ff), x read through L2
+template <class M>
+__device__ __forceinline__ void team_spmv_row_ff(const M& m, int w, int lane, const float* xff, float ohi[3], float olo[3])
+{
+	float h0 = 0, h1 = 0, h2 = 0, l0 = 0, l1 = 0, l2 = 0;
+	for (int k = 0; k < w; k += kGroup)
+	{
+		const int off = 32 * k + 4 * lane;
+		const int4 jj = m.cols(off);
+		float a[9][4];
+#pragma unroll
+		for (int p = 0; p < 9; ++p) m.plane(p, off, a[p]);
+		const int js[4] = {jj.x, jj.y, jj.z, jj.w};
+#pragma unroll
+		for (int u = 0; u < 4; ++u)
+		{
+			float xh[3], xl[3];
+			vld<float, LdCG>(xff, 2 * js[u], xh);
+			vld<float, LdCG>(xff, 2 * js[u] + 1, xl);
+#pragma unroll
+			for (int c = 0; c < 3; ++c)
+			{
+				const float a0 = a[3 * 0 + c][u], a1 = a[3 * 1 + c][u], a2 = a[3 * 2 + c][u];
+				float p = __fmul_rn(a0, xh[c]);
+				ff_add(h0, l0, p, fmaf(a0, xh[c], -p) + a0 * xl[c]);
+				p = __fmul_rn(a1, xh[c]);
+				ff_add(h1, l1, p, fmaf(a1, xh[c], -p) + a1 * xl[c]);
+				p = __fmul_rn(a2, xh[c]);
+				ff_add(h2, l2, p, fmaf(a2, xh[c], -p) + a2 * xl[c]);
+			}
+		}
+	}
+	ohi[0] = h0; ohi[1] = h1; ohi[2] = h2;
+	olo[0] = l0; olo[1] = l1; olo[2] = l2;
+}
+
+// Bytes of shared memory per slot of the matrix, and per slice of the row-local vectors: r, d, q
+// and the scalar Jacobi (4-wide), x (4-wide, or 8 floats in float-float).
+template <class TA>
+__host__ __device__ constexpr int solve_slot_bytes() { return 9 * (int)sizeof(TA) + 4; }
+template <class TV, bool FF>
+__host__ __device__ constexpr int solve_vec_bytes() { return 32 * (4 * 4 + (FF ? 8 : 4)) * (int)sizeof(TV); }
+// the BF16 mode's: r, q, p, the Jacobi and x of the outer iteration, r, d, q and z of the inner one
+constexpr int kFcgVecBytes = 32 * (8 * 4 + 8) * (int)sizeof(float);
+
+// One lane's row vectors in shared memory or in the body's arrays.
+template <class TV, bool FF>
+struct RowVecs
+{
+	TV *r, *d, *q, *m, *x;
+	__device__ __forceinline__ RowVecs(const DevBody& B, unsigned char* vec, int j, int vec_slices, int lane, int i)
+	{
+		if (j < vec_slices)
+		{
+			TV* p = (TV*)(vec + (size_t)j * solve_vec_bytes<TV, FF>());
+			r = p + 4 * lane;
+			d = p + 128 + 4 * lane;
+			q = p + 256 + 4 * lane;
+			m = p + 384 + 4 * lane;
+			x = p + 512 + (FF ? 8 : 4) * lane;
+		}
+		else
+		{
+			r = (TV*)B.r + 4 * (size_t)i;
+			d = (TV*)B.d + 4 * (size_t)i;
+			q = (TV*)B.q + 4 * (size_t)i;
+			m = (TV*)B.Minv + 4 * (size_t)i;
+			x = FF ? (TV*)B.xff + 8 * (size_t)i : (TV*)B.py + 4 * (size_t)i;
+		}
+	}
+};
+
+struct FcgRowVecs
+{
+	float *r, *q, *p, *m, *x, *ri, *di, *qi, *z;
+	__device__ __forceinline__ FcgRowVecs(const DevBody& B, const FcgVecs& W, unsigned char* vec, int j, int vec_slices,
+	                                      int lane, int i)
+	{
+		if (j < vec_slices)
+		{
+			float* b = (float*)(vec + (size_t)j * kFcgVecBytes) + 4 * lane;
+			r = b;
+			q = b + 128;
+			p = b + 256;
+			m = b + 384;
+			ri = b + 512;
+			di = b + 640;
+			qi = b + 768;
+			z = b + 896;
+			x = b + 1024 + 4 * lane;
+		}
+		else
+		{
+			const size_t o = 4 * (size_t)i;
+			r = (float*)B.r + o;
+			q = (float*)B.q + o;
+			p = (float*)B.d + o;
+			m = (float*)B.Minv + o;
+			ri = W.r + o;
+			di = W.d + o;
+			qi = W.q + o;
+			z = W.z + o;
+			x = B.xff + 2 * o;
+		}
+	}
+};
+
+// The slices a CTA owns, which of them keep their vectors and their matrix (of storage type TA)
+// in shared memory: vectors first, since every iteration reads and writes them, then matrices.
+template <class TA>
+struct OwnSlices
+{
+	const DevBody& B;
+	const TA* A;
+	int s0, ns, base0, vec_slices, mat_slices;
+	unsigned char *vec, *mat;
+	unsigned long long pol;
+
+	__device__ __forceinline__ OwnSlices(const DevBody& body, const TA* a, unsigned char* smem, int room, int vecb)
+	    : B(body), A(a)
+	{
+		s0 = (int)((long long)blockIdx.x * B.nslices / gridDim.x);
+		ns = (int)((long long)(blockIdx.x + 1) * B.nslices / gridDim.x) - s0;
+		vec_slices = min(ns, room / vecb);
+		vec = smem;
+		mat = smem + (size_t)vec_slices * vecb;
+		base0 = B.slice_ptr[s0];
+		mat_slices = 0;
+		pol = evict_first_policy();
+		if (vec_slices < ns) return;
+		const int cap = (room - vec_slices * vecb) / solve_slot_bytes<TA>();
+		int lo = 0, hi = ns;
+		while (lo < hi)
+		{
+			const int mid = (lo + hi + 1) >> 1;
+			if (B.slice_ptr[s0 + mid] - base0 <= cap) lo = mid;
+			else hi = mid - 1;
+		}
+		mat_slices = lo;
+	}
+	// the cached matrices, each copied by the warp that will read it
+	__device__ __forceinline__ void load() const
+	{
+		const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+		for (int j = threadIdx.x >> 5; j < mat_slices; j += nw)
+		{
+			const int base = B.slice_ptr[s0 + j], slots = B.slice_ptr[s0 + j + 1] - base;
+			unsigned char* c = mat + (size_t)(base - base0) * solve_slot_bytes<TA>();
+			constexpr int kPer = 16 / (int)sizeof(TA);
+			for (int p = 0; p < 9; ++p)
+				for (int k = lane; k < slots / kPer; k += 32)
+					((uint4*)c)[(size_t)p * (slots / kPer) + k] = mat_ld16<MatNC>(A + (size_t)p * B.nslots + base + k * kPer, pol);
+			uint4* cc = (uint4*)(c + (size_t)9 * slots * sizeof(TA));
+			for (int k = lane; k < slots / 4; k += 32) cc[k] = mat_ld16<MatNC>(B.col + base + 4 * k, pol);
+		}
+		__syncwarp();
+	}
+	// f(local slice j, row i) for the rows of this warp's slices
+	template <class F>
+	__device__ __forceinline__ void rows(F f) const
+	{
+		const int nw = blockDim.x >> 5;
+		for (int j = threadIdx.x >> 5; j < ns; j += nw)
+		{
+			const int i = (s0 + j) * kSlice + (threadIdx.x & 31);
+			if (i < B.n) f(j, i);
+		}
+	}
+	// the sum of f(j, i), a term of type T per row, over this warp's rows; all lanes return it
+	template <class T, class F>
+	__device__ __forceinline__ Fixed row_sum(F f) const
+	{
+		const int nw = blockDim.x >> 5;
+		Fixed s;
+		s.m = 0;
+		s.e = kFixedZero;
+		for (int j = threadIdx.x >> 5; j < ns; j += nw)
+		{
+			const int i = (s0 + j) * kSlice + (threadIdx.x & 31);
+			T t = (T)0;
+			if (i < B.n) t = f(j, i);
+			const Fixed w = fixed_warp_sum(to_fixed(t));
+			s = j < nw ? w : fixed_add(s, w);
+		}
+		return s;
+	}
+	// f(matrix of local slice j, its width)
+	template <class F>
+	__device__ __forceinline__ void matrix(int j, F f) const
+	{
+		const int base = B.slice_ptr[s0 + j];
+		const int slots = B.slice_ptr[s0 + j + 1] - base;
+		if (j < mat_slices) f(SmemMat<TA>{mat + (size_t)(base - base0) * solve_slot_bytes<TA>(), slots}, slots / kSlice);
+		else f(GlobalMat<TA>{A, B.col, (size_t)B.nslots, (size_t)base, pol}, slots / kSlice);
+	}
+};
+
+template <class TV>
+__device__ __forceinline__ void row_precond(const DevBody& B, const TV* m, int i, const TV r[3], TV s[3])
+{
+	if (B.precond == B3G_PRECOND_BLOCK_JACOBI)
+	{
+		precond_row<TV>(B, i, r, s);
+		return;
+	}
+	TV mm[3];
+	vld<TV, LdPlain>(m, 0, mm);
+#pragma unroll
+	for (int c = 0; c < 3; ++c) s[c] = mm[c] * r[c];
+}
+
+template <class TV, bool FF>
+__device__ __forceinline__ void row_x_update(TV* x, const TV* dp, TV alpha)
+{
+	TV d[3];
+	vld<TV, LdPlain>(dp, 0, d);
+	if constexpr (FF)
+	{
+		// refinement: the solution accumulates in float-float (the product alpha d and its
+		// rounding error are both added)
+		float xh[3], xl[3];
+		ff_ld(x, 0, xh, xl);
+#pragma unroll
+		for (int c = 0; c < 3; ++c)
+		{
+			const float p = __fmul_rn(alpha, d[c]);
+			ff_add(xh[c], xl[c], p, fmaf(alpha, d[c], -p));
+		}
+		ff_st(x, 0, xh, xl);
+	}
+	else
+	{
+		TV xx[3];
+		vld<TV, LdPlain>(x, 0, xx);
+#pragma unroll
+		for (int c = 0; c < 3; ++c) xx[c] += alpha * d[c];
+		vst(x, 0, xx);
+	}
+}
+
+// The row's solution as the velocity change dv
+template <class TV, bool FF>
+__device__ __forceinline__ float3 row_dv(const TV* x)
+{
+	if constexpr (FF)
+	{
+		float yh[3], yl[3];
+		ff_ld(x, 0, yh, yl);
+		return f3(yh[0] + yl[0], yh[1] + yl[1], yh[2] + yl[2]);
+	}
+	else
+	{
+		TV y[3];
+		vld<TV, LdPlain>(x, 0, y);
+		return f3((float)y[0], (float)y[1], (float)y[2]);
+	}
+}
+
+struct SolveEnd
+{
+	int status, iter;
+	double delta, delta0;
+};
+
+// What follows a solve: in a body step the final update (sparse_force_solver.cpp:194-223), which
+// with a single Newton iteration also ends the step, or else the Newton loop's exit test and, when
+// it ends, the step's end; then the statistics. rows(f) calls f(row i, dv) for this warp's rows.
+template <bool FILTER, class G, class R>
+__device__ __forceinline__ void team_end(G& T, const DevBody& B, const SolveArgs& P, const SolveEnd& S, R rows)
+{
+	Scalars* sc = B.sc;
+	const bool lead = T.rank == 0 && threadIdx.x == 0;
+	if (P.newton >= 0)
+	{
+		bool finish = P.newton_max == 1;
+		double part = 0.0;
+		rows([&](int i, float3 dv) { part += final_vertex_dv<LdPlain, FILTER>(B, i, P.h, P.newton == 0, finish, dv); });
+		const double err = T.template sum<false>(fixed_warp_sum(to_fixed(part)));
+		const double err0 = P.newton == 0 ? err : sc->newton_err0;
+		const bool ndone = P.newton == 0 ? err <= P.newton_tol2 : err <= P.newton_tol2 * err0;
+		if (!finish && (ndone || !P.forces_left))
+		{
+			finish = true;
+			rows([&](int i, float3) { post_vertex<LdPlain>(B, i, P.h); });
+		}
+		if (lead)
+		{
+			sc->newton_err = err;
+			sc->newton_err0 = err0;
+			sc->min_it = P.newton == 0 ? S.iter : min(sc->min_it, S.iter);
+			sc->max_it = P.newton == 0 ? S.iter : max(sc->max_it, S.iter);
+			sc->newton_iter = P.newton + 1;
+			sc->total_iters += (unsigned long long)S.iter;
+			if (finish) sc->total_steps += 1ull;
+			sc->newton_done = finish ? 1 : 0;
+		}
+	}
+	if (lead)
+	{
+		sc->iter = S.iter;
+		sc->delta = S.delta;
+		sc->delta0 = S.delta0;
+		sc->status = S.status;
+		sc->done = 1;
+	}
+	if (!T.ok && threadIdx.x == 0) sc->fault = 1;
+}
+
+// A sum that never completed: the step's results are not valid (DEVICE_TIMEOUT)
+__device__ __forceinline__ void team_fault(const DevBody& B)
+{
+	B.sc->fault = 1;
+	B.sc->newton_done = 1;
+}
+
+// sparse_solver.cpp:57-73: whether a solve is over before its first iteration
+__device__ __forceinline__ bool solve_over(double delta0, double tol2, int max_iter, int& status)
+{
+	status = B3G_SOLVE_CONVERGED;
+	if (!isfinite(delta0)) status = B3G_SOLVE_NONFINITE;
+	else if (delta0 <= tol2 * delta0) status = B3G_SOLVE_CONVERGED;
+	else if (max_iter <= 0) status = B3G_SOLVE_MAX_ITERATIONS;
+	else return false;
+	return true;
+}
+
+template <class TA, class TV, bool FF, bool FILTER, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
+{
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ SolveSh sh;
+	if (P.newton > 0 && B.sc->newton_done) return;
+	typedef RowVecs<TV, FF> Row;
+	constexpr int kDepth = THREADS <= 256 ? (sizeof(TV) == 8 ? 2 : 4) : (THREADS <= 512 && sizeof(TV) == 4 ? 2 : 1);
+	const int lane = threadIdx.x & 31;
+	GridTeam<TV> T(&sh, B.team);
+	const OwnSlices<TA> O(B, sizeof(TA) == sizeof(float) ? (const TA*)B.A32 : (const TA*)B.Alo, smem, P.smem,
+	                      solve_vec_bytes<TV, FF>());
+	const TV* sv = (const TV*)B.s;
+	if (blockIdx.x == 0 && threadIdx.x == 0 && P.newton <= 0) B.sc->fault = 0;
+	auto row = [&](int j, int i) { return Row(B, O.vec, j, O.vec_slices, lane, i); };
+
+	// r = b - A x and s = M^-1 r with x in global memory; this warp's part of r.s
+	auto residual = [&]() -> Fixed {
+		return O.template row_sum<TV>([&](int j, int i) {
+			const Row v = row(j, i);
+			TV b[3], rr[3], ss[3];
+			vld<TV, LdPlain>((const TV*)B.pb, i, b);
+			O.matrix(j, [&](const auto& m, int w) {
+				if constexpr (FF)
+				{
+					float qh[3], ql[3];
+					team_spmv_row_ff(m, w, lane, B.xff, qh, ql);
+#pragma unroll
+					for (int c = 0; c < 3; ++c) rr[c] = ff_residual(b[c], qh[c], ql[c]);
+				}
+				else
+				{
+					TV q[3], own[3];
+					team_spmv_row<TA, TV, kDepth>(m, w, lane, (const TV*)B.py, q, own);
+#pragma unroll
+					for (int c = 0; c < 3; ++c) rr[c] = b[c] - q[c];
+				}
+			});
+			row_precond<TV>(B, v.m, i, rr, ss);
+			vst(v.r, 0, rr);
+			vst((TV*)B.s, i, ss);
+			return term3(rr, ss);
+		});
+	};
+	// the rows' x to global memory, where a refresh gathers it
+	auto publish_x = [&] {
+		O.rows([&](int j, int i) {
+			if (j >= O.vec_slices) return;
+			const Row v = row(j, i);
+			if constexpr (FF)
+			{
+				float xh[3], xl[3];
+				ff_ld(v.x, 0, xh, xl);
+				ff_st(B.xff, i, xh, xl);
+			}
+			else
+			{
+				TV x[3];
+				vld<TV, LdPlain>(v.x, 0, x);
+				vst((TV*)B.py, i, x);
+			}
+		});
+	};
+	auto update_x = [&](TV alpha) {
+		O.rows([&](int j, int i) {
+			const Row v = row(j, i);
+			row_x_update<TV, FF>(v.x, v.d, alpha);
+		});
+	};
+
+	O.load();
+	// the rows' vectors: the assembly left s = M^-1 b for a start from x = 0 (r = b); a warm start
+	// takes x as it is
+	Fixed part = O.template row_sum<TV>([&](int j, int i) {
+		const Row v = row(j, i);
+		TV t[3];
+		if (j < O.vec_slices && B.precond != B3G_PRECOND_BLOCK_JACOBI)
+		{
+			vld<TV, LdPlain>((const TV*)B.Minv, i, t);
+			vst(v.m, 0, t);
+		}
+		if (P.warm)
+		{
+			if (j >= O.vec_slices) return (TV)0;
+			if constexpr (FF)
+			{
+				float xh[3], xl[3];
+				ff_ld(B.xff, i, xh, xl);
+				ff_st(v.x, 0, xh, xl);
+			}
+			else
+			{
+				vld<TV, LdPlain>((const TV*)B.py, i, t);
+				vst(v.x, 0, t);
+			}
+			return (TV)0;
+		}
+		const TV zero[3] = {0, 0, 0};
+		TV ss[3];
+		vld<TV, LdPlain>((const TV*)B.pb, i, t);
+		vst(v.r, 0, t);
+		vld<TV, LdPlain>(sv, i, ss);
+		if constexpr (FF) ff_st(v.x, 0, zero, zero);
+		else vst(v.x, 0, zero);
+		return term3(t, ss);
+	});
+	if (P.warm) part = residual();
+	SolveEnd S;
+	S.iter = 0;
+	S.delta = S.delta0 = T.template sum<true>(part);
+	bool done = solve_over(S.delta0, P.tol2, P.max_iter, S.status);
+	const double enough = P.tol2 * S.delta0;
+	auto beta_of = [&](double t) { return quotient(t, S.delta, (TV)0); };
+	TV beta = (TV)0;
+	while (!done && T.ok)
+	{
+		const bool first = S.iter == 0;
+		part = O.template row_sum<TV>([&](int j, int i) {
+			const Row v = row(j, i);
+			TV o[3], dn[3];
+			O.matrix(j, [&](const auto& m, int w) { team_spmv_row<TA, TV, kDepth>(m, w, lane, sv, o, dn); });
+			if (!first)
+			{
+				TV dp[3], qp[3];
+				vld<TV, LdPlain>(v.d, 0, dp);
+				vld<TV, LdPlain>(v.q, 0, qp);
+#pragma unroll
+				for (int c = 0; c < 3; ++c)
+				{
+					dn[c] = dn[c] + beta * dp[c];
+					o[c] = o[c] + beta * qp[c];
+				}
+			}
+			vst(v.q, 0, o);
+			vst(v.d, 0, dn);
+			return term3(dn, o);
+		});
+		const double dq = T.template sum<false>(part, [] {}, [&](double t) { return quotient(S.delta, t, (TV)0); });
+		if (!T.ok) break;
+		if (!bits_finite(dq))
+		{
+			S.status = B3G_SOLVE_NONFINITE;
+			break;
+		}
+		if (!bits_positive(dq))
+		{
+			S.status = B3G_SOLVE_BREAKDOWN;
+			break;
+		}
+		const TV alpha = T.ratio;
+		double dn;
+		if (P.refresh > 0 && (S.iter % P.refresh) == 0)
+		{
+			// sparse_solver.cpp:83-90: r = b - A x
+			update_x(alpha);
+			publish_x();
+			T.publish();
+			if (!T.ok) break;
+			dn = T.template sum<true>(residual(), [] {}, beta_of);
+		}
+		else
+		{
+			part = O.template row_sum<TV>([&](int j, int i) {
+				const Row v = row(j, i);
+				TV r[3], q[3], s[3];
+				vld<TV, LdPlain>(v.r, 0, r);
+				vld<TV, LdPlain>(v.q, 0, q);
+#pragma unroll
+				for (int c = 0; c < 3; ++c) r[c] -= alpha * q[c];
+				row_precond<TV>(B, v.m, i, r, s);
+				vst(v.r, 0, r);
+				vst((TV*)B.s, i, s);
+				return term3(r, s);
+			});
+			dn = T.template sum<true>(part, [&] { update_x(alpha); }, beta_of);
+		}
+		beta = T.ratio;
+		S.delta = dn;
+		S.iter += 1;
+		if (!bits_finite(dn)) S.status = B3G_SOLVE_NONFINITE;
+		else if (bits_at_most(dn, enough)) S.status = B3G_SOLVE_CONVERGED;
+		else if (S.iter >= P.max_iter) S.status = B3G_SOLVE_MAX_ITERATIONS;
+		else continue;
+		break;
+	}
+	if (!T.ok)
+	{
+		team_fault(B);
+		return;
+	}
+	if (P.newton < 0 || P.forces_left) publish_x();  // the result, or the next iteration's start
+	team_end<FILTER>(T, B, P, S, [&](auto f) {
+		O.rows([&](int j, int i) { f(i, row_dv<TV, FF>(row(j, i).x)); });
+	});
+}
+
+// The BF16 mode's solve: a flexible CG (Notay's, one stored direction) on the FP32 blocks, with
+// float-float x, preconditioned by a fixed number of Jacobi-PCG iterations with the BF16 blocks
+// from z = 0. Per outer iteration: z = P(r), p = z - (z.q_prev / p_prev.q_prev) p_prev, q = A p,
+// alpha = p.r / p.q, x += alpha p, r -= alpha q or, when a refresh is due, r = b - A x. The BF16
+// blocks, read most often, are what is kept in shared memory; the FP32 blocks stream.
+template <bool FILTER, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, SolveArgs P, int inner)
+{
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ SolveSh sh;
+	if (P.newton > 0 && B.sc->newton_done) return;
+	typedef FcgRowVecs Row;
+	constexpr int kDepth = THREADS <= 256 ? 4 : (THREADS <= 512 ? 2 : 1);
+	typedef __nv_bfloat16 TA;
+	const int lane = threadIdx.x & 31;
+	GridTeam<float> T(&sh, B.team);
+	const OwnSlices<TA> O(B, (const TA*)B.Alo, smem, P.smem, kFcgVecBytes);
+	const float* sv = (const float*)B.s;
+	const float* pv = (const float*)B.d2;
+	if (blockIdx.x == 0 && threadIdx.x == 0 && P.newton <= 0) B.sc->fault = 0;
+	auto row = [&](int j, int i) { return Row(B, W, O.vec, j, O.vec_slices, lane, i); };
+	auto matrix32 = [&](int j, auto f) {
+		const int base = B.slice_ptr[O.s0 + j];
+		f(GlobalMat<float>{B.A32, B.col, (size_t)B.nslots, (size_t)base, O.pol}, (B.slice_ptr[O.s0 + j + 1] - base) / kSlice);
+	};
+	// r = b - A x with the FP32 blocks and x in global memory; this warp's part of r.M^-1 r
+	auto residual = [&]() -> Fixed {
+		return O.row_sum<float>([&](int j, int i) {
+			const Row v = row(j, i);
+			float b[3], rr[3], ss[3], qh[3], ql[3];
+			vld<float, LdPlain>((const float*)B.pb, i, b);
+			matrix32(j, [&](const auto& m, int w) { team_spmv_row_ff(m, w, lane, B.xff, qh, ql); });
+#pragma unroll
+			for (int c = 0; c < 3; ++c) rr[c] = ff_residual(b[c], qh[c], ql[c]);
+			row_precond<float>(B, v.m, i, rr, ss);
+			vst(v.r, 0, rr);
+			return term3(rr, ss);
+		});
+	};
+	auto publish_x = [&] {
+		O.rows([&](int j, int i) {
+			if (j >= O.vec_slices) return;
+			float xh[3], xl[3];
+			ff_ld(row(j, i).x, 0, xh, xl);
+			ff_st(B.xff, i, xh, xl);
+		});
+	};
+	const float zero[3] = {0.0f, 0.0f, 0.0f};
+
+	O.load();
+	Fixed part = O.row_sum<float>([&](int j, int i) {
+		const Row v = row(j, i);
+		float t[3], ss[3];
+		if (j < O.vec_slices && B.precond != B3G_PRECOND_BLOCK_JACOBI)
+		{
+			vld<float, LdPlain>((const float*)B.Minv, i, t);
+			vst(v.m, 0, t);
+		}
+		if (P.warm)
+		{
+			if (j >= O.vec_slices) return 0.0f;
+			float xh[3], xl[3];
+			ff_ld(B.xff, i, xh, xl);
+			ff_st(v.x, 0, xh, xl);
+			return 0.0f;
+		}
+		vld<float, LdPlain>((const float*)B.pb, i, t);
+		vst(v.r, 0, t);
+		vld<float, LdPlain>(sv, i, ss);
+		ff_st(v.x, 0, zero, zero);
+		return term3(t, ss);
+	});
+	if (P.warm) part = residual();
+	SolveEnd S;
+	S.iter = 0;
+	S.delta = S.delta0 = T.sum<true>(part);
+	bool done = solve_over(S.delta0, P.tol2, P.max_iter, S.status);
+	double pq_prev = 0.0;
+	while (!done && T.ok)
+	{
+		// inner solve: r, s = M^-1 r, z = 0
+		part = O.row_sum<float>([&](int j, int i) {
+			const Row v = row(j, i);
+			float r[3], s[3];
+			vld<float, LdPlain>(v.r, 0, r);
+			row_precond<float>(B, v.m, i, r, s);
+			vst(v.ri, 0, r);
+			vst((float*)B.s, i, s);
+			vst(v.z, 0, zero);
+			return term3(r, s);
+		});
+		double delta = T.sum<true>(part);
+		if (!T.ok) break;
+		float beta = 0.0f;
+		if (isfinite(delta) && delta > 0.0)
+			for (int it = 0; it < inner; ++it)
+			{
+				part = O.row_sum<float>([&](int j, int i) {
+					const Row v = row(j, i);
+					float o[3], dn[3];
+					O.matrix(j, [&](const auto& m, int w) { team_spmv_row<TA, float, kDepth>(m, w, lane, sv, o, dn); });
+					if (it > 0)
+					{
+						float dp[3], qp[3];
+						vld<float, LdPlain>(v.di, 0, dp);
+						vld<float, LdPlain>(v.qi, 0, qp);
+#pragma unroll
+						for (int c = 0; c < 3; ++c)
+						{
+							dn[c] = dn[c] + beta * dp[c];
+							o[c] = o[c] + beta * qp[c];
+						}
+					}
+					vst(v.qi, 0, o);
+					vst(v.di, 0, dn);
+					return term3(dn, o);
+				});
+				const double dq = T.sum<false>(part, [] {}, [&](double t) { return quotient(delta, t, 0.0f); });
+				if (!T.ok || !bits_finite(dq) || !bits_positive(dq)) break;
+				const float alpha = T.ratio;
+				part = O.row_sum<float>([&](int j, int i) {
+					const Row v = row(j, i);
+					float r[3], q[3], s[3];
+					vld<float, LdPlain>(v.ri, 0, r);
+					vld<float, LdPlain>(v.qi, 0, q);
+#pragma unroll
+					for (int c = 0; c < 3; ++c) r[c] -= alpha * q[c];
+					row_precond<float>(B, v.m, i, r, s);
+					vst(v.ri, 0, r);
+					vst((float*)B.s, i, s);
+					return term3(r, s);
+				});
+				const double dn = T.sum<true>(part, [&] {
+					O.rows([&](int j, int i) {
+						const Row v = row(j, i);
+						row_x_update<float, false>(v.z, v.di, alpha);
+					});
+				}, [&](double t) { return quotient(t, delta, 0.0f); });
+				if (!T.ok) break;
+				beta = T.ratio;
+				delta = dn;
+				if (!bits_finite(dn) || !bits_positive(dn)) break;
+			}
+		if (!T.ok) break;
+		// the direction p, made A-orthogonal to the previous one, in global memory for the product
+		float bp = 0.0f;
+		if (S.iter > 0)
+		{
+			part = O.row_sum<float>([&](int j, int i) {
+				const Row v = row(j, i);
+				float z[3], q[3];
+				vld<float, LdPlain>(v.z, 0, z);
+				vld<float, LdPlain>(v.q, 0, q);
+				return term3(z, q);
+			});
+			const double gamma = T.sum<false>(part);
+			if (!T.ok) break;
+			bp = (float)(-gamma / pq_prev);
+		}
+		O.rows([&](int j, int i) {
+			const Row v = row(j, i);
+			float z[3];
+			vld<float, LdPlain>(v.z, 0, z);
+			if (S.iter > 0)
+			{
+				float p[3];
+				vld<float, LdPlain>(v.p, 0, p);
+#pragma unroll
+				for (int c = 0; c < 3; ++c) z[c] = z[c] + bp * p[c];
+			}
+			vst(v.p, 0, z);
+			vst((float*)B.d2, i, z);
+		});
+		T.publish();
+		if (!T.ok) break;
+		part = O.row_sum<float>([&](int j, int i) {
+			const Row v = row(j, i);
+			float o[3], p[3];
+			matrix32(j, [&](const auto& m, int w) { team_spmv_row<float, float, kDepth>(m, w, lane, pv, o, p); });
+			vst(v.q, 0, o);
+			return term3(p, o);
+		});
+		const double pq = T.sum<false>(part);
+		if (!T.ok) break;
+		const double pr = T.sum<false>(O.row_sum<float>([&](int j, int i) {
+			const Row v = row(j, i);
+			float p[3], r[3];
+			vld<float, LdPlain>(v.p, 0, p);
+			vld<float, LdPlain>(v.r, 0, r);
+			return term3(p, r);
+		}));
+		if (!T.ok) break;
+		pq_prev = pq;
+		if (!isfinite(pq) || !isfinite(pr))
+		{
+			S.status = B3G_SOLVE_NONFINITE;
+			break;
+		}
+		if (!(pq > 0.0))
+		{
+			S.status = B3G_SOLVE_BREAKDOWN;
+			break;
+		}
+		const float alpha = (float)(pr / pq);
+		const bool refresh = P.refresh > 0 && (S.iter % P.refresh) == 0;
+		part = O.row_sum<float>([&](int j, int i) {
+			const Row v = row(j, i);
+			row_x_update<float, true>(v.x, v.p, alpha);
+			if (refresh) return 0.0f;
+			float r[3], q[3], s[3];
+			vld<float, LdPlain>(v.r, 0, r);
+			vld<float, LdPlain>(v.q, 0, q);
+#pragma unroll
+			for (int c = 0; c < 3; ++c) r[c] -= alpha * q[c];
+			row_precond<float>(B, v.m, i, r, s);
+			vst(v.r, 0, r);
+			return term3(r, s);
+		});
+		if (refresh)
+		{
+			publish_x();
+			T.publish();
+			if (!T.ok) break;
+			part = residual();
+		}
+		const double dn = T.sum<false>(part);
+		S.delta = dn;
+		S.iter += 1;
+		if (!isfinite(dn)) S.status = B3G_SOLVE_NONFINITE;
+		else if (dn <= P.tol2 * S.delta0) S.status = B3G_SOLVE_CONVERGED;
+		else if (S.iter >= P.max_iter) S.status = B3G_SOLVE_MAX_ITERATIONS;
+		else continue;
+		break;
+	}
+	if (!T.ok)
+	{
+		team_fault(B);
+		return;
+	}
+	if (P.newton < 0 || P.forces_left) publish_x();
+	team_end<FILTER>(T, B, P, S, [&](auto f) {
+		O.rows([&](int j, int i) { f(i, row_dv<float, true>(row(j, i).x)); });
+	});
+}
+
+} // namespace
+
+} // namespace b3g

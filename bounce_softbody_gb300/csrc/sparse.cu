@@ -81,7 +81,7 @@ struct SpPattern
 	uint32_t n = 0;
 	std::vector<int> rp;     // n + 1
 	std::vector<int> cols;   // per row: the diagonal, then the other columns ascending
-	int nslices = 0;
+	int nslices = 0, maxw = 0;
 	size_t nslots = 0;
 	std::vector<int> slice_ptr;
 	int* d_slice_ptr = nullptr;
@@ -151,6 +151,7 @@ int make_pattern(int device, uint32_t n, std::vector<std::pair<int, int>>& pairs
 		}
 		w = (w + kGroup - 1) / kGroup * kGroup;
 		P->slice_ptr[s + 1] = P->slice_ptr[s] + kSlice * w;
+		P->maxw = std::max(P->maxw, w);
 	}
 	P->nslots = (size_t)P->slice_ptr[P->nslices];
 	std::vector<int> col(std::max<size_t>(P->nslots, 1));
@@ -729,6 +730,7 @@ struct SparseWork
 	DevBuf vecs;               // r d d2 q s minv py w pb: 9 x 4 n floats
 	Scalars* sc = nullptr;
 	double* partials = nullptr;
+	TeamMemory* team = nullptr;
 	double* sum = nullptr;
 	DevBuf pA;                 // BE system values
 	PatPtr sys;                // union pattern of dfdx and dfdv
@@ -1133,6 +1135,7 @@ void release_sparse(b3g_context* c)
 		w->sys.reset();
 		if (w->sc) cudaFree(w->sc);
 		if (w->partials) cudaFree(w->partials);
+		if (w->team) cudaFree(w->team);
 		delete w;
 		c->sparse_work = nullptr;
 	}
@@ -1852,6 +1855,7 @@ int work_for(b3g_context* ctx, uint32_t n, SparseWork** out)
 		if (e == cudaSuccess) e = cudaMemset(w->partials, 0, (kMaxPartials + 1) * sizeof(double));
 		w->sum = w->partials + kMaxPartials;
 	}
+	if (e == cudaSuccess && !w->team) e = cudaMalloc(&w->team, sizeof(TeamMemory));
 	if (e != cudaSuccess) return cuda_fail(e, "sparse solver workspace");
 	*out = w;
 	return B3G_OK;
@@ -1883,24 +1887,23 @@ int run_cg(b3g_context* ctx, SparseWork* w, const SpPattern* P, const float* A, 
 	D.py = x;
 	D.xff = nullptr;
 	D.sc = w->sc;
-	D.partials = w->partials;
 	cudaStream_t st = ctx->stream;
-	const int refresh = 50;  // sparse_solver.cpp:83
-	cudaError_t e = op_begin(D, st, (int)max_it, tol * tol, refresh, 0.0);
-	if (e == cudaSuccess) e = op_pcg_init(D, kP32, st);
-	int done = 0;
-	for (uint32_t it = 0; it < max_it && e == cudaSuccess && !done; it += kPcgChunk)
-	{
-		for (uint32_t j = it; j < std::min<uint32_t>(it + kPcgChunk, max_it) && e == cudaSuccess; ++j)
-			e = op_pcg_iteration(D, kP32, (int)j, refresh, st);
-		if (e == cudaSuccess) e = cudaMemcpyAsync(&ctx->h_scalars->done, &w->sc->done, sizeof(int), cudaMemcpyDeviceToHost, st);
-		if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-		done = ctx->h_scalars->done;
-	}
+	D.team = w->team;
+	D.maxw = P->maxw;
+	SolveArgs S;
+	std::memset(&S, 0, sizeof(S));
+	S.tol2 = tol * tol;
+	S.max_iter = (int)max_it;
+	S.refresh = 50;  // sparse_solver.cpp:83
+	S.newton = -1;
+	S.warm = 1;
+	cudaError_t e = op_solve_clear(D, st);
+	if (e == cudaSuccess) e = op_solve(D, S, kP32, st);
 	if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_scalars, w->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st);
 	if (e == cudaSuccess) e = cudaStreamSynchronize(st);
 	if (e != cudaSuccess) return cuda_fail(e, "sparse CG");
 	*out = *ctx->h_scalars;
+	if (out->fault) out->status = B3G_SOLVE_DEVICE_TIMEOUT;
 	return B3G_OK;
 }
 
