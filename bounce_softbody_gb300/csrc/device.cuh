@@ -54,6 +54,19 @@ __device__ __forceinline__ unsigned long long evict_first_policy()
 	return pol;
 }
 
+__device__ __forceinline__ unsigned long long evict_normal_policy()
+{
+	unsigned long long pol;
+	asm("createpolicy.fractional.L2::evict_normal.b64 %0, 1.0;" : "=l"(pol));
+	return pol;
+}
+__device__ __forceinline__ unsigned long long evict_last_policy()
+{
+	unsigned long long pol;
+	asm("createpolicy.fractional.L2::evict_last.b64 %0, 1.0;" : "=l"(pol));
+	return pol;
+}
+
 template <class M>
 __device__ __forceinline__ uint4 mat_ld16(const void* p, unsigned long long pol);
 template <>

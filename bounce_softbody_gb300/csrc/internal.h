@@ -111,7 +111,6 @@ struct TeamMemory
 {
 	unsigned arrived;
 	unsigned pad[31];
-	unsigned long long slots[2][kTeamMax];
 	unsigned long long tagged[2][kTeamReplicas][kTeamMax];
 };
 

@@ -52,6 +52,7 @@ struct SolveArgs
 	int forces_left;   // another Newton iteration may follow this one
 	int warm;          // start from the solution at hand (r = b - A x) instead of zero
 	int smem;          // bytes of shared memory of a CTA (set by op_solve)
+	int keep;          // 1/1024 of a CTA's slices whose matrix stays in L2 (set by op_solve)
 };
 cudaError_t op_solve(const DevBody& B, const SolveArgs& P, int prec, cudaStream_t st);
 // the team's reduction slots cleared before a solve (op_assemble does it for a body step)

@@ -19,6 +19,7 @@
 
 #include "device.cuh"
 #include "ops.h"
+#include "solve.cuh"
 
 #include <atomic>
 #include <cooperative_groups.h>
@@ -121,11 +122,6 @@ struct Team
 	}
 };
 
-
-// Phases timed by the optional instrumentation (cycles of thread 0 of each CTA, barriers and
-// reductions included in the phase that ends with them). The direction update runs inside the
-// SpMV sweep, so kPhDir stays zero; its slot keeps the numbering the host reads.
-enum { kPhElem = 0, kPhAsm = 1, kPhSpmv = 2, kPhUpdate = 3, kPhDir = 4, kPhFinal = 5, kPhIdle = 6, kPhases = 8 };
 
 struct PhaseClock
 {
@@ -524,52 +520,6 @@ __device__ void team_step_assemble(Team<CL>& T, const DevBody& B, const BatchPar
 	if (T.tid() == 0) B.sc->delta0 = delta0;
 }
 
-// Part 2: the PCG, the final update and the statistics.
-template <int CL, class TA, class TV>
-__device__ void team_step_solve(Team<CL>& T, const DevBody& B, const BatchParams& P, bool bf16)
-{
-	typedef typename std::conditional<CL == 1, LdPlain, LdCG>::type LD;
-	const int lane = threadIdx.x & 31;
-	PhaseClock pc;
-	pc.start(P.prof);
-	double delta0;
-	if (P.flat)
-	{
-		// the flat row launch left r and s: delta0 = r.s, summed in the order the team assembly
-		// sums it (each warp its slices, then the team), so it is the same value bitwise
-		double part = 0.0;
-		for (int sl = T.warp(); sl < B.nslices; sl += T.nwarps())
-		{
-			const int i = sl * kSlice + lane;
-			if (i >= B.n) continue;
-			TV rr[3], ss[3];
-			vld<TV, LD>((const TV*)B.r, i, rr);
-			vld<TV, LD>((const TV*)B.s, i, ss);
-			part += dot3<TV>(rr, ss);
-		}
-		delta0 = T.reduce(part);
-		if (T.tid() == 0)
-		{
-			B.sc->fault = 0;
-			B.sc->delta0 = delta0;
-		}
-	}
-	else
-		delta0 = __ldcg(&B.sc->delta0);
-	const SolveOut so = team_pcg<CL, TA, TV, LD>(T, B, P, bf16, delta0, pc);
-	T.sync();
-	double part = 0.0;
-	for (int sl = T.warp(); sl < B.nslices; sl += T.nwarps())
-	{
-		const int i = sl * kSlice + lane;
-		if (i < B.n)
-			part += B.filt ? final_vertex_filtered<TV, LD>(B, i, P.h, true, true) : final_vertex<TV, LD>(B, i, P.h, true, true);
-	}
-	const double err = T.reduce(part);
-	pc.tick(kPhFinal);
-	team_finish<CL, TV, LD>(T, B, P, so, delta0, 1, so.iter, so.iter, (unsigned long long)so.iter, err, pc);
-}
-
 __device__ void load_body(DevBody* dst, const DevBody* src)
 {
 	const int words = (int)(sizeof(DevBody) / sizeof(int));
@@ -578,29 +528,23 @@ __device__ void load_body(DevBody* dst, const DevBody* src)
 	for (int k = threadIdx.x; k < words; k += blockDim.x) d[k] = __ldcg(s + k);
 }
 
-#ifndef B3G_SOLVE_MIN_BLOCKS  // resident CTAs per SM of the PCG launch (64 registers a thread)
-#define B3G_SOLVE_MIN_BLOCKS (B3G_PCG_THREADS >= 512 ? 2 : 4)
-#endif
-
-// Launch phases: the whole step (any number of Newton iterations), or the two parts of a
-// single-Newton step. Each part takes its work from its own pair of counters.
-enum { kPhaseWhole = 0, kPhaseAssemble = 1, kPhaseSolve = 2 };
+// Launch phases of the team kernel: the whole step (any number of Newton iterations), or the
+// assembly of a single-Newton step, which k_batch_solve completes from its own pair of counters.
+enum { kPhaseWhole = 0, kPhaseAssemble = 1 };
 
 template <int CL, class TA, class TV, int PH>
 __device__ __forceinline__ void team_run(Team<CL>& T, const DevBody& B, const BatchParams& P, bool bf16)
 {
 	if (PH == kPhaseWhole) team_step<CL, TA, TV>(T, B, P, bf16);
-	else if (PH == kPhaseAssemble) team_step_assemble<CL, TA, TV>(T, B, P, bf16);
-	else team_step_solve<CL, TA, TV>(T, B, P, bf16);
+	else team_step_assemble<CL, TA, TV>(T, B, P, bf16);
 }
 
 template <int CL, class TA, class TV, int PH>
-__global__ void __launch_bounds__(kPThreads, PH == kPhaseSolve ? B3G_SOLVE_MIN_BLOCKS : B3G_BATCH_MIN_BLOCKS)
-k_batch(BatchParams P, int bf16)
+__global__ void __launch_bounds__(kPThreads, B3G_BATCH_MIN_BLOCKS) k_batch(BatchParams P, int bf16)
 {
 	__shared__ TeamShared sh;
 	__shared__ __align__(16) DevBody sb;
-	unsigned* queue = P.queue + (PH == kPhaseSolve ? 2 : 0);
+	unsigned* queue = P.queue;
 
 	if (CL > 1)
 	{
@@ -637,6 +581,82 @@ k_batch(BatchParams P, int bf16)
 		__syncthreads();
 		for (int st = 0; st < P.steps; ++st) team_run<1, TA, TV, PH>(T1, sb, P, bf16 != 0);
 		__syncthreads();
+	}
+}
+
+// The PCG, the final update and the statistics of every body of a batch (single-Newton steps), by
+// clusters of CL CTAs and then by single CTAs, as k_batch distributes them; each body is solved by
+// team_solve with its rows' vectors and as much of its matrix as fits in shared memory.
+// One CTA of 512 threads per SM (128 registers a thread, the SM's shared memory to itself). Measured
+// on 160 / 12 uneven blocks and 16 blocks and cloths, ms a step: 512 x 1 12.1 / 1.54 / 7.0, 640 x 1
+// 12.2 / 1.59 / 6.6, 768 x 1 14.4 / 1.68 / 7.4 (spills), 320 x 2 12.9 / 1.90 / 8.8, 256 x 2 14.5 /
+// 1.97 / 10.8; the launch before (256 x 4, every vector and matrix through L2 and HBM) 14.0 / 2.99 / 12.1.
+
+__device__ __noinline__ double final_vertex_dv_filtered(const DevBody& B, int i, float h, bool finish, float3 dv)
+{
+	return final_vertex_dv<LdPlain, true>(B, i, h, true, finish, dv);
+}
+
+template <class TA, class TV, class Team>
+__device__ __forceinline__ void batch_solve_body(Team& T, const DevBody& B, const BatchParams& P, unsigned char* smem, int room)
+{
+	PhaseClock pc;
+	pc.start(P.prof);
+	SolveArgs A;
+	A.tol2 = P.tol2;
+	A.newton_tol2 = P.newton_tol2;
+	A.max_iter = P.max_iter;
+	A.refresh = P.refresh;
+	A.h = P.h;
+	A.newton = 0;
+	A.newton_max = 1;
+	A.forces_left = 0;
+	A.warm = 0;
+	A.smem = room;
+	A.keep = 1024;
+	team_solve<TA, TV, false, 1>(
+	    T, B, A, smem,
+	    [&](int i, float3 dv, bool finish) {
+		    return B.filt ? final_vertex_dv_filtered(B, i, A.h, finish, dv) : final_vertex_dv<LdPlain, false>(B, i, A.h, true, finish, dv);
+	    },
+	    [&](int phase) { pc.tick(phase); });
+}
+
+template <int CL, class TA, class TV>
+__global__ void __launch_bounds__(kSolveMaxThreads, 1) k_batch_solve(BatchParams P, int room)
+{
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ SolveSh sh;
+	__shared__ __align__(16) DevBody sb;
+	__shared__ int s_item;
+	unsigned* queue = P.queue + 2;
+	if (CL > 1)
+	{
+		cg::cluster_group cl = cg::this_cluster();
+		ClusterTeam<TV, CL> T(&sh);
+		for (;;)
+		{
+			if (T.rank == 0 && threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
+			cl.sync();
+			const int item = *cl.map_shared_rank(&s_item, 0);
+			cl.sync();
+			if (item >= P.nbig) break;
+			load_body(&sb, P.bodies + P.big[item]);
+			__syncthreads();
+			batch_solve_body<TA, TV>(T, sb, P, smem, room);
+		}
+	}
+	ClusterTeam<TV, 1> T(&sh);
+	for (;;)
+	{
+		__syncthreads();
+		if (threadIdx.x == 0) s_item = (int)atomicAdd(queue + 1, 1u);
+		__syncthreads();
+		const int item = s_item;
+		if (item >= P.nsmall) break;
+		load_body(&sb, P.bodies + P.small[item]);
+		__syncthreads();
+		batch_solve_body<TA, TV>(T, sb, P, smem, room);
 	}
 }
 
@@ -688,8 +708,40 @@ int max_clusters_ph()
 	return n;
 }
 
-// Co-resident clusters of the solve launch (more CTAs per SM than the assembly launch), queried
-// once per instantiation.
+// Shared memory of a CTA of the solve launch: what its static part leaves of its share of the SM.
+inline int solve_room()
+{
+	static const int room = [] {
+		int dev = 0, block = 0, sm = 0;
+		cudaGetDevice(&dev);
+		cudaDeviceGetAttribute(&block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
+		cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
+		return (std::min(block, sm - 1024) - (int)(sizeof(SolveSh) + sizeof(DevBody)) - 256) & ~127;
+	}();
+	return room;
+}
+
+template <int CL, class TA, class TV>
+cudaError_t solve_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int ctas, cudaStream_t st)
+{
+	cudaError_t e = cudaFuncSetAttribute(k_batch_solve<CL, TA, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve_room());
+	if (e == cudaSuccess && CL > 8)
+		e = cudaFuncSetAttribute(k_batch_solve<CL, TA, TV>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+	*cfg = {};
+	cfg->gridDim = dim3((unsigned)ctas, 1, 1);
+	cfg->blockDim = dim3(kSolveMaxThreads, 1, 1);
+	cfg->dynamicSmemBytes = (size_t)solve_room();
+	cfg->stream = st;
+	attr->id = cudaLaunchAttributeClusterDimension;
+	attr->val.clusterDim.x = CL;
+	attr->val.clusterDim.y = 1;
+	attr->val.clusterDim.z = 1;
+	cfg->attrs = attr;
+	cfg->numAttrs = 1;
+	return e;
+}
+
+// Co-resident clusters of the solve launch, queried once per instantiation.
 template <int CL, class TA, class TV>
 int solve_clusters()
 {
@@ -697,7 +749,13 @@ int solve_clusters()
 	int m = cached.load(std::memory_order_relaxed);
 	if (m < 0)
 	{
-		m = max_clusters_ph<CL, TA, TV, kPhaseSolve>();
+		cudaLaunchConfig_t cfg;
+		cudaLaunchAttribute attr;
+		m = 0;
+		if (solve_config<CL, TA, TV>(&cfg, &attr, CL, nullptr) == cudaSuccess &&
+		    cudaOccupancyMaxActiveClusters(&m, k_batch_solve<CL, TA, TV>, &cfg) != cudaSuccess)
+			m = 0;
+		cudaGetLastError();
 		cached.store(m, std::memory_order_relaxed);
 	}
 	return m;
@@ -716,7 +774,11 @@ cudaError_t launch_cl(const BatchParams& P, int ctas, int bf16, int part, cudaSt
 		if (e != cudaSuccess || part == 1) return e;
 	}
 	const int m = solve_clusters<CL, TA, TV>();
-	return launch_ph<CL, TA, TV, kPhaseSolve>(P, m > 0 ? m * CL : ctas, bf16, st);
+	cudaLaunchConfig_t cfg;
+	cudaLaunchAttribute attr;
+	cudaError_t e = solve_config<CL, TA, TV>(&cfg, &attr, m > 0 ? m * CL : CL, st);
+	if (e != cudaSuccess) return e;
+	return cudaLaunchKernelEx(&cfg, k_batch_solve<CL, TA, TV>, P, solve_room());
 }
 
 // The body of flat item g: the last k with off[k] <= g.
@@ -775,8 +837,8 @@ k_batch_rows(BatchParams P)
 		}
 		__syncwarp();
 		const int sl = (int)(g - __ldg(P.slice_off + b));
-		if (FILT && B.filt) assemble_row_filtered<TA, TV, LdPlain>(B, sl, lane, sp, kInitAll);
-		else assemble_row<TA, TV, LdPlain, false, TETS>(B, sl, lane, sp, kInitAll);
+		if (FILT && B.filt) assemble_row_filtered<TA, TV, LdPlain>(B, sl, lane, sp, kInitTeam);
+		else assemble_row<TA, TV, LdPlain, false, TETS>(B, sl, lane, sp, kInitTeam);
 	}
 }
 
@@ -825,7 +887,7 @@ cudaError_t launch_prec(const BatchParams& P, int cluster, int ctas, int bf16, i
 template <int CL, class TA, class TV>
 int max_clusters()
 {
-	solve_clusters<CL, TA, TV>();
+	if (solve_clusters<CL, TA, TV>() <= 0) return 0;
 	return max_clusters_ph<CL, TA, TV, kPhaseAssemble>();
 }
 

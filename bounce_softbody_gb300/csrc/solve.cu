@@ -28,12 +28,19 @@ const Device& device()
 	return d;
 }
 
-// A CTA takes consecutive slices, one warp each up to 32 warps. At least four slices a CTA: on
-// small bodies fewer CTAs make the sums cheaper than more CTAs make the sweeps (10^3 block, 32
-// slices: 32 / 16 / 8 / 4 CTAs 263 / 265 / 256 / 300 us a step).
+// A CTA takes consecutive slices, one warp each up to 16 warps (128 registers a thread; 1024 threads
+// at 64 registers spill in the sweep: 64^3 block 13.6 ms a step against 11.1). At least four slices a
+// CTA: on small bodies fewer CTAs make the sums cheaper than more CTAs make the sweeps (10^3 block,
+// 32 slices: 32 / 16 / 8 / 4 CTAs 263 / 265 / 256 / 300 us a step).
+// keep: what shared memory does not hold of the matrix goes through L2 once per iteration. Up to
+// kL2Keep bytes of it all stay there. Beyond, a cyclic sweep under LRU would find nothing left, so
+// kL2Keep bytes are kept (evict last) and the rest streams past them (evict first). 64^3 block,
+// 165 MB: 0 / 25 / 37 / 50 / 62 / 75 / 100 % kept 12.8 / 12.4 / 12.0 / 11.7 / 12.7 / 13.6 / 14.1 ms.
+constexpr size_t kL2Keep = (size_t)80 << 20;
+
 struct Geometry
 {
-	int ctas, threads, smem;
+	int ctas, threads, smem, keep;
 };
 
 Geometry geometry(const DevBody& B, size_t vec_bytes, size_t slot_bytes)
@@ -43,9 +50,14 @@ Geometry geometry(const DevBody& B, size_t vec_bytes, size_t slot_bytes)
 	Geometry g;
 	g.ctas = std::max(1, (B.nslices + per - 1) / per);
 	const int slices = (B.nslices + g.ctas - 1) / g.ctas;
-	g.threads = 32 * std::max(1, std::min(slices, kSolveMaxThreads / 32));
+	const int rounds = (slices + kSolveMaxThreads / 32 - 1) / (kSolveMaxThreads / 32);
+	g.threads = 32 * std::max(1, (slices + rounds - 1) / rounds);
 	const size_t want = (size_t)slices * (vec_bytes + (size_t)B.maxw * kSlice * slot_bytes);
 	g.smem = (int)(std::min(want, (size_t)dv.room) & ~(size_t)127);
+	const size_t total = (size_t)B.nslots * slot_bytes;
+	const size_t held = (size_t)g.ctas * (size_t)std::max(0, g.smem - (int)std::min<size_t>(slices * vec_bytes, g.smem));
+	const size_t stream = total > held ? total - held : 0;
+	g.keep = stream <= kL2Keep ? 1024 : (int)(1024 * kL2Keep / stream);
 	return g;
 }
 
@@ -73,9 +85,9 @@ cudaError_t launch_solve(const DevBody& B, SolveArgs P, cudaStream_t st)
 {
 	const Geometry g = geometry(B, solve_vec_bytes<TV, FF>(), solve_slot_bytes<TA>());
 	P.smem = g.smem;
+	P.keep = g.keep;
 	if (g.threads <= 256) return launch_team(k_solve<TA, TV, FF, FILTER, 256>, g, st, B, P);
-	if (g.threads <= 512) return launch_team(k_solve<TA, TV, FF, FILTER, 512>, g, st, B, P);
-	return launch_team(k_solve<TA, TV, FF, FILTER, 1024>, g, st, B, P);
+	return launch_team(k_solve<TA, TV, FF, FILTER, 512>, g, st, B, P);
 }
 
 template <bool FILTER>
@@ -83,9 +95,9 @@ cudaError_t launch_fcg(const DevBody& B, const FcgVecs& W, SolveArgs P, int inne
 {
 	const Geometry g = geometry(B, kFcgVecBytes, solve_slot_bytes<__nv_bfloat16>());
 	P.smem = g.smem;
+	P.keep = g.keep;
 	if (g.threads <= 256) return launch_team(k_solve_fcg<FILTER, 256>, g, st, B, W, P, inner);
-	if (g.threads <= 512) return launch_team(k_solve_fcg<FILTER, 512>, g, st, B, W, P, inner);
-	return launch_team(k_solve_fcg<FILTER, 1024>, g, st, B, W, P, inner);
+	return launch_team(k_solve_fcg<FILTER, 512>, g, st, B, W, P, inner);
 }
 
 } // namespace

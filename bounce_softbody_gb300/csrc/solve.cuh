@@ -5,23 +5,24 @@
 // the solver vectors' round trips. Here the whole solve is one launch. A CTA owns a contiguous run
 // of 32-row slices for the launch: their vectors (r, d, q, x, and the scalar Jacobi) stay in shared
 // memory, and so does as much of their matrix as fits; only s, which neighbours gather, goes
-// through global memory (L2). Two team-wide sums per iteration are all that is exchanged:
-//   d.q     after q = A s + beta q, d = s + beta d  (nothing is written that others read: no fence)
-//   r.s     after r -= alpha q, s = M^-1 r          (release / acquire: s becomes visible)
-// and x += alpha d runs while the second sum is on its way.
+// through global memory (L2). Besides s, two team-wide sums per iteration are all that is exchanged:
+// d.q after q = A s + beta q, d = s + beta d, and r.s after r -= alpha q, s = M^-1 r. x += alpha d
+// runs while the second sum is on its way.
 //
-// Team sums. One warp of every CTA adds the CTAs' partials up in CTA order, so every thread holds
-// the same bits and takes the same decisions. Measured on one GB300 (us a sum, 4 / 32 / 152 CTAs):
-// * r.s, which publishes s: partials in slots, arrivals counted by one release atomic that one lane
-//   of every CTA polls, then the slots are read: 1.2 / 1.4 / 1.5. Polling the slots themselves
-//   behind a fence instead: 1.1 / 1.7 / 2.2 at best;
-// * d.q, which publishes nothing: the partials carry two bits of the sum's number in their lowest
-//   mantissa bits (4e-16 of the partial), and the slots are polled without any fence or atomic:
-//   0.4 / 0.95 / 1.6. Above 16 CTAs the slots exist 16 times, a replica for every 16th CTA: with
-//   one copy the pollers' traffic on the same lines costs 0.4 / 1.4 / 3.8.
-// Two slot arrays alternate in both kinds: a CTA can only overwrite its slot of sum e with that of
-// sum e + 2 after every CTA has arrived at sum e + 1, and so has read sum e. Polls are bounded; a
-// sum that never completes sets Scalars::fault and ends the launch.
+// Team sums. Every CTA stores its partial in its slot with two bits of the sum's number in the
+// lowest mantissa bits (4e-16 of the partial); one warp of every CTA polls all slots and adds them
+// up, so every thread holds the same bits and takes the same decisions. No fence and no atomic is on
+// that path. Above 16 CTAs the slots exist 16 times, a replica for every 16th CTA: with one copy
+// the pollers' traffic on the same lines costs 0.4 / 1.4 / 3.8 us a sum for 4 / 32 / 152 CTAs, with
+// sixteen 0.9 / 0.95 / 1.6. Two slot arrays alternate: a CTA can only overwrite its slot of sum e
+// with that of sum e + 2 after every CTA has arrived at sum e + 1, and so has read sum e. The same
+// holds for s, rewritten only after the sum that follows the sweep which gathers it.
+// s itself needs no barrier in the FP32 and BF16 modes: its fourth component carries the number of
+// its version, a vertex's 16 bytes are written and read as one access, and a gather that meets an
+// older version reads again. What does not fit one access (FP64 vectors, x of a refresh) is
+// published by a release atomic on an arrival counter that the CTAs poll, behind the sum's slots: the
+// fence alone costs 900 clocks.
+// All polls are bounded; a wait that runs out sets Scalars::fault and ends the launch.
 // FP64 is slow on this GPU: an FP64 instruction occupies the SM's pipe for 16 clocks a warp and its
 // result takes about 100; a division takes about 1000. Measured per iteration of a small body with
 // FP64 trees and divisions: 1500 clocks of the update and 1000 of each sum. So sums are exact integer sums of
@@ -34,11 +35,14 @@
 #include "device.cuh"
 #include "ops.h"
 
+#include <cooperative_groups.h>
+#include <type_traits>
+
 namespace b3g {
 
 namespace {
 
-constexpr int kSolveMaxThreads = 1024;
+constexpr int kSolveMaxThreads = 512;
 constexpr int kPollLimit = 1 << 20;           // polls before a warp gives up (about a second)
 constexpr int kTeamWarpSlots = kTeamMax / 32; // slots a lane of the polling warp reads
 
@@ -107,28 +111,31 @@ __device__ __forceinline__ Fixed fixed_add(Fixed a, Fixed b)
 	const int e = max(a.e, b.e);
 	return fixed_norm((a.m >> min(e - a.e, 63)) + (b.m >> min(e - b.e, 63)), e);
 }
-// the 32 lanes' sum, in all lanes: aligned to the largest exponent, in limbs of 20 bits whose sums
-// fit 32 bits
+// the 32 lanes' sum, in all lanes, |m| < 2^63: aligned to the largest exponent, in limbs of 20 bits
+// whose sums fit 32 bits
 __device__ __forceinline__ Fixed fixed_warp_sum(Fixed a)
 {
-	const int e = __reduce_max_sync(0xffffffffu, a.e);
-	const long long q = a.m >> min(e - a.e, 63);
+	Fixed t;
+	t.e = __reduce_max_sync(0xffffffffu, a.e);
+	const long long q = a.m >> min(t.e - a.e, 63);
 	const int l0 = (int)__reduce_add_sync(0xffffffffu, (unsigned)(q & 0xfffff));
 	const int l1 = (int)__reduce_add_sync(0xffffffffu, (unsigned)((q >> 20) & 0xfffff));
 	const int l2 = __reduce_add_sync(0xffffffffu, (int)(q >> 40));
-	return fixed_norm((long long)l0 + ((long long)l1 << 20) + ((long long)l2 << 40), e);
+	t.m = (long long)l0 + ((long long)l1 << 20) + ((long long)l2 << 40);
+	return t;
 }
-// the nearest double towards zero
+// the nearest double towards zero (|m| < 2^63)
 __device__ __forceinline__ double fixed_value(Fixed a)
 {
-	if (a.e >= kNotFinite) return __longlong_as_double(0x7ff8000000000000ll);
 	const unsigned long long u = (unsigned long long)(a.m < 0 ? -a.m : a.m);
 	const int lead = 63 - __clzll((long long)u);  // u = 1.xxx 2^lead
 	const int ex = a.e + lead + 1023;
-	if (u == 0 || ex <= 0) return 0.0;
+	const unsigned long long frac = ((u << (63 - lead)) >> 11) & 0xfffffffffffffull;
+	const unsigned long long v = ((unsigned long long)ex << 52) | frac | (a.m < 0 ? 1ull << 63 : 0ull);
+	if (u == 0 && a.e < kNotFinite) return 0.0;
+	if (ex <= 0) return 0.0;
 	if (ex >= 0x7ff) return __longlong_as_double(0x7ff8000000000000ll);
-	const unsigned long long frac = (lead >= 52 ? u >> (lead - 52) : u << (52 - lead)) & 0xfffffffffffffull;
-	return __longlong_as_double((long long)((a.m < 0 ? 1ull << 63 : 0ull) | ((unsigned long long)ex << 52) | frac));
+	return __longlong_as_double((long long)v);
 }
 
 // Comparisons on the bits of doubles (an FP64 comparison waits for the FP64 pipe)
@@ -137,26 +144,52 @@ __device__ __forceinline__ bool bits_positive(double x) { return __double_as_lon
 // x <= y for finite x and y >= 0
 __device__ __forceinline__ bool bits_at_most(double x, double y) { return __double_as_longlong(x) <= __double_as_longlong(y); }
 
-// a / b rounded to the vector type. For float, the mantissas are split into two floats each and
-// divided in double-single arithmetic (Dekker, A floating-point technique for extending the
-// available precision, 1971: quotient estimate and one correction from the remainder), good to
-// about 2^-44 before the rounding to 24 bits.
-__device__ __forceinline__ double quotient(double a, double b, double) { return a / b; }
-__device__ __forceinline__ float quotient(double a, double b, float)
+// a / b rounded to the vector type. For float, in double-single arithmetic (Dekker, A floating-point
+// technique for extending the available precision, 1971): each mantissa as two floats, the
+// denominator's reciprocal as an estimate and its correction, good to about 2^-44 before the rounding
+// to 24 bits. The reciprocal is formed ahead where the denominator is known ahead.
+template <class TV>
+struct Divisor;
+template <>
+struct Divisor<double>
 {
-	const unsigned long long ua = (unsigned long long)__double_as_longlong(a), ub = (unsigned long long)__double_as_longlong(b);
-	const int ea = (int)((ua >> 52) & 0x7ff), eb = (int)((ub >> 52) & 0x7ff);
-	if (ea == 0 || eb == 0 || ea == 0x7ff || eb == 0x7ff) return (float)(a / b);
-	// mantissas in [1, 2): 23 fraction bits in the high float, 29 in the low one
-	const float ah = __uint_as_float(0x3f800000u | (unsigned)((ua >> 29) & 0x7fffffu));
-	const float bh = __uint_as_float(0x3f800000u | (unsigned)((ub >> 29) & 0x7fffffu));
-	const float al = (float)(unsigned)(ua & 0x1fffffffu) * 0x1p-52f, bl = (float)(unsigned)(ub & 0x1fffffffu) * 0x1p-52f;
-	const float inv = __fdividef(1.0f, bh);
-	const float q0 = ah * inv;
-	const float rem = fmaf(-q0, bh, ah) + fmaf(-q0, bl, al);
-	const float q = fmaf(rem, inv, q0);
-	return scalbnf(((ua ^ ub) >> 63) ? -q : q, ea - eb);
-}
+	double b;
+	__device__ __forceinline__ explicit Divisor(double v) : b(v) {}
+	__device__ __forceinline__ double divide(double a) const { return a / b; }
+};
+template <>
+struct Divisor<float>
+{
+	double b;
+	float hi, lo;
+	int e;       // exponent field of b; 0 or 0x7ff: the FP64 division
+	bool neg;
+	__device__ __forceinline__ explicit Divisor(double v) : b(v)
+	{
+		const unsigned long long u = (unsigned long long)__double_as_longlong(v);
+		e = (int)((u >> 52) & 0x7ff);
+		neg = (u >> 63) != 0;
+		// mantissa in [1, 2): 23 fraction bits in the high float, 29 in the low one
+		const float bh = __uint_as_float(0x3f800000u | (unsigned)((u >> 29) & 0x7fffffu));
+		const float bl = (float)(unsigned)(u & 0x1fffffffu) * 0x1p-52f;
+		hi = __fdividef(1.0f, bh);
+		lo = hi * (fmaf(-bh, hi, 1.0f) - bl * hi);
+	}
+	__device__ __forceinline__ float divide(double a) const
+	{
+		const unsigned long long u = (unsigned long long)__double_as_longlong(a);
+		const int ea = (int)((u >> 52) & 0x7ff);
+		const float ah = __uint_as_float(0x3f800000u | (unsigned)((u >> 29) & 0x7fffffu));
+		const float al = (float)(unsigned)(u & 0x1fffffffu) * 0x1p-52f;
+		const float q0 = ah * hi;
+		const float q = q0 + (fmaf(ah, hi, -q0) + fmaf(ah, lo, al * hi));
+		const unsigned qb = __float_as_uint(q);
+		const int ex = (int)(qb >> 23) + (ea - e);
+		// a zero, a denormal, a value that is not finite, or a quotient outside the normal floats
+		if (ea == 0 || ea == 0x7ff || e == 0 || e == 0x7ff || ex <= 0 || ex >= 0xff) return (float)(a / b);
+		return __uint_as_float((qb & 0x7fffffu) | ((unsigned)ex << 23) | (((u >> 63) != 0) != neg ? 0x80000000u : 0u));
+	}
+};
 
 // One row's term of a dot product in the vector type (dot3 widens it)
 template <class TV>
@@ -169,82 +202,101 @@ struct SolveSh
 {
 	Fixed w[2][32];
 	double total, ratio;
-	int ok;
+	int ok, lost;
+	unsigned long long slot[2][kMaxTeamCtas];  // a cluster's partials
 };
 
-// The reduction memory of a team (cleared before the launch): an arrival counter, slots of the
-// sums that publish data, and the replicated slots of the others.
+// The sum of a CTA's warps, in warp 0 (v is each warp's value, already in sh->w[buf])
+__device__ __forceinline__ double cta_total(const SolveSh* sh, int buf, Fixed v)
+{
+	const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
+	if (nw > 1)
+	{
+		Fixed z;
+		z.m = 0;
+		z.e = kFixedZero;
+		if (lane < nw) z = sh->w[buf][lane];
+		v = fixed_warp_sum(z);
+	}
+	return fixed_value(v);
+}
+
+// The reduction memory (cleared before the launch) and this CTA's place in the team.
 template <class TV>
 struct GridTeam
 {
+	static constexpr bool kManyCtas = true;
 	SolveSh* sh;
 	TeamMemory* mem;
 	int ctas, rank;
 	int replicas;
-	unsigned published, plain;  // sums of each kind so far
+	unsigned sums, fences;  // so far
 	int ok;
 	TV ratio;
 
 	__device__ __forceinline__ GridTeam(SolveSh* s, TeamMemory* m)
-	    : sh(s), mem(m), ctas(gridDim.x), rank(blockIdx.x), replicas(gridDim.x > 16 ? kTeamReplicas : 1), published(0),
-	      plain(0), ok(1), ratio((TV)0)
+	    : sh(s), mem(m), ctas(gridDim.x), rank(blockIdx.x), replicas(gridDim.x > 16 ? kTeamReplicas : 1), sums(0), fences(0),
+	      ok(1), ratio((TV)0)
 	{
+		if (threadIdx.x == 0) sh->lost = 0;
 	}
 
 	// This warp's value v (the same in all lanes) summed over the team. `between` runs after this
-	// CTA's partial is on its way; ratio(total) is evaluated once per CTA and left in `ratio`.
-	// VISIBLE: what the team's threads wrote before the sum may be read by all of them after it.
-	template <bool VISIBLE, class F, class R>
+	// CTA's partial is on its way; ratio_of(total) is evaluated once per CTA and left in `ratio`.
+	// FENCE: what the team's threads wrote before the sum may be read by all of them after it.
+	template <bool FENCE, class F, class R>
 	__device__ __forceinline__ double sum(Fixed v, F between, R ratio_of)
 	{
-		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5;
-		const int buf = (published + plain) & 1;
-		if (nw > 1)
-		{
-			if (lane == 0) sh->w[buf][warp] = v;
-			__syncthreads();
-		}
-		else
-			__syncwarp();
-		unsigned long long* mine = nullptr;
-		unsigned long long tag = 0;
+		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+		const int buf = sums & 1;
+		if (lane == 0) sh->w[buf][warp] = v;
+		__syncthreads();
+		const unsigned long long tag = (unsigned long long)(((sums >> 1) + 1) & 3);
+		unsigned long long(*all)[kTeamMax] = mem->tagged[buf];
 		if (warp == 0)
 		{
-			if (nw > 1)
-			{
-				Fixed z;
-				z.m = 0;
-				z.e = kFixedZero;
-				v = fixed_warp_sum(lane < nw ? sh->w[buf][lane] : z);
-			}
-			const unsigned long long bits = (unsigned long long)__double_as_longlong(fixed_value(v));
-			if (VISIBLE)
-			{
-				mine = mem->slots[published & 1];
-				if (lane == 0)
-				{
-					st_relaxed(mine + rank, bits);
-					red_release(&mem->arrived);
-				}
-			}
-			else
-			{
-				tag = (unsigned long long)(((plain >> 1) + 1) & 3);
-				unsigned long long(*all)[kTeamMax] = mem->tagged[plain & 1];
-				mine = all[rank & (replicas - 1)];
-				if (lane < replicas) st_relaxed(all[lane] + rank, (bits & ~3ull) | tag);
-			}
+			const unsigned long long bits = (unsigned long long)__double_as_longlong(cta_total(sh, buf, v));
+			if (lane < replicas) st_relaxed(all[lane] + rank, (bits & ~3ull) | tag);
+			if (FENCE && lane == 0) red_release(&mem->arrived);
 		}
 		between();
 		if (warp == 0)
 		{
+			const unsigned long long* mine = all[rank & (replicas - 1)];
 			unsigned long long u[kTeamWarpSlots];
 			int polls = 0;
-			bool there = true;
-			if (VISIBLE)
+			bool there;
+			for (;;)
 			{
-				const unsigned want = (published + 1) * (unsigned)ctas;
-				// every lane polls, so that each lane's slot reads follow its own acquire
+				there = true;
+#pragma unroll
+				for (int q = 0; q < kTeamWarpSlots; ++q)
+				{
+					u[q] = lane + 32 * q < ctas ? ld_relaxed(mine + lane + 32 * q) : tag;
+					there = there && (u[q] & 3ull) == tag;
+				}
+				there = __all_sync(0xffffffffu, there) != 0;
+				if (there || ++polls > kPollLimit) break;
+			}
+			// a lane's slots aligned to their largest exponent: 53-bit mantissas, so five of them
+			// stay below 2^58
+			Fixed f[kTeamWarpSlots], t;
+			t.e = kFixedZero;
+#pragma unroll
+			for (int q = 0; q < kTeamWarpSlots; ++q)
+			{
+				f[q] = to_fixed(__longlong_as_double((long long)(u[q] & ~3ull)));
+				t.e = max(t.e, f[q].e);
+			}
+			t.m = 0;
+#pragma unroll
+			for (int q = 0; q < kTeamWarpSlots; ++q) t.m += (f[q].m >> 3) >> min(t.e - f[q].e, 60);
+			t.e += 3;
+			const double total = fixed_value(fixed_warp_sum(t));
+			const TV r = ratio_of(total);
+			if (FENCE)
+			{
+				const unsigned want = (fences + 1) * (unsigned)ctas;
 				while (ld_acquire(&mem->arrived) < want)
 					if (++polls > kPollLimit)
 					{
@@ -252,46 +304,25 @@ struct GridTeam
 						break;
 					}
 				there = __all_sync(0xffffffffu, there) != 0;
-#pragma unroll
-				for (int q = 0; q < kTeamWarpSlots; ++q) u[q] = lane + 32 * q < ctas ? ld_relaxed(mine + lane + 32 * q) : 0ull;
 			}
-			else
-				for (;;)
-				{
-					there = true;
-#pragma unroll
-					for (int q = 0; q < kTeamWarpSlots; ++q)
-					{
-						u[q] = lane + 32 * q < ctas ? ld_relaxed(mine + lane + 32 * q) : tag;
-						there = there && (u[q] & 3ull) == tag;
-					}
-					there = __all_sync(0xffffffffu, there) != 0;
-					if (there || ++polls > kPollLimit) break;
-				}
-			Fixed t = to_fixed(__longlong_as_double((long long)(VISIBLE ? u[0] : u[0] & ~3ull)));
-#pragma unroll
-			for (int q = 1; q < kTeamWarpSlots; ++q)
-				if (32 * q < ctas) t = fixed_add(t, to_fixed(__longlong_as_double((long long)(VISIBLE ? u[q] : u[q] & ~3ull))));
-			const double total = fixed_value(fixed_warp_sum(t));
-			const TV r = ratio_of(total);
 			if (lane == 0)
 			{
 				sh->total = total;
 				*(TV*)&sh->ratio = r;
-				sh->ok = there ? 1 : 0;
+				sh->ok = there && !sh->lost ? 1 : 0;
 			}
 		}
-		if (VISIBLE) ++published;
-		else ++plain;
+		++sums;
+		if (FENCE) ++fences;
 		__syncthreads();
 		ok = sh->ok;
 		ratio = *(const TV*)&sh->ratio;
 		return sh->total;
 	}
-	template <bool VISIBLE>
+	template <bool FENCE>
 	__device__ __forceinline__ double sum(Fixed v)
 	{
-		return sum<VISIBLE>(v, [] {}, [](double) { return (TV)0; });
+		return sum<FENCE>(v, [] {}, [](double) { return (TV)0; });
 	}
 	// execution and visibility only
 	__device__ __forceinline__ void publish()
@@ -302,6 +333,114 @@ struct GridTeam
 		sum<true>(z);
 	}
 };
+
+// A thread-block cluster of CL CTAs (or one CTA). Partials go straight into the slots of every CTA's
+// shared memory, where its warp 0 polls them: one trip through the cluster's network a sum. The
+// number's two bits work as in the grid team, over the team's whole life.
+template <class TV, int CL>
+struct ClusterTeam
+{
+	static constexpr bool kManyCtas = CL > 1;
+	SolveSh* sh;
+	int rank;
+	unsigned sums;
+	int ok;
+	TV ratio;
+	static constexpr int ctas = CL;
+
+	// (the caller synchronises the cluster after this)
+	__device__ __forceinline__ explicit ClusterTeam(SolveSh* s) : sh(s), rank(0), sums(0), ok(1), ratio((TV)0)
+	{
+		if (CL > 1) rank = (int)cooperative_groups::this_cluster().block_rank();
+		if (threadIdx.x < 2 * kMaxTeamCtas) (&sh->slot[0][0])[threadIdx.x] = 0ull;
+		if (threadIdx.x == 0) sh->lost = 0;
+	}
+	template <bool FENCE, class F, class R>
+	__device__ __forceinline__ double sum(Fixed v, F between, R ratio_of)
+	{
+		const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+		const int buf = sums & 1;
+		if (lane == 0) sh->w[buf][warp] = v;
+		__syncthreads();
+		const unsigned long long tag = (unsigned long long)(((sums >> 1) + 1) & 3);
+		double total = 0.0;
+		if (warp == 0)
+		{
+			total = cta_total(sh, buf, v);
+			if (CL > 1 && lane < CL)
+			{
+				const unsigned long long bits = ((unsigned long long)__double_as_longlong(total) & ~3ull) | tag;
+				unsigned remote;
+				asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+				             : "=r"(remote)
+				             : "r"((unsigned)__cvta_generic_to_shared(&sh->slot[buf][rank])), "r"(lane));
+				asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(bits) : "memory");
+			}
+		}
+		between();
+		if (FENCE && CL > 1) cooperative_groups::this_cluster().sync();
+		if (warp == 0)
+		{
+			bool there = true;
+			if (CL > 1)
+			{
+				unsigned long long u = tag;
+				const unsigned mine = (unsigned)__cvta_generic_to_shared(&sh->slot[buf][lane < CL ? lane : 0]);
+				for (int polls = 0;;)
+				{
+					if (lane < CL)
+						asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(u) : "r"(mine) : "memory");
+					there = __all_sync(0xffffffffu, (u & 3ull) == tag) != 0;
+					if (there || ++polls > 16 * kPollLimit) break;
+				}
+				total = fixed_value(fixed_warp_sum(to_fixed(__longlong_as_double((long long)(u & ~3ull)))));
+			}
+			const TV r = ratio_of(total);
+			if (lane == 0)
+			{
+				sh->total = total;
+				*(TV*)&sh->ratio = r;
+				sh->ok = there && !sh->lost ? 1 : 0;
+			}
+		}
+		++sums;
+		__syncthreads();
+		ok = sh->ok;
+		ratio = *(const TV*)&sh->ratio;
+		return sh->total;
+	}
+	template <bool FENCE>
+	__device__ __forceinline__ double sum(Fixed v)
+	{
+		return sum<FENCE>(v, [] {}, [](double) { return (TV)0; });
+	}
+	__device__ __forceinline__ void publish()
+	{
+		if (CL > 1) cooperative_groups::this_cluster().sync();
+		else __syncthreads();
+	}
+};
+
+// A vertex's s with the number of its version in the fourth component, as one 16-byte access each
+// way: the versions of a vector are told apart without a barrier.
+__device__ __forceinline__ float4 ld_version(const float* s, int i)
+{
+	unsigned long long lo, hi;
+	asm volatile("{ .reg .b128 t; ld.relaxed.gpu.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+	             : "=l"(lo), "=l"(hi)
+	             : "l"(s + 4 * (size_t)i)
+	             : "memory");
+	return make_float4(__uint_as_float((unsigned)lo), __uint_as_float((unsigned)(lo >> 32)), __uint_as_float((unsigned)hi),
+	                   __uint_as_float((unsigned)(hi >> 32)));
+}
+__device__ __forceinline__ void st_version(float* s, int i, const float o[3], unsigned version)
+{
+	const unsigned long long lo = (unsigned long long)__float_as_uint(o[0]) | ((unsigned long long)__float_as_uint(o[1]) << 32);
+	const unsigned long long hi = (unsigned long long)__float_as_uint(o[2]) | ((unsigned long long)version << 32);
+	asm volatile("{ .reg .b128 t; mov.b128 t, {%0, %1}; st.relaxed.gpu.global.b128 [%2], t; }" ::"l"(lo), "l"(hi),
+	             "l"(s + 4 * (size_t)i)
+	             : "memory");
+}
 
 // Where a slice's matrix comes from: shared memory (a chunk of nine planes and the column ids of
 // its w x 32 slots) or global memory with an L2 policy.
@@ -332,27 +471,88 @@ struct GlobalMat
 };
 
 // o = (A s)_i and own = s_i (the diagonal block leads every row); the products are summed in slot
-// order, as spmv_row sums them. DEPTH groups of four blocks have their columns' s in flight at a
-// time: the gathers go to L2, and a thread that waits for them group by group pays that trip four
-// times a row.
-template <class TA, class TV, int DEPTH, class M>
-__device__ __forceinline__ void team_spmv_row(const M& m, int w, int lane, const TV* s, TV o[3], TV own[3])
+// order, as spmv_row sums them. VERSIONED: s is a float vector whose entries carry their version;
+// entries older than `version` are read again (sh->lost: a wait ran out).
+// DEPTH groups of four blocks have their columns' s in flight at a time: the gathers go to L2, and a
+// thread that waits for them group by group pays that trip four times a row (matrix in shared
+// memory, few warps). With DEPTH 1 (many warps, matrix from L2) the column ids are read a group
+// ahead, so that a group's planes and gathers are in flight together.
+template <class TA, class TV, int DEPTH, bool VERSIONED, class M>
+__device__ __forceinline__ void team_spmv_row(const M& m, int w, int lane, const TV* s, unsigned version, SolveSh* sh,
+                                              TV o[3], TV own[3])
 {
 	typedef typename Acc<TA>::type AT;
 	AT o0 = 0, o1 = 0, o2 = 0;
+	int4 ahead;
+	if (DEPTH == 1) ahead = m.cols(4 * lane);
 	for (int k0 = 0; k0 < w; k0 += DEPTH * kGroup)
 	{
-		TV xv[DEPTH][4][3];
+		AT a[9][4];
+		int jj[DEPTH][4];
+		if (DEPTH == 1)
+		{
+#pragma unroll
+			for (int p = 0; p < 9; ++p) m.plane(p, 32 * k0 + 4 * lane, a[p]);
+		}
 #pragma unroll
 		for (int g = 0; g < DEPTH; ++g)
 			if (g == 0 || k0 + g * kGroup < w)
 			{
-				const int4 jj = m.cols(32 * (k0 + g * kGroup) + 4 * lane);
-				vld<TV, LdCG>(s, jj.x, xv[g][0]);
-				vld<TV, LdCG>(s, jj.y, xv[g][1]);
-				vld<TV, LdCG>(s, jj.z, xv[g][2]);
-				vld<TV, LdCG>(s, jj.w, xv[g][3]);
+				const int4 c = DEPTH == 1 ? ahead : m.cols(32 * (k0 + g * kGroup) + 4 * lane);
+				jj[g][0] = c.x;
+				jj[g][1] = c.y;
+				jj[g][2] = c.z;
+				jj[g][3] = c.w;
 			}
+		TV xv[DEPTH][4][3];
+		if constexpr (VERSIONED)
+		{
+			float4 r[DEPTH][4];
+#pragma unroll
+			for (int g = 0; g < DEPTH; ++g)
+				if (g == 0 || k0 + g * kGroup < w)
+#pragma unroll
+					for (int u = 0; u < 4; ++u) r[g][u] = ld_version(s, jj[g][u]);
+			if (DEPTH == 1 && k0 + kGroup < w) ahead = m.cols(32 * (k0 + kGroup) + 4 * lane);
+			for (int polls = 0;; ++polls)
+			{
+				bool old = false;
+#pragma unroll
+				for (int g = 0; g < DEPTH; ++g)
+					if (g == 0 || k0 + g * kGroup < w)
+#pragma unroll
+						for (int u = 0; u < 4; ++u)
+							if (__float_as_uint(r[g][u].w) != version)
+							{
+								r[g][u] = ld_version(s, jj[g][u]);
+								old = true;
+							}
+				if (!old) break;
+				if (polls > kPollLimit || *(volatile int*)&sh->lost)
+				{
+					sh->lost = 1;
+					break;
+				}
+			}
+#pragma unroll
+			for (int g = 0; g < DEPTH; ++g)
+#pragma unroll
+				for (int u = 0; u < 4; ++u)
+				{
+					xv[g][u][0] = r[g][u].x;
+					xv[g][u][1] = r[g][u].y;
+					xv[g][u][2] = r[g][u].z;
+				}
+		}
+		else
+		{
+#pragma unroll
+			for (int g = 0; g < DEPTH; ++g)
+				if (g == 0 || k0 + g * kGroup < w)
+#pragma unroll
+					for (int u = 0; u < 4; ++u) vld<TV, LdCG>(s, jj[g][u], xv[g][u]);
+			if (DEPTH == 1 && k0 + kGroup < w) ahead = m.cols(32 * (k0 + kGroup) + 4 * lane);
+		}
 		if (k0 == 0)
 		{
 #pragma unroll
@@ -362,9 +562,11 @@ __device__ __forceinline__ void team_spmv_row(const M& m, int w, int lane, const
 		for (int g = 0; g < DEPTH; ++g)
 			if (g == 0 || k0 + g * kGroup < w)
 			{
-				AT a[9][4];
+				if (DEPTH > 1)
+				{
 #pragma unroll
-				for (int p = 0; p < 9; ++p) m.plane(p, 32 * (k0 + g * kGroup) + 4 * lane, a[p]);
+					for (int p = 0; p < 9; ++p) m.plane(p, 32 * (k0 + g * kGroup) + 4 * lane, a[p]);
+				}
 #pragma unroll
 				for (int u = 0; u < 4; ++u)
 				{
@@ -496,19 +698,23 @@ struct OwnSlices
 	const TA* A;
 	int s0, ns, base0, vec_slices, mat_slices;
 	unsigned char *vec, *mat;
-	unsigned long long pol;
+	unsigned long long pol, keep_pol;
+	int keep_slices;  // local slices below it are kept in L2 (keep_pol), the others stream through it
 
-	__device__ __forceinline__ OwnSlices(const DevBody& body, const TA* a, unsigned char* smem, int room, int vecb)
+	__device__ __forceinline__ OwnSlices(const DevBody& body, const TA* a, unsigned char* smem, int room, int vecb, int keep,
+	                                     int rank, int ctas)
 	    : B(body), A(a)
 	{
-		s0 = (int)((long long)blockIdx.x * B.nslices / gridDim.x);
-		ns = (int)((long long)(blockIdx.x + 1) * B.nslices / gridDim.x) - s0;
+		s0 = (int)((long long)rank * B.nslices / ctas);
+		ns = (int)((long long)(rank + 1) * B.nslices / ctas) - s0;
 		vec_slices = min(ns, room / vecb);
 		vec = smem;
 		mat = smem + (size_t)vec_slices * vecb;
 		base0 = B.slice_ptr[s0];
 		mat_slices = 0;
 		pol = evict_first_policy();
+		keep_pol = keep < 1024 ? evict_last_policy() : evict_normal_policy();
+		keep_slices = (int)((long long)ns * keep >> 10);
 		if (vec_slices < ns) return;
 		const int cap = (room - vec_slices * vecb) / solve_slot_bytes<TA>();
 		int lo = 0, hi = ns;
@@ -562,7 +768,7 @@ struct OwnSlices
 			T t = (T)0;
 			if (i < B.n) t = f(j, i);
 			const Fixed w = fixed_warp_sum(to_fixed(t));
-			s = j < nw ? w : fixed_add(s, w);
+			s = fixed_add(s, fixed_norm(w.m, w.e));
 		}
 		return s;
 	}
@@ -573,7 +779,7 @@ struct OwnSlices
 		const int base = B.slice_ptr[s0 + j];
 		const int slots = B.slice_ptr[s0 + j + 1] - base;
 		if (j < mat_slices) f(SmemMat<TA>{mat + (size_t)(base - base0) * solve_slot_bytes<TA>(), slots}, slots / kSlice);
-		else f(GlobalMat<TA>{A, B.col, (size_t)B.nslots, (size_t)base, pol}, slots / kSlice);
+		else f(GlobalMat<TA>{A, B.col, (size_t)B.nslots, (size_t)base, j < keep_slices ? keep_pol : pol}, slots / kSlice);
 	}
 };
 
@@ -646,9 +852,10 @@ struct SolveEnd
 
 // What follows a solve: in a body step the final update (sparse_force_solver.cpp:194-223), which
 // with a single Newton iteration also ends the step, or else the Newton loop's exit test and, when
-// it ends, the step's end; then the statistics. rows(f) calls f(row i, dv) for this warp's rows.
-template <bool FILTER, class G, class R>
-__device__ __forceinline__ void team_end(G& T, const DevBody& B, const SolveArgs& P, const SolveEnd& S, R rows)
+// it ends, the step's end; then the statistics. rows(f) calls f(row i, dv) for this warp's rows,
+// update(i, dv, whether the step ends) is the final update of a row.
+template <class G, class R, class V>
+__device__ __forceinline__ void team_end(G& T, const DevBody& B, const SolveArgs& P, const SolveEnd& S, R rows, V update)
 {
 	Scalars* sc = B.sc;
 	const bool lead = T.rank == 0 && threadIdx.x == 0;
@@ -656,8 +863,9 @@ __device__ __forceinline__ void team_end(G& T, const DevBody& B, const SolveArgs
 	{
 		bool finish = P.newton_max == 1;
 		double part = 0.0;
-		rows([&](int i, float3 dv) { part += final_vertex_dv<LdPlain, FILTER>(B, i, P.h, P.newton == 0, finish, dv); });
-		const double err = T.template sum<false>(fixed_warp_sum(to_fixed(part)));
+		rows([&](int i, float3 dv) { part += update(i, dv, finish); });
+		const Fixed ws = fixed_warp_sum(to_fixed(part));
+		const double err = T.template sum<false>(fixed_norm(ws.m, ws.e));
 		const double err0 = P.newton == 0 ? err : sc->newton_err0;
 		const bool ndone = P.newton == 0 ? err <= P.newton_tol2 : err <= P.newton_tol2 * err0;
 		if (!finish && (ndone || !P.forces_left))
@@ -706,29 +914,52 @@ __device__ __forceinline__ bool solve_over(double delta0, double tol2, int max_i
 	return true;
 }
 
-template <class TA, class TV, bool FF, bool FILTER, int THREADS>
-__global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
+// Phases timed by the optional instrumentation of the batch kernels (cycles of thread 0 of each CTA,
+// barriers and reductions included in the phase that ends with them). The direction update runs
+// inside the SpMV sweep, so kPhDir stays zero; its slot keeps the numbering the host reads.
+enum { kPhElem = 0, kPhAsm = 1, kPhSpmv = 2, kPhUpdate = 3, kPhDir = 4, kPhFinal = 5, kPhIdle = 6, kPhases = 8 };
+
+// The PCG of one body by one team (sparse_solver.cpp:57-108) and what follows it. update: team_end;
+// tick(phase): the phase's end.
+template <class TA, class TV, bool FF, int DEPTH, class Team, class V, class C>
+__device__ __forceinline__ void team_solve(Team& T, const DevBody& B, const SolveArgs& P, unsigned char* smem, V update, C tick)
 {
-	extern __shared__ __align__(16) unsigned char smem[];
-	__shared__ SolveSh sh;
-	if (P.newton > 0 && B.sc->newton_done) return;
 	typedef RowVecs<TV, FF> Row;
-	constexpr int kDepth = THREADS <= 256 ? (sizeof(TV) == 8 ? 2 : 4) : (THREADS <= 512 && sizeof(TV) == 4 ? 2 : 1);
 	const int lane = threadIdx.x & 31;
-	GridTeam<TV> T(&sh, B.team);
 	const OwnSlices<TA> O(B, sizeof(TA) == sizeof(float) ? (const TA*)B.A32 : (const TA*)B.Alo, smem, P.smem,
-	                      solve_vec_bytes<TV, FF>());
+	                      solve_vec_bytes<TV, FF>(), P.keep, T.rank, T.ctas);
 	const TV* sv = (const TV*)B.s;
-	if (blockIdx.x == 0 && threadIdx.x == 0 && P.newton <= 0) B.sc->fault = 0;
+	// FP32 vectors: s carries its version, 0 as the assembly leaves it; FP64: every new s is fenced
+	constexpr bool kVersions = sizeof(TV) == 4 && Team::kManyCtas;
+	constexpr bool kFence = !kVersions;
+	// BF16 blocks: the refresh uses the FP32 ones, and a residual that met the tolerance is confirmed
+	// by a refresh before the solve ends
+	constexpr bool kConfirm = sizeof(TA) == 2;
+	bool confirm = false;
+	unsigned version = 0;
+	auto store_s = [&](int i, const TV* o) {
+		if constexpr (kVersions) st_version((float*)B.s, i, o, version);
+		else vst((TV*)B.s, i, o);
+	};
+	if (T.rank == 0 && threadIdx.x == 0 && P.newton <= 0) B.sc->fault = 0;
 	auto row = [&](int j, int i) { return Row(B, O.vec, j, O.vec_slices, lane, i); };
 
+	auto refresh_matrix = [&](int j, auto f) {
+		if constexpr (kConfirm)
+		{
+			const int base = B.slice_ptr[O.s0 + j];
+			f(GlobalMat<float>{B.A32, B.col, (size_t)B.nslots, (size_t)base, O.pol}, (B.slice_ptr[O.s0 + j + 1] - base) / kSlice);
+		}
+		else
+			O.matrix(j, f);
+	};
 	// r = b - A x and s = M^-1 r with x in global memory; this warp's part of r.s
 	auto residual = [&]() -> Fixed {
 		return O.template row_sum<TV>([&](int j, int i) {
 			const Row v = row(j, i);
 			TV b[3], rr[3], ss[3];
 			vld<TV, LdPlain>((const TV*)B.pb, i, b);
-			O.matrix(j, [&](const auto& m, int w) {
+			refresh_matrix(j, [&](const auto& m, int w) {
 				if constexpr (FF)
 				{
 					float qh[3], ql[3];
@@ -739,14 +970,14 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
 				else
 				{
 					TV q[3], own[3];
-					team_spmv_row<TA, TV, kDepth>(m, w, lane, (const TV*)B.py, q, own);
+					team_spmv_row<typename std::conditional<kConfirm, float, TA>::type, TV, DEPTH, false>(m, w, lane, (const TV*)B.py, 0u, T.sh, q, own);
 #pragma unroll
 					for (int c = 0; c < 3; ++c) rr[c] = b[c] - q[c];
 				}
 			});
 			row_precond<TV>(B, v.m, i, rr, ss);
 			vst(v.r, 0, rr);
-			vst((TV*)B.s, i, ss);
+			store_s(i, ss);
 			return term3(rr, ss);
 		});
 	};
@@ -812,13 +1043,18 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
 		else vst(v.x, 0, zero);
 		return term3(t, ss);
 	});
-	if (P.warm) part = residual();
+	if (P.warm)
+	{
+		// the earlier s may carry any version: fenced once
+		++version;
+		part = residual();
+		T.publish();
+	}
 	SolveEnd S;
 	S.iter = 0;
-	S.delta = S.delta0 = T.template sum<true>(part);
+	S.delta = S.delta0 = T.template sum<false>(part);
 	bool done = solve_over(S.delta0, P.tol2, P.max_iter, S.status);
 	const double enough = P.tol2 * S.delta0;
-	auto beta_of = [&](double t) { return quotient(t, S.delta, (TV)0); };
 	TV beta = (TV)0;
 	while (!done && T.ok)
 	{
@@ -826,7 +1062,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
 		part = O.template row_sum<TV>([&](int j, int i) {
 			const Row v = row(j, i);
 			TV o[3], dn[3];
-			O.matrix(j, [&](const auto& m, int w) { team_spmv_row<TA, TV, kDepth>(m, w, lane, sv, o, dn); });
+			O.matrix(j, [&](const auto& m, int w) { team_spmv_row<TA, TV, DEPTH, kVersions>(m, w, lane, sv, version, T.sh, o, dn); });
 			if (!first)
 			{
 				TV dp[3], qp[3];
@@ -843,7 +1079,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
 			vst(v.d, 0, dn);
 			return term3(dn, o);
 		});
-		const double dq = T.template sum<false>(part, [] {}, [&](double t) { return quotient(S.delta, t, (TV)0); });
+		const double dq = T.template sum<false>(part, [] {}, [&](double t) { return Divisor<TV>(t).divide(S.delta); });
+		tick(kPhSpmv);
 		if (!T.ok) break;
 		if (!bits_finite(dq))
 		{
@@ -856,18 +1093,24 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
 			break;
 		}
 		const TV alpha = T.ratio;
+		const Divisor<TV> by_delta(S.delta);
+		auto beta_of = [&](double t) { return by_delta.divide(t); };
 		double dn;
-		if (P.refresh > 0 && (S.iter % P.refresh) == 0)
+		const bool refresh = (P.refresh > 0 && (S.iter % P.refresh) == 0) || (kConfirm && confirm);
+		if (refresh)
 		{
 			// sparse_solver.cpp:83-90: r = b - A x
 			update_x(alpha);
 			publish_x();
 			T.publish();
 			if (!T.ok) break;
-			dn = T.template sum<true>(residual(), [] {}, beta_of);
+			++version;
+			part = residual();
+			dn = T.template sum<kFence>(part, [] {}, beta_of);
 		}
 		else
 		{
+			++version;
 			part = O.template row_sum<TV>([&](int j, int i) {
 				const Row v = row(j, i);
 				TV r[3], q[3], s[3];
@@ -877,18 +1120,23 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
 				for (int c = 0; c < 3; ++c) r[c] -= alpha * q[c];
 				row_precond<TV>(B, v.m, i, r, s);
 				vst(v.r, 0, r);
-				vst((TV*)B.s, i, s);
+				store_s(i, s);
 				return term3(r, s);
 			});
-			dn = T.template sum<true>(part, [&] { update_x(alpha); }, beta_of);
+			dn = T.template sum<kFence>(part, [&] { update_x(alpha); }, beta_of);
 		}
+		tick(kPhUpdate);
 		beta = T.ratio;
 		S.delta = dn;
 		S.iter += 1;
 		if (!bits_finite(dn)) S.status = B3G_SOLVE_NONFINITE;
-		else if (bits_at_most(dn, enough)) S.status = B3G_SOLVE_CONVERGED;
+		else if (bits_at_most(dn, enough) && (!kConfirm || refresh)) S.status = B3G_SOLVE_CONVERGED;
 		else if (S.iter >= P.max_iter) S.status = B3G_SOLVE_MAX_ITERATIONS;
-		else continue;
+		else
+		{
+			if (kConfirm) confirm = bits_at_most(dn, enough);
+			continue;
+		}
 		break;
 	}
 	if (!T.ok)
@@ -897,9 +1145,25 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
 		return;
 	}
 	if (P.newton < 0 || P.forces_left) publish_x();  // the result, or the next iteration's start
-	team_end<FILTER>(T, B, P, S, [&](auto f) {
+	team_end(T, B, P, S, [&](auto f) {
 		O.rows([&](int j, int i) { f(i, row_dv<TV, FF>(row(j, i).x)); });
-	});
+	}, update);
+	tick(kPhFinal);
+}
+
+
+template <class TA, class TV, bool FF, bool FILTER, int THREADS>
+__global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
+{
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ SolveSh sh;
+	if (P.newton > 0 && B.sc->newton_done) return;
+	constexpr int kDepth = THREADS <= 256 ? (sizeof(TV) == 8 ? 2 : 4) : 1;
+	GridTeam<TV> T(&sh, B.team);
+	team_solve<TA, TV, FF, kDepth>(
+	    T, B, P, smem,
+	    [&](int i, float3 dv, bool finish) { return final_vertex_dv<LdPlain, FILTER>(B, i, P.h, P.newton == 0, finish, dv); },
+	    [](int) {});
 }
 
 // The BF16 mode's solve: a flexible CG (Notay's, one stored direction) on the FP32 blocks, with
@@ -914,12 +1178,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 	__shared__ SolveSh sh;
 	if (P.newton > 0 && B.sc->newton_done) return;
 	typedef FcgRowVecs Row;
-	constexpr int kDepth = THREADS <= 256 ? 4 : (THREADS <= 512 ? 2 : 1);
+	constexpr int kDepth = THREADS <= 256 ? 4 : 1;
 	typedef __nv_bfloat16 TA;
 	const int lane = threadIdx.x & 31;
 	GridTeam<float> T(&sh, B.team);
-	const OwnSlices<TA> O(B, (const TA*)B.Alo, smem, P.smem, kFcgVecBytes);
+	const OwnSlices<TA> O(B, (const TA*)B.Alo, smem, P.smem, kFcgVecBytes, P.keep, T.rank, T.ctas);
 	const float* sv = (const float*)B.s;
+	unsigned version = 0;  // of s
 	const float* pv = (const float*)B.d2;
 	if (blockIdx.x == 0 && threadIdx.x == 0 && P.newton <= 0) B.sc->fault = 0;
 	auto row = [&](int j, int i) { return Row(B, W, O.vec, j, O.vec_slices, lane, i); };
@@ -977,23 +1242,26 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 	if (P.warm) part = residual();
 	SolveEnd S;
 	S.iter = 0;
-	S.delta = S.delta0 = T.sum<true>(part);
+	S.delta = S.delta0 = T.sum<false>(part);
 	bool done = solve_over(S.delta0, P.tol2, P.max_iter, S.status);
 	double pq_prev = 0.0;
 	while (!done && T.ok)
 	{
 		// inner solve: r, s = M^-1 r, z = 0
+		++version;
 		part = O.row_sum<float>([&](int j, int i) {
 			const Row v = row(j, i);
 			float r[3], s[3];
 			vld<float, LdPlain>(v.r, 0, r);
 			row_precond<float>(B, v.m, i, r, s);
 			vst(v.ri, 0, r);
-			vst((float*)B.s, i, s);
+			st_version((float*)B.s, i, s, version);
 			vst(v.z, 0, zero);
 			return term3(r, s);
 		});
-		double delta = T.sum<true>(part);
+		// a warm start finds an s of any version: fenced once
+		if (P.warm && S.iter == 0) T.publish();
+		double delta = T.sum<false>(part);
 		if (!T.ok) break;
 		float beta = 0.0f;
 		if (isfinite(delta) && delta > 0.0)
@@ -1002,7 +1270,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 				part = O.row_sum<float>([&](int j, int i) {
 					const Row v = row(j, i);
 					float o[3], dn[3];
-					O.matrix(j, [&](const auto& m, int w) { team_spmv_row<TA, float, kDepth>(m, w, lane, sv, o, dn); });
+					O.matrix(j, [&](const auto& m, int w) { team_spmv_row<TA, float, kDepth, true>(m, w, lane, sv, version, &sh, o, dn); });
 					if (it > 0)
 					{
 						float dp[3], qp[3];
@@ -1019,9 +1287,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 					vst(v.di, 0, dn);
 					return term3(dn, o);
 				});
-				const double dq = T.sum<false>(part, [] {}, [&](double t) { return quotient(delta, t, 0.0f); });
+				const double dq = T.sum<false>(part, [] {}, [&](double t) { return Divisor<float>(t).divide(delta); });
 				if (!T.ok || !bits_finite(dq) || !bits_positive(dq)) break;
 				const float alpha = T.ratio;
+				const Divisor<float> by_delta(delta);
+				++version;
 				part = O.row_sum<float>([&](int j, int i) {
 					const Row v = row(j, i);
 					float r[3], q[3], s[3];
@@ -1031,15 +1301,15 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 					for (int c = 0; c < 3; ++c) r[c] -= alpha * q[c];
 					row_precond<float>(B, v.m, i, r, s);
 					vst(v.ri, 0, r);
-					vst((float*)B.s, i, s);
+					st_version((float*)B.s, i, s, version);
 					return term3(r, s);
 				});
-				const double dn = T.sum<true>(part, [&] {
+				const double dn = T.sum<false>(part, [&] {
 					O.rows([&](int j, int i) {
 						const Row v = row(j, i);
 						row_x_update<float, false>(v.z, v.di, alpha);
 					});
-				}, [&](double t) { return quotient(t, delta, 0.0f); });
+				}, [&](double t) { return by_delta.divide(t); });
 				if (!T.ok) break;
 				beta = T.ratio;
 				delta = dn;
@@ -1080,7 +1350,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 		part = O.row_sum<float>([&](int j, int i) {
 			const Row v = row(j, i);
 			float o[3], p[3];
-			matrix32(j, [&](const auto& m, int w) { team_spmv_row<float, float, kDepth>(m, w, lane, pv, o, p); });
+			matrix32(j, [&](const auto& m, int w) { team_spmv_row<float, float, kDepth, false>(m, w, lane, pv, 0u, &sh, o, p); });
 			vst(v.q, 0, o);
 			return term3(p, o);
 		});
@@ -1142,9 +1412,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 		return;
 	}
 	if (P.newton < 0 || P.forces_left) publish_x();
-	team_end<FILTER>(T, B, P, S, [&](auto f) {
-		O.rows([&](int j, int i) { f(i, row_dv<float, true>(row(j, i).x)); });
-	});
+	team_end(
+	    T, B, P, S,
+	    [&](auto f) { O.rows([&](int j, int i) { f(i, row_dv<float, true>(row(j, i).x)); }); },
+	    [&](int i, float3 dv, bool finish) { return final_vertex_dv<LdPlain, FILTER>(B, i, P.h, P.newton == 0, finish, dv); });
 }
 
 } // namespace
