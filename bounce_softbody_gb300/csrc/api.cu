@@ -384,13 +384,16 @@ int b3g_context_create(int device, b3g_context** out)
 	if (!c) return fail(B3G_ERROR_OUT_OF_MEMORY, "context");
 	c->device = device;
 	e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
-	if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_scalars, sizeof(Scalars) * 1024);
+	// one page-locked block: the scalars, then the hits of small ray casts
+	static_assert(sizeof(Scalars) % alignof(b3g_ray_hit) == 0, "the hits follow the scalars");
+	if (e == cudaSuccess) e = cudaMallocHost((void**)&c->h_scalars, sizeof(Scalars) * 1024 + sizeof(b3g_ray_hit) * kRayPick);
 	if (e != cudaSuccess)
 	{
 		if (c->stream) cudaStreamDestroy(c->stream);
 		delete c;
 		return cuda_fail(e, "context setup");
 	}
+	c->h_hits = (b3g_ray_hit*)(c->h_scalars + 1024);
 	cudaDeviceProp prop;
 	if (cudaGetDeviceProperties(&prop, device) == cudaSuccess) c->sm_count = prop.multiProcessorCount;
 	*out = c;
@@ -642,6 +645,7 @@ int b3g_body_create(b3g_context* ctx, const b3g_body_desc* d, b3g_body** out)
 		D.sc = C.take<Scalars>(1);
 		D.team = C.take<TeamMemory>(1);
 		b->staging = C.take<float>(3 * (size_t)n);
+		b->ray_scratch = C.take<RayScratch>(1);
 	};
 	DevBody D{};
 	Carver sizer;
@@ -1075,6 +1079,15 @@ int b3g_body_ray_cast(b3g_body* b, const float* segments, uint32_t count, b3g_ra
 		if (!std::isfinite(segments[k])) return fail(B3G_ERROR_INVALID_ARGUMENT, "segment %u is not finite", (uint32_t)(k / 6));
 	cudaSetDevice(b->ctx->device);
 	cudaStream_t st = b->ctx->stream;
+	if (count <= kRayPick)
+	{
+		std::lock_guard<std::mutex> lock(b->ctx->ray_mutex);
+		cudaError_t e = op_ray_pick(b->d, (int)b->ntr_fix, segments, count, b->ray_scratch, b->ctx->h_hits, st);
+		if (e == cudaSuccess) e = cudaStreamSynchronize(st);
+		if (e != cudaSuccess) return cuda_fail(e, "ray cast");
+		std::memcpy(hits, b->ctx->h_hits, sizeof(b3g_ray_hit) * (size_t)count);
+		return B3G_OK;
+	}
 	auto layout = [](uint32_t cap, size_t* off_keys, size_t* off_hits) {
 		*off_keys = align_up(6 * sizeof(float) * (size_t)cap);
 		*off_hits = *off_keys + align_up(sizeof(unsigned long long) * (size_t)cap);

@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include <mutex>
 #include <vector>
 
 struct BatchCache;
@@ -20,6 +21,8 @@ struct b3g_context
 	int sm_count = 0;
 	cudaStream_t stream = nullptr;
 	b3g::Scalars* h_scalars = nullptr;   // pinned, 1024 entries
+	b3g_ray_hit* h_hits = nullptr;       // pinned, kRayPick entries; one ray cast at a time (ray_mutex)
+	std::mutex ray_mutex;
 	BatchCache* batch = nullptr;
 	// b3g_batch_set_launch_timing: batched steps launch directly (no graph) with events around
 	// the assembly and PCG launches; device milliseconds accumulate here
@@ -93,6 +96,7 @@ struct b3g_body
 	char* arena = nullptr;
 	size_t arena_bytes = 0;
 	float* staging = nullptr;            // 3 floats per vertex of upload space
+	b3g::RayScratch* ray_scratch = nullptr;  // of small ray casts, in the arena (zero between calls)
 	b3g::PrecBuffers prec[3];
 	// host copies needed by ResetMass / SetType
 	std::vector<int32_t> h_type;

@@ -5,7 +5,7 @@
 #include "ops.h"
 
 #include <cstdlib>
-#include <utility>
+#include <cstring>
 
 #include <algorithm>
 
@@ -124,12 +124,9 @@ __global__ void __launch_bounds__(kThreads) k_ray_cast(DevBody B, int ntri, cons
 	}
 }
 
-// One thread per segment: the winner's normal, oriented as the reference orients it.
-__global__ void k_ray_finish(DevBody B, const float* __restrict__ seg, unsigned count,
-                             const unsigned long long* __restrict__ keys, b3g_ray_hit* hits)
+// A segment's hit from its key: the winner's normal, oriented as the reference orients it.
+__device__ __forceinline__ b3g_ray_hit ray_hit(const DevBody& B, float3 p1, float3 d, unsigned long long key)
 {
-	const unsigned r = blockIdx.x * blockDim.x + threadIdx.x;
-	if (r >= count) return;
 	b3g_ray_hit o;
 	o.hit = 0;
 	o.triangle = 0;
@@ -153,7 +150,56 @@ __global__ void k_ray_finish(DevBody B, const float* __restrict__ seg, unsigned 
 		o.normal[1] = n.y;
 		o.normal[2] = n.z;
 	}
-	hits[r] = o;
+	return o;
+}
+
+// One thread per segment
+__global__ void k_ray_finish(DevBody B, const float* __restrict__ seg, unsigned count,
+                             const unsigned long long* __restrict__ keys, b3g_ray_hit* hits)
+{
+	const unsigned r = blockIdx.x * blockDim.x + threadIdx.x;
+	if (r >= count) return;
+	const float3 p1 = f3(seg[6 * r], seg[6 * r + 1], seg[6 * r + 2]);
+	hits[r] = ray_hit(B, p1, f3(seg[6 * r + 3], seg[6 * r + 4], seg[6 * r + 5]) - p1, keys[r]);
+}
+
+// A few segments in one launch: they come in the kernel's parameters, the last CTA of a segment writes
+// its hit, and keys (kept inverted, so that zero is "no hit yet") and arrival counters are left at
+// zero for the next call. A pick is all latency: a copy, a memset, two launches and a copy back
+// took 45 us a call from Python for 8 segments on 18432 triangles, the kernels 9 of them.
+__global__ void __launch_bounds__(kThreads) k_ray_pick(DevBody B, int ntri, RaySegments S, RayScratch* w, b3g_ray_hit* hits)
+{
+	const int lane = threadIdx.x & 31, r = blockIdx.y;
+	const float* seg = S.s[r];
+	const float3 p1 = f3(seg[0], seg[1], seg[2]);
+	const float3 d = f3(seg[3], seg[4], seg[5]) - p1;
+	unsigned long long best = 0ull;
+	for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < ntri; e += gridDim.x * blockDim.x)
+	{
+		const uint4 id = B.tri[e];
+		float t, num;
+		float3 n;
+		if (ray_triangle(p1, d, ld3(B.x, id.x), ld3(B.x, id.y), ld3(B.x, id.z), t, num, n))
+		{
+			const unsigned long long key = ~ray_key(t, (unsigned)e);
+			best = key > best ? key : best;
+		}
+	}
+#pragma unroll
+	for (int o = 16; o > 0; o >>= 1)
+	{
+		const unsigned long long other = __shfl_xor_sync(0xffffffffu, best, o);
+		best = other > best ? other : best;
+	}
+	if (lane == 0 && best) atomicMax(&w->key[r], best);
+	__syncthreads();
+	if (threadIdx.x != 0) return;
+	__threadfence();
+	if (atomicAdd(&w->arrived[r], 1u) != gridDim.x - 1) return;
+	__threadfence();
+	const unsigned long long key = ~atomicExch(&w->key[r], 0ull);
+	w->arrived[r] = 0u;
+	hits[r] = ray_hit(B, p1, d, key);
 }
 
 // Filtered contacts: the contact update and each vertex's constraint at the start of a step
@@ -254,6 +300,19 @@ int vertex_grid(const DevBody& B)
 
 } // namespace
 
+// CTAs over the triangles: enough to fill the GPU for one segment, fewer per segment when there are
+// many segments
+static int ray_ctas(int ntri, uint32_t count)
+{
+	static const int sms = [] {
+		int dev = 0, n = 0;
+		cudaGetDevice(&dev);
+		cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+		return n > 0 ? n : 1;
+	}();
+	return std::max(1, std::min(grid_for(ntri, kThreads), 4 * sms / (int)std::min<uint32_t>(count, 64)));
+}
+
 cudaError_t op_ray_cast(const DevBody& B, int ntri, const float* segments, uint32_t count, unsigned long long* keys,
                         b3g_ray_hit* hits, cudaStream_t st)
 {
@@ -262,19 +321,22 @@ cudaError_t op_ray_cast(const DevBody& B, int ntri, const float* segments, uint3
 	if (e != cudaSuccess) return e;
 	if (ntri > 0)
 	{
-		// enough CTAs over the triangles to fill the GPU for one segment, fewer per segment when
-		// there are many segments
-		static const int sms = [] {
-			int dev = 0, n = 0;
-			cudaGetDevice(&dev);
-			cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
-			return n > 0 ? n : 1;
-		}();
-		const int per_seg = std::max(1, std::min(grid_for(ntri, kThreads), 4 * sms / (int)std::min<uint32_t>(count, 64)));
+		const int per_seg = ray_ctas(ntri, count);
 		dim3 grid((unsigned)per_seg, std::min<uint32_t>(count, 65535u));
 		k_ray_cast<<<grid, kThreads, 0, st>>>(B, ntri, segments, count, keys);
 	}
 	k_ray_finish<<<(count + 127) / 128, 128, 0, st>>>(B, segments, count, keys, hits);
+	return cudaGetLastError();
+}
+
+cudaError_t op_ray_pick(const DevBody& B, int ntri, const float* segments, uint32_t count, RayScratch* scratch,
+                        b3g_ray_hit* hits, cudaStream_t st)
+{
+	if (count == 0) return cudaSuccess;
+	RaySegments S;
+	std::memcpy(S.s, segments, 6 * sizeof(float) * (size_t)count);
+	const dim3 grid((unsigned)ray_ctas(ntri, count), count);
+	k_ray_pick<<<grid, kThreads, 0, st>>>(B, ntri, S, scratch, hits);
 	return cudaGetLastError();
 }
 

@@ -91,6 +91,21 @@ cudaError_t op_batch_gather(const XferBody* table, uint32_t count, uint32_t max_
 cudaError_t op_ray_cast(const DevBody& B, int ntri, const float* segments, uint32_t count, unsigned long long* keys,
                         b3g_ray_hit* hits, cudaStream_t st);
 
+// The same for up to kRayPick segments (host) in one launch. scratch: zero before the first call, left
+// zero; hits may be page-locked host memory.
+constexpr uint32_t kRayPick = 64;
+struct RaySegments
+{
+	float s[kRayPick][6];
+};
+struct RayScratch
+{
+	unsigned long long key[kRayPick];
+	unsigned arrived[kRayPick];
+};
+cudaError_t op_ray_pick(const DevBody& B, int ntri, const float* segments, uint32_t count, RayScratch* scratch,
+                        b3g_ray_hit* hits, cudaStream_t st);
+
 // Persistent batch kernel: every body listed in `big` (teams of `cluster` CTAs) and in `small`
 // (one CTA each) steps `steps` times in one launch.
 struct BatchArgs
