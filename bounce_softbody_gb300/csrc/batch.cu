@@ -39,6 +39,8 @@ struct BatchCache
 	int lpt = 0;                 // queues ordered by estimated solve time (1) or by size (0)
 	int cluster = 1;
 	int threshold = 1 << 30;
+	int per = 0;                 // slices a CTA of a body's team should have (0: teams by threshold)
+	int tier_end[kTiers] = {};
 	int nbig = 0;
 	int ctas = 0;
 	bool tuned = false;
@@ -89,6 +91,7 @@ BatchArgs make_args(BatchCache* c, float h, int steps, const b3g_solver_config& 
 	A.small = c->d_order + c->nbig;
 	A.nsmall = (int)c->order.size() - c->nbig;
 	A.queue = c->d_queue;
+	std::copy(c->tier_end, c->tier_end + kTiers, A.tier_end);
 	A.steps = steps;
 	A.h = h;
 	A.newton = (int)std::max<uint32_t>(1u, cfg.force_iterations);
@@ -114,43 +117,64 @@ BatchArgs make_args(BatchCache* c, float h, int steps, const b3g_solver_config& 
 	return A;
 }
 
-// Estimated solve time of body k on a team of `warps` warps, in units of one warp's pass over one
-// slice: every PCG iteration is a sweep of ceil(slices / warps) passes plus about two passes'
-// worth of team barriers and reductions. Iteration counts come from a step already taken; before
-// one is known every body counts one iteration, so the order is by size.
-double est_time(const BatchCache* c, int k, int warps)
+// CTAs of body k's team in the solve launch
+int team_width(const BatchCache* c, int k)
+{
+	if (c->per <= 0) return c->cluster > 1 && (int)c->bodies[k]->n >= c->threshold ? c->cluster : 1;
+	const int slices = ((int)c->bodies[k]->n + kSlice - 1) / kSlice;
+	int w = 1;
+	while (w < c->cluster && slices > c->per * w) w *= 2;
+	return w;
+}
+
+// Estimated solve time of body k on a team of `width` CTAs, in units of a CTA's pass over one slice:
+// a sweep of ceil(slices / width) passes an iteration and about eleven passes' worth of team sums
+// and latency. Iteration counts come from a step already taken; before one is known every body
+// counts one iteration, so the order is by size.
+double est_time(const BatchCache* c, int k, int width)
 {
 	const double slices = std::ceil((double)c->bodies[k]->n / kSlice);
 	const double it = c->iters.empty() || c->iters[k] <= 0 ? 1.0 : (double)c->iters[k];
-	return it * (2.0 + std::ceil(slices / warps));
+	return it * (11.0 + std::ceil(slices / width));
 }
 
-// Bodies of at least `threshold` vertices are stepped by clusters of `cluster` CTAs, the others by
-// single CTAs. Each queue runs largest first, or with lpt longest estimated solve first
+// The solve launch's schedule: clusters of `cluster` CTAs; with per > 0 a body's team is the part of
+// a cluster (a power of two) that gives each CTA about `per` slices, else the whole cluster for
+// bodies of at least `threshold` vertices and one CTA for the others. Wide teams run first; within
+// a width the queue runs largest first, or with lpt longest estimated solve first
 // (longest-processing-time order), so that a small body with many PCG iterations does not start
 // last and trail the launch; the autotuner tries both.
-void set_schedule(BatchCache* c, int cluster, int threshold, int sms, cudaStream_t st, int lpt = 0)
+void set_schedule(BatchCache* c, int cluster, int threshold, int sms, cudaStream_t st, int lpt = 0, int per = 0)
 {
 	c->cluster = cluster;
 	c->threshold = threshold;
 	c->lpt = lpt;
-	constexpr int kCtaWarps = 8;  // warps of one CTA of the PCG launch
-	std::vector<int> big, small;
-	for (int k = 0; k < (int)c->bodies.size(); ++k)
-		((cluster > 1 && (int)c->bodies[k]->n >= threshold) ? big : small).push_back(k);
-	auto by_time = [&](std::vector<int>& v, int warps) {
-		std::vector<double> t(c->bodies.size());
-		for (int k : v) t[k] = lpt ? est_time(c, k, warps) : (double)c->bodies[k]->n;
-		std::stable_sort(v.begin(), v.end(), [&](int a, int b) {
-			if (t[a] != t[b]) return t[a] > t[b];
-			return c->bodies[a]->n > c->bodies[b]->n;
-		});
-	};
-	by_time(big, kCtaWarps * cluster);
-	by_time(small, kCtaWarps);
-	c->order = big;
-	c->order.insert(c->order.end(), small.begin(), small.end());
-	c->nbig = (int)big.size();
+	c->per = per;
+	const int count = (int)c->bodies.size();
+	std::vector<int> width(count);
+	std::vector<double> t(count);
+	for (int k = 0; k < count; ++k)
+	{
+		width[k] = team_width(c, k);
+		t[k] = lpt ? est_time(c, k, width[k]) : (double)c->bodies[k]->n;
+	}
+	c->order.resize(count);
+	std::iota(c->order.begin(), c->order.end(), 0);
+	std::stable_sort(c->order.begin(), c->order.end(), [&](int a, int b) {
+		if (width[a] != width[b]) return width[a] > width[b];
+		if (t[a] != t[b]) return t[a] > t[b];
+		return c->bodies[a]->n > c->bodies[b]->n;
+	});
+	auto at_least = [&](int w) { return (int)std::count_if(width.begin(), width.end(), [&](int x) { return x >= w; }); };
+	for (int k = 0; k < kTiers; ++k) c->tier_end[k] = at_least(kMaxTeamCtas >> k);
+	c->nbig = at_least(2);
+	if (per > 0)
+	{
+		// the smallest body on more than one CTA, for the record
+		c->threshold = 1 << 30;
+		for (int k = 0; k < count; ++k)
+			if (width[k] > 1) c->threshold = std::min(c->threshold, (int)c->bodies[k]->n);
+	}
 	c->ctas = schedule_ctas(c->prec, cluster, sms);
 	if (!c->order.empty())
 		cudaMemcpyAsync(c->d_order, c->order.data(), c->order.size() * sizeof(int), cudaMemcpyHostToDevice, st);
@@ -225,34 +249,26 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 	std::vector<Snapshot> L = snapshot_list(c, store, &total);
 	for (const Snapshot& s : L) cudaMemcpyAsync(s.dst, s.src, s.bytes, cudaMemcpyDeviceToDevice, st);
 
-	int maxn = 0;
-	for (b3g_body* b : c->bodies) maxn = std::max(maxn, (int)b->n);
-	// candidates: (cluster size, size threshold of cluster-stepped bodies, queue order)
+	// candidates: (cluster size, slices per CTA of a team, queue order)
 	struct Cand
 	{
-		int cl, thr, lpt;
+		int cl, per, lpt;
 	};
 	std::vector<Cand> cands;
-	cands.push_back({1, 1 << 30, 0});
-	cands.push_back({1, 1 << 30, 1});
-	// threshold 1: every body stepped by a cluster. Small bodies on single CTAs run after the
-	// clusters have drained the queue of large ones and can trail the launch; on a cluster they
-	// take their turn in the same queue (512-body batch: PCG launch 28.6 -> 27.9 ms)
-	const int thresholds[] = {1, 1024, 2048, 4096, 8192, 16384, 32768};
-	const int clusters[] = {2, 4, 8, 16};
+	const int clusters[] = {16, 8, 4};
+	const int pers[] = {2, 4, 8, 16, 32, 64};
 	for (int cl : clusters)
 		if (batch_max_clusters(c->prec, cl) > 0)  // 16-CTA clusters need hardware support
-			for (int t : thresholds)
-				if (t <= maxn)
-					for (int o = 0; o < 2; ++o) cands.push_back({cl, t, o});
+			for (int p : pers)
+				for (int o = 0; o < 2; ++o) cands.push_back({cl, p, o});
 	cudaEvent_t e0, e1;
 	cudaEventCreate(&e0);
 	cudaEventCreate(&e1);
 	float best = 1e30f;
-	Cand best_c = {c->cluster, c->threshold, c->lpt};
-	for (auto& cd : cands)
+	Cand best_c = {0, 0, 0};
+	for (const Cand& cd : cands)
 	{
-		set_schedule(c, cd.cl, cd.thr, ctx->sm_count, st, cd.lpt);
+		set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per);
 		BatchArgs A = make_args(c, h, 1, cfg);
 		e = run_once(c, A, st);  // warm-up
 		if (e == cudaSuccess && c->iters.empty())
@@ -265,7 +281,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 				e = cudaErrorUnknown;
 				break;
 			}
-			set_schedule(c, cd.cl, cd.thr, ctx->sm_count, st, cd.lpt);
+			set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per);
 			A = make_args(c, h, 1, cfg);
 		}
 		for (const Snapshot& s : L) cudaMemcpyAsync((void*)s.src, s.dst, s.bytes, cudaMemcpyDeviceToDevice, st);
@@ -277,7 +293,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 		if (e != cudaSuccess) break;
 		float ms = 0.0f;
 		cudaEventElapsedTime(&ms, e0, e1);
-		c->tune_log.push_back({cd.lpt * 100000000 + cd.cl * 1000000 + std::min(cd.thr, 999999), (double)ms});
+		c->tune_log.push_back({cd.lpt * 100000000 + cd.cl * 1000000 + cd.per, (double)ms});
 		if (ms < best)
 		{
 			best = ms;
@@ -289,7 +305,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 	cudaEventDestroy(e1);
 	cudaFree(store);
 	if (e != cudaSuccess) return cuda_fail(e, "batch autotune");
-	set_schedule(c, best_c.cl, best_c.thr, ctx->sm_count, st, best_c.lpt);
+	if (best_c.cl > 0) set_schedule(c, best_c.cl, 0, ctx->sm_count, st, best_c.lpt, best_c.per);
 	c->tuned = true;
 	return B3G_OK;
 }
@@ -311,10 +327,9 @@ int build_cache(b3g_context* ctx, b3g_body* const* bodies, uint32_t count, int p
 	}
 	c->order.resize(count);
 	std::iota(c->order.begin(), c->order.end(), 0);
-	std::stable_sort(c->order.begin(), c->order.end(), [&](int a, int b) { return bodies[a]->n > bodies[b]->n; });
 	cudaError_t e = cudaMalloc(&c->d_bodies, std::max<size_t>(1, count) * sizeof(DevBody));
 	if (e == cudaSuccess) e = cudaMalloc(&c->d_order, std::max<size_t>(1, count) * sizeof(int));
-	if (e == cudaSuccess) e = cudaMalloc(&c->d_queue, 4 * sizeof(unsigned));
+	if (e == cudaSuccess) e = cudaMalloc(&c->d_queue, kQueueCounters * sizeof(unsigned));
 	// flat numbering of all bodies' elements and row slices (count + 1 offsets each)
 	std::vector<unsigned> off(2 * (size_t)(count + 1), 0);
 	uint64_t ne = 0, nsl = 0;
@@ -377,11 +392,8 @@ int build_cache(b3g_context* ctx, b3g_body* const* bodies, uint32_t count, int p
 		if (cudaMalloc(&c->d_prof, bytes) == cudaSuccess) cudaMemset(c->d_prof, 0, bytes);
 		else cudaGetLastError();
 	}
-	// size heuristic: clusters of 4 for bodies of 16k vertices or more
-	int maxn = 0;
-	for (uint32_t k = 0; k < count; ++k) maxn = std::max(maxn, (int)bodies[k]->n);
-	if (maxn >= 16384) set_schedule(c, 4, 16384, ctx->sm_count, ctx->stream);
-	else set_schedule(c, 1, 1 << 30, ctx->sm_count, ctx->stream);
+	// until the autotuner has looked (or where it may not): about 16 slices a CTA
+	set_schedule(c, 8, 0, ctx->sm_count, ctx->stream, 0, 16);
 	*out = c;
 	return B3G_OK;
 }
@@ -961,6 +973,7 @@ extern "C" int b3g_step_batch_noalloc(b3g_context* ctx, b3g_body* const* bodies,
 	A.nbig = nbig;
 	A.small = d_order + nbig;
 	A.nsmall = (int)count - nbig;
+	two_tiers(&A, cluster, nbig, (int)count);
 	A.queue = d_queue;  // op_batch clears the work counters before each step's launches
 	A.steps = 1;        // one step per op_batch: a single-Newton step is two launches (assembly, then PCG)
 	A.h = dt;

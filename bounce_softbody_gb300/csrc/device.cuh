@@ -1284,25 +1284,13 @@ __device__ __forceinline__ double row_finish(const DevBody& B, int i, float3 bi,
 	return dot3<TV>(bv, sv);
 }
 
-// Assembles row i of the pre-filtered system: pA = S A S^T + I - S and pb = S b with
-//   A = M - h dfdv - h^2 dfdx,  b = M (v0 - v) + h (fe + fi) + h dfdx (x0 - x + h v + y)
-// (sparse_force_solver.cpp:165-174), S = I for dynamic vertices and 0 otherwise
-// (force_solver.cpp:110-129). Also forms the Jacobi preconditioner and, when init_pcg is set
-// (initial guess zero), r = pb, s = M^-1 r, d = s; returns this row's r.s. FILTER: filtered
-// contacts (B.filt) replace the penalty contacts: S_i = I - n n^T for a constrained vertex and
-// pb = S (b - A z), z nonzero in the first Newton iteration only.
-// TETS: the body has tetrahedra only and no contact spheres (no explicit blocks or vectors, no
-// contact terms), so those parts are compiled out: fewer registers, the same arithmetic.
-template <class TA, class TV, class L = LdPlain, bool FILTER = false, bool TETS = false>
-__device__ __forceinline__ double assemble_row(const DevBody& B, int slice, int lane, const StepParams& P,
-                                               int init_pcg)
+// Row i's right-hand side before the filter (b of assemble_row), what its vertex adds to the diagonal
+// of A, and its contacts' stiffness Kc (positive form).
+template <class L, bool FILTER, bool TETS>
+__device__ __forceinline__ float3 row_vertex_terms(const DevBody& B, int i, const StepParams& P, bool Si, float& diagExtra,
+                                                   float Kc[9])
 {
-	const int i = slice * kSlice + lane;
-	if (i >= B.n) return 0.0;
 	const float h = P.h;
-	const int w = B.rowlen[i];
-	const int base = B.slice_ptr[slice];
-	const bool Si = B.type[i] == B3G_DYNAMIC;
 	const float* X = P.first_newton ? B.x : B.xi;
 	const float* Vv = P.first_newton ? B.v : B.vi;
 	const float m = B.mass[i];
@@ -1315,13 +1303,14 @@ __device__ __forceinline__ double assemble_row(const DevBody& B, int slice, int 
 	float3 fe = ldl3<L>(B.fext, i);
 	if (Si) fe = fe + m * f3(B.gravity[0], B.gravity[1], B.gravity[2]);
 	float3 fi = f3(0, 0, 0);
-	float diagExtra = Mi;
+	diagExtra = Mi;
 	if (damp > 0.0f)
 	{
 		fi = fi + (-damp * m) * vi;
 		diagExtra += h * damp * m;
 	}
-	float Kc[9] = {0, 0, 0, 0, 0, 0, 0, 0, 0};
+#pragma unroll
+	for (int q = 0; q < 9; ++q) Kc[q] = 0.0f;
 	if (!FILTER && !TETS && B.contacts)
 	{
 		const float r1 = B.srad[i];
@@ -1405,6 +1394,92 @@ __device__ __forceinline__ double assemble_row(const DevBody& B, int slice, int 
 			bi = (e & 1) ? bi - c : bi + c;
 		}
 	}
+
+	return bi;
+}
+
+// The block of A of one slot (item `slot` of the contribution lists) before the diagonal's vertex
+// terms and the filter: its tetrahedra in list order, four records in flight at a time, then its
+// explicit blocks.
+template <class L>
+__device__ __forceinline__ void slot_block(const DevBody& B, int slot, float a[9])
+{
+	const size_t nt = (size_t)B.nt;
+	const uint32_t st = __ldg(B.tet_cstart + slot);
+	const int cnt = __ldg(B.tet_ccnt + slot);
+	const bool uniform = B.tet_ratio >= 0.0f;
+	float p[9];
+#pragma unroll
+	for (int q = 0; q < 9; ++q) a[q] = p[q] = 0.0f;
+	for (int t = 0; t < cnt; t += 4)
+	{
+		uint32_t cd[4];
+		float4 ua[4], ub[4];
+#pragma unroll
+		for (int u = 0; u < 4; ++u) cd[u] = t + u < cnt ? __ldg(B.tet_clist + st + kSlice * (t + u)) : 0u;
+#pragma unroll
+		for (int u = 0; u < 4; ++u)
+			if (t + u < cnt)
+			{
+				const float4* r0 = B.tet_rec + (cd[u] >> 4);
+				ua[u] = L::ld(r0 + ((cd[u] >> 2) & 3u) * nt);
+				ub[u] = L::ld(r0 + (cd[u] & 3u) * nt);
+			}
+#pragma unroll
+		for (int u = 0; u < 4; ++u)
+			if (t + u < cnt)
+			{
+				if (uniform) add_outer(p, ua[u], ub[u]);
+				else add_tet_block(a, ua[u], ub[u]);
+			}
+	}
+	if (uniform) add_tet_blocks_uniform(a, p, B.tet_ratio);
+	const uint32_t bst = __ldg(B.blk_cstart + slot);
+	const int bcnt = __ldg(B.blk_ccnt + slot);
+	for (int t = 0; t < bcnt; ++t)
+	{
+		const uint32_t code = __ldg(B.blk_clist + bst + kSlice * t);
+		const float* blk = B.blocks + 9 * (size_t)(code >> 1);
+		const float sgn = (code & 1) ? -1.0f : 1.0f;
+#pragma unroll
+		for (int q = 0; q < 9; ++q) a[q] += sgn * L::ld(blk + q);
+	}
+}
+
+template <class TA>
+__device__ __forceinline__ void store_block(const DevBody& B, size_t bs, const float a[9])
+{
+#pragma unroll
+	for (int q = 0; q < 9; ++q) B.A32[(size_t)q * B.nslots + bs] = a[q];
+	if (B.Alo)
+	{
+#pragma unroll
+		for (int q = 0; q < 9; ++q) ((TA*)B.Alo)[(size_t)q * B.nslots + bs] = from_f<TA>(a[q]);
+	}
+}
+
+// Assembles row i of the pre-filtered system: pA = S A S^T + I - S and pb = S b with
+//   A = M - h dfdv - h^2 dfdx,  b = M (v0 - v) + h (fe + fi) + h dfdx (x0 - x + h v + y)
+// (sparse_force_solver.cpp:165-174), S = I for dynamic vertices and 0 otherwise
+// (force_solver.cpp:110-129). Also forms the Jacobi preconditioner and, when init_pcg is set
+// (initial guess zero), r = pb, s = M^-1 r, d = s; returns this row's r.s. FILTER: filtered
+// contacts (B.filt) replace the penalty contacts: S_i = I - n n^T for a constrained vertex and
+// pb = S (b - A z), z nonzero in the first Newton iteration only.
+// TETS: the body has tetrahedra only and no contact spheres (no explicit blocks or vectors, no
+// contact terms), so those parts are compiled out: fewer registers, the same arithmetic.
+template <class TA, class TV, class L = LdPlain, bool FILTER = false, bool TETS = false>
+__device__ __forceinline__ double assemble_row(const DevBody& B, int slice, int lane, const StepParams& P,
+                                               int init_pcg)
+{
+	const int i = slice * kSlice + lane;
+	if (i >= B.n) return 0.0;
+	const float h = P.h;
+	const int w = B.rowlen[i];
+	const int base = B.slice_ptr[slice];
+	const bool Si = B.type[i] == B3G_DYNAMIC;
+	float diagExtra, Kc[9];
+	float3 bi = row_vertex_terms<L, FILTER, TETS>(B, i, P, Si, diagExtra, Kc);
+	const size_t nt = (size_t)B.nt;
 
 	float4 fi4 = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
 	if (FILTER) fi4 = B.filt[i];
@@ -1584,13 +1659,7 @@ __device__ __forceinline__ double assemble_row(const DevBody& B, int slice, int 
 #pragma unroll
 			for (int q = 0; q < 9; ++q) a[q] = 0.0f;
 		}
-#pragma unroll
-		for (int q = 0; q < 9; ++q) B.A32[(size_t)q * B.nslots + bs] = a[q];
-		if (B.Alo)
-		{
-#pragma unroll
-			for (int q = 0; q < 9; ++q) ((TA*)B.Alo)[(size_t)q * B.nslots + bs] = from_f<TA>(a[q]);
-		}
+		store_block<TA>(B, bs, a);
 	}
 	if (!Si) bi = f3(0, 0, 0);
 	else if (FILTER)

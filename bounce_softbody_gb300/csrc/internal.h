@@ -44,6 +44,8 @@ constexpr int kGroup = 4;
 B3G_HD size_t block_slot(size_t base, int k, int lane) { return base + 128 * (size_t)(k >> 2) + 4 * lane + (k & 3); }
 constexpr int kMaxWorld = 16;   // world fixtures per body
 constexpr int kMaxTeamCtas = 16;
+constexpr int kTiers = 5;                    // team widths 16, 8, 4, 2, 1
+constexpr int kQueueCounters = 2 + kTiers;   // the team launch's two, one per tier of the solve launch
 
 // Device-resident solver scalars of one body; everything the PCG decides is taken here.
 struct Scalars

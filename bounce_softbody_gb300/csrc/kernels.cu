@@ -132,13 +132,10 @@ __device__ __forceinline__ b3g_ray_hit ray_hit(const DevBody& B, float3 p1, floa
 	o.triangle = 0;
 	o.fraction = 0.0f;
 	o.normal[0] = o.normal[1] = o.normal[2] = 0.0f;
-	const unsigned long long key = keys[r];
 	if (key != ~0ull)
 	{
 		const unsigned e = (unsigned)(key & 0xffffffffu);
 		const uint4 id = B.tri[e];
-		const float3 p1 = f3(seg[6 * r], seg[6 * r + 1], seg[6 * r + 2]);
-		const float3 d = f3(seg[6 * r + 3], seg[6 * r + 4], seg[6 * r + 5]) - p1;
 		float t, num;
 		float3 n;
 		ray_triangle(p1, d, ld3(B.x, id.x), ld3(B.x, id.y), ld3(B.x, id.z), t, num, n);
@@ -221,6 +218,76 @@ __global__ void __launch_bounds__(kThreads) k_assemble(DevBody B, StepParams P, 
 		assemble_row<TA, TV, LdPlain, FILTER>(B, s, lane, P, init);
 }
 
+// The row assembly of a small body, one CTA per slice: a warp per slot column (slot k of the slice's 32
+// rows) and one for the rows' right-hand sides and vertex terms, where k_assemble has one warp do them
+// in turn. A small body leaves most of the GPU idle, and a row's slots are a chain of dependent
+// gathers: 10^3 block 50 us with one warp a slice (4 CTAs). Every block and right-hand side is summed in
+// k_assemble's order.
+constexpr int kSlotWarps = 17;
+
+template <class TA, class TV>
+__global__ void __launch_bounds__(32 * kSlotWarps) k_assemble_slots(DevBody B, StepParams P, int init)
+{
+	if (newton_over(B, P)) return;
+	for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < (int)(sizeof(TeamMemory) / 4); k += gridDim.x * blockDim.x)
+		((unsigned*)B.team)[k] = 0u;
+	__shared__ float sb[3][32], sk[9][32], sd[32];
+	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slots = (int)(blockDim.x >> 5) - 1;
+	const int i = blockIdx.x * kSlice + lane;
+	const bool row = i < B.n;
+	const bool Si = row && B.type[i] == B3G_DYNAMIC;
+	const int base = B.slice_ptr[blockIdx.x];
+	const int w = row ? B.rowlen[i] : 0;
+	float a[9];
+	if (warp == slots)
+	{
+		if (row)
+		{
+			float extra, Kc[9];
+			const float3 bi = row_vertex_terms<LdPlain, false, false>(B, i, P, Si, extra, Kc);
+			sb[0][lane] = bi.x;
+			sb[1][lane] = bi.y;
+			sb[2][lane] = bi.z;
+			sd[lane] = extra;
+#pragma unroll
+			for (int q = 0; q < 9; ++q) sk[q][lane] = Kc[q];
+		}
+	}
+	else
+	{
+		// a later column than the diagonal of warp 0 comes first, so that the diagonal stays in a
+		for (int k = warp + (B.maxw - 1 - warp) / slots * slots; k >= 0; k -= slots)
+		{
+			if (k >= w) continue;
+			slot_block<LdPlain>(B, base + k * kSlice + lane, a);
+			if (k == 0) break;
+			const size_t bs = block_slot((size_t)base, k, lane);
+			if (!(Si && B.type[B.col[bs]] == B3G_DYNAMIC))
+			{
+#pragma unroll
+				for (int q = 0; q < 9; ++q) a[q] = 0.0f;
+			}
+			store_block<TA>(B, bs, a);
+		}
+	}
+	__syncthreads();
+	if (warp != 0 || !row) return;
+#pragma unroll
+	for (int q = 0; q < 9; ++q) a[q] += P.h * P.h * sk[q][lane];
+	a[0] += sd[lane];
+	a[4] += sd[lane];
+	a[8] += sd[lane];
+	float3 bi = f3(sb[0][lane], sb[1][lane], sb[2][lane]);
+	if (!Si)
+	{
+#pragma unroll
+		for (int q = 0; q < 9; ++q) a[q] = (q == 0 || q == 4 || q == 8) ? 1.0f : 0.0f;
+		bi = f3(0, 0, 0);
+	}
+	store_block<TA>(B, block_slot((size_t)base, 0, lane), a);
+	row_finish<TV>(B, i, bi, a, init);
+}
+
 __global__ void __launch_bounds__(kThreads) k_nostep(DevBody B)
 {
 	for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < B.n; i += gridDim.x * blockDim.x)
@@ -268,6 +335,12 @@ __global__ void k_fill(float* p, size_t n, float v)
 {
 	for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) p[i] = v;
 }
+
+// Bodies up to this many slices are assembled by k_assemble_slots (6 CTAs per SM). Measured with
+// k_assemble / k_assemble_slots, us a step: 378 vertices with three Newton iterations 707 / 644, 10^3
+// block 206 / 186, FP64 block of 397 slices 615 / 573, cloth of 512 slices 1257 / 1240; blocks of 2229 and 8192
+// slices, which fill the GPU with a warp a slice, 3431 / 3544 and 11491 / 11673.
+constexpr int kSlotAssemblySlices = 1024;
 
 StepParams dev_params(const StepParamsHost& P)
 {
@@ -360,6 +433,13 @@ cudaError_t op_assemble(const DevBody& B, const StepParamsHost& Ph, int prec, in
 		if (prec == kP64) k_assemble<double, double, true><<<g, kThreads, 0, st>>>(B, P, in);
 		else if (prec == kPBF) k_assemble<__nv_bfloat16, float, true><<<g, kThreads, 0, st>>>(B, P, in);
 		else k_assemble<float, float, true><<<g, kThreads, 0, st>>>(B, P, in);
+	}
+	else if (B.nslices <= kSlotAssemblySlices)
+	{
+		const int t = 32 * std::min(kSlotWarps, B.maxw + 1);
+		if (prec == kP64) k_assemble_slots<double, double><<<B.nslices, t, 0, st>>>(B, P, in);
+		else if (prec == kPBF) k_assemble_slots<__nv_bfloat16, float><<<B.nslices, t, 0, st>>>(B, P, in);
+		else k_assemble_slots<float, float><<<B.nslices, t, 0, st>>>(B, P, in);
 	}
 	else if (prec == kP64) k_assemble<double, double, false><<<g, kThreads, 0, st>>>(B, P, in);
 	else if (prec == kPBF) k_assemble<__nv_bfloat16, float, false><<<g, kThreads, 0, st>>>(B, P, in);

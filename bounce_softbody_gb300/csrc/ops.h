@@ -115,7 +115,10 @@ struct BatchArgs
 	int nbig;
 	const int* small;        // device array: indices of bodies stepped by single CTAs
 	int nsmall;
-	unsigned* queue;         // device: four work counters (two per launch), cleared by op_batch
+	// The solve launch's teams: body k of the order (big, then small) is solved by a team of
+	// kMaxTeamCtas >> t CTAs for the first t with k < tier_end[t]; teams are at most `cluster` wide.
+	int tier_end[kTiers];
+	unsigned* queue;         // device: kQueueCounters work counters, cleared by op_batch
 	int steps;
 	float h;
 	int newton;
@@ -151,6 +154,11 @@ struct BatchArgs
 	unsigned elem_mid = 0, slice_mid = 0;
 	int split_elem_per_sm = 0, split_rows_per_sm = 0;
 };
+// Two kinds of solve teams: the first nbig bodies by teams of `cluster` CTAs, the rest by one CTA.
+inline void two_tiers(BatchArgs* A, int cluster, int nbig, int count)
+{
+	for (int t = 0; t < kTiers; ++t) A->tier_end[t] = t == kTiers - 1 ? count : ((kMaxTeamCtas >> t) <= cluster ? nbig : 0);
+}
 cudaError_t op_batch(const BatchArgs& A, cudaStream_t st);
 // Co-resident clusters of the batch kernel for this precision and cluster size (0 on error).
 int batch_max_clusters(int prec, int cluster);

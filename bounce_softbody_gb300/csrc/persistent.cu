@@ -95,6 +95,7 @@ cudaError_t op_batch(const BatchArgs& A, cudaStream_t st)
 	P.small = A.small;
 	P.nsmall = A.nsmall;
 	P.queue = A.queue;
+	for (int t = 0; t < kTiers; ++t) P.tier_end[t] = A.tier_end[t];
 	P.steps = A.steps;
 	P.h = A.h;
 	P.newton = A.newton < 1 ? 1 : A.newton;
@@ -118,8 +119,8 @@ cudaError_t op_batch(const BatchArgs& A, cudaStream_t st)
 	P.flat = (P.newton == 1 && A.elem_off && A.slice_off && A.nslices > 0) ? 1 : 0;
 	if (A.part != 2)
 	{
-		// two counters per launch; the solve-only part reuses what the assembly part cleared
-		cudaError_t e = cudaMemsetAsync(A.queue, 0, 4 * sizeof(unsigned), st);
+		// the solve-only part reuses what the assembly part cleared
+		cudaError_t e = cudaMemsetAsync(A.queue, 0, kQueueCounters * sizeof(unsigned), st);
 		if (e != cudaSuccess) return e;
 		if (P.flat)
 		{

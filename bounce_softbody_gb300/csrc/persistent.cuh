@@ -38,6 +38,7 @@ struct BatchParams
 	const int* small;
 	int nsmall;
 	unsigned* queue;
+	int tier_end[kTiers];  // of the order `big` (which runs on into `small`): the solve launch's teams
 	int steps;
 	float h;
 	int newton;
@@ -584,8 +585,8 @@ __global__ void __launch_bounds__(kPThreads, B3G_BATCH_MIN_BLOCKS) k_batch(Batch
 	}
 }
 
-// The PCG, the final update and the statistics of every body of a batch (single-Newton steps), by
-// clusters of CL CTAs and then by single CTAs, as k_batch distributes them; each body is solved by
+// The PCG, the final update and the statistics of every body of a batch (single-Newton steps). A body's
+// team is a cluster or an aligned half, quarter ... of one (its tier); each body is solved by
 // team_solve with its rows' vectors and as much of its matrix as fits in shared memory.
 // One CTA of 512 threads per SM (128 registers a thread, the SM's shared memory to itself). Measured
 // on 160 / 12 uneven blocks and 16 blocks and cloths, ms a step: 512 x 1 12.1 / 1.54 / 7.0, 640 x 1
@@ -622,42 +623,35 @@ __device__ __forceinline__ void batch_solve_body(Team& T, const DevBody& B, cons
 	    [&](int phase) { pc.tick(phase); });
 }
 
-template <int CL, class TA, class TV>
+template <class TA, class TV>
 __global__ void __launch_bounds__(kSolveMaxThreads, 1) k_batch_solve(BatchParams P, int room)
 {
 	extern __shared__ __align__(16) unsigned char smem[];
 	__shared__ SolveSh sh;
 	__shared__ __align__(16) DevBody sb;
-	__shared__ int s_item;
-	unsigned* queue = P.queue + 2;
-	if (CL > 1)
+	cg::cluster_group cl = cg::this_cluster();
+	ClusterTeam<TV> T(&sh);
+	cl.sync();
+	// widest teams first; a cluster whose wider teams find no more bodies splits into narrower ones
+	int begin = 0;
+	for (int t = 0; t < kTiers; ++t)
 	{
-		cg::cluster_group cl = cg::this_cluster();
-		ClusterTeam<TV, CL> T(&sh);
-		for (;;)
+		const int end = P.tier_end[t], width = kMaxTeamCtas >> t;
+		if (end > begin && width <= (int)cl.num_blocks())
 		{
-			if (T.rank == 0 && threadIdx.x == 0) s_item = (int)atomicAdd(queue, 1u);
-			cl.sync();
-			const int item = *cl.map_shared_rank(&s_item, 0);
-			cl.sync();
-			if (item >= P.nbig) break;
-			load_body(&sb, P.bodies + P.big[item]);
-			__syncthreads();
-			batch_solve_body<TA, TV>(T, sb, P, smem, room);
+			T.form(width);
+			for (;;)
+			{
+				const int item = begin + T.agree([&] { return (int)min(atomicAdd(P.queue + 2 + t, 1u), 1u << 29); });
+				if (item >= end || !T.ok) break;
+				load_body(&sb, P.bodies + P.big[item]);
+				__syncthreads();
+				batch_solve_body<TA, TV>(T, sb, P, smem, room);
+			}
 		}
+		begin = end;
 	}
-	ClusterTeam<TV, 1> T(&sh);
-	for (;;)
-	{
-		__syncthreads();
-		if (threadIdx.x == 0) s_item = (int)atomicAdd(queue + 1, 1u);
-		__syncthreads();
-		const int item = s_item;
-		if (item >= P.nsmall) break;
-		load_body(&sb, P.bodies + P.small[item]);
-		__syncthreads();
-		batch_solve_body<TA, TV>(T, sb, P, smem, room);
-	}
+	cl.sync();
 }
 
 // Clusters of more than 8 CTAs are a non-portable size the kernel has to opt in to.
@@ -716,24 +710,24 @@ inline int solve_room()
 		cudaGetDevice(&dev);
 		cudaDeviceGetAttribute(&block, cudaDevAttrMaxSharedMemoryPerBlockOptin, dev);
 		cudaDeviceGetAttribute(&sm, cudaDevAttrMaxSharedMemoryPerMultiprocessor, dev);
-		return (std::min(block, sm - 1024) - (int)(sizeof(SolveSh) + sizeof(DevBody)) - 256) & ~127;
+		return (std::min(block, sm - 1024) - (int)(sizeof(SolveSh) + sizeof(DevBody)) - 256 - kL1Room) & ~127;
 	}();
 	return room;
 }
 
-template <int CL, class TA, class TV>
-cudaError_t solve_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int ctas, cudaStream_t st)
+template <class TA, class TV>
+cudaError_t solve_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int cluster, int ctas, cudaStream_t st)
 {
-	cudaError_t e = cudaFuncSetAttribute(k_batch_solve<CL, TA, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve_room());
-	if (e == cudaSuccess && CL > 8)
-		e = cudaFuncSetAttribute(k_batch_solve<CL, TA, TV>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+	cudaError_t e = cudaFuncSetAttribute(k_batch_solve<TA, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, solve_room());
+	if (e == cudaSuccess && cluster > 8)
+		e = cudaFuncSetAttribute(k_batch_solve<TA, TV>, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
 	*cfg = {};
 	cfg->gridDim = dim3((unsigned)ctas, 1, 1);
 	cfg->blockDim = dim3(kSolveMaxThreads, 1, 1);
 	cfg->dynamicSmemBytes = (size_t)solve_room();
 	cfg->stream = st;
 	attr->id = cudaLaunchAttributeClusterDimension;
-	attr->val.clusterDim.x = CL;
+	attr->val.clusterDim.x = (unsigned)cluster;
 	attr->val.clusterDim.y = 1;
 	attr->val.clusterDim.z = 1;
 	cfg->attrs = attr;
@@ -741,22 +735,22 @@ cudaError_t solve_config(cudaLaunchConfig_t* cfg, cudaLaunchAttribute* attr, int
 	return e;
 }
 
-// Co-resident clusters of the solve launch, queried once per instantiation.
-template <int CL, class TA, class TV>
-int solve_clusters()
+// Co-resident clusters of the solve launch, queried once per precision and cluster size.
+template <class TA, class TV>
+int solve_clusters(int cluster)
 {
-	static std::atomic<int> cached(-1);
-	int m = cached.load(std::memory_order_relaxed);
+	static std::atomic<int> cached[kMaxTeamCtas + 1];  // count + 1; 0: not known yet
+	int m = cached[cluster].load(std::memory_order_relaxed) - 1;
 	if (m < 0)
 	{
 		cudaLaunchConfig_t cfg;
 		cudaLaunchAttribute attr;
 		m = 0;
-		if (solve_config<CL, TA, TV>(&cfg, &attr, CL, nullptr) == cudaSuccess &&
-		    cudaOccupancyMaxActiveClusters(&m, k_batch_solve<CL, TA, TV>, &cfg) != cudaSuccess)
+		if (solve_config<TA, TV>(&cfg, &attr, cluster, cluster, nullptr) == cudaSuccess &&
+		    cudaOccupancyMaxActiveClusters(&m, k_batch_solve<TA, TV>, &cfg) != cudaSuccess)
 			m = 0;
 		cudaGetLastError();
-		cached.store(m, std::memory_order_relaxed);
+		cached[cluster].store(m + 1, std::memory_order_relaxed);
 	}
 	return m;
 }
@@ -773,12 +767,12 @@ cudaError_t launch_cl(const BatchParams& P, int ctas, int bf16, int part, cudaSt
 		cudaError_t e = launch_ph<CL, TA, TV, kPhaseAssemble>(P, ctas, bf16, st);
 		if (e != cudaSuccess || part == 1) return e;
 	}
-	const int m = solve_clusters<CL, TA, TV>();
+	const int m = solve_clusters<TA, TV>(CL);
 	cudaLaunchConfig_t cfg;
 	cudaLaunchAttribute attr;
-	cudaError_t e = solve_config<CL, TA, TV>(&cfg, &attr, m > 0 ? m * CL : CL, st);
+	cudaError_t e = solve_config<TA, TV>(&cfg, &attr, CL, m > 0 ? m * CL : CL, st);
 	if (e != cudaSuccess) return e;
-	return cudaLaunchKernelEx(&cfg, k_batch_solve<CL, TA, TV>, P, solve_room());
+	return cudaLaunchKernelEx(&cfg, k_batch_solve<TA, TV>, P, solve_room());
 }
 
 // The body of flat item g: the last k with off[k] <= g.
@@ -887,7 +881,7 @@ cudaError_t launch_prec(const BatchParams& P, int cluster, int ctas, int bf16, i
 template <int CL, class TA, class TV>
 int max_clusters()
 {
-	if (solve_clusters<CL, TA, TV>() <= 0) return 0;
+	if (solve_clusters<TA, TV>(CL) <= 0) return 0;
 	return max_clusters_ph<CL, TA, TV, kPhaseAssemble>();
 }
 

@@ -499,6 +499,7 @@ int step_active(b3g_server* s, int count, int nbig)
 	A.small = s->d_order + nbig;
 	A.nsmall = count - nbig;
 	A.queue = s->d_queue;
+	two_tiers(&A, s->cluster, nbig, count);
 	A.steps = 1;
 	A.h = s->dt;
 	A.newton = (int)std::max<uint32_t>(1u, s->cfg.force_iterations);
@@ -627,7 +628,7 @@ int b3g_server_create(b3g_context* ctx, uint64_t memory_budget_bytes, uint32_t m
 	if (e == cudaSuccess) e = cudaMalloc(&s->d_order, max_active * sizeof(int));
 	if (e == cudaSuccess) e = cudaMalloc(&s->d_flat_off, 2 * (max_active + 1) * sizeof(unsigned));
 	if (e == cudaSuccess) e = cudaMallocHost(&s->h_flat_off, 2 * (max_active + 1) * sizeof(unsigned));
-	if (e == cudaSuccess) e = cudaMalloc(&s->d_queue, 4 * sizeof(unsigned));
+	if (e == cudaSuccess) e = cudaMalloc(&s->d_queue, kQueueCounters * sizeof(unsigned));
 	if (e == cudaSuccess) e = cudaMallocHost(&s->h_table, max_active * sizeof(DevBody));
 	if (e == cudaSuccess) e = cudaMallocHost(&s->h_order, max_active * sizeof(int));
 	if (e == cudaSuccess) e = cudaEventCreate(&s->ev0);

@@ -43,6 +43,7 @@ namespace b3g {
 namespace {
 
 constexpr int kSolveMaxThreads = 512;
+constexpr int kL1Room = 32 << 10;             // shared memory left to the L1 where it serves the gathers
 constexpr int kPollLimit = 1 << 20;           // polls before a warp gives up (about a second)
 constexpr int kTeamWarpSlots = kTeamMax / 32; // slots a lane of the polling warp reads
 
@@ -225,7 +226,6 @@ __device__ __forceinline__ double cta_total(const SolveSh* sh, int buf, Fixed v)
 template <class TV>
 struct GridTeam
 {
-	static constexpr bool kManyCtas = true;
 	SolveSh* sh;
 	TeamMemory* mem;
 	int ctas, rank;
@@ -334,26 +334,33 @@ struct GridTeam
 	}
 };
 
-// A thread-block cluster of CL CTAs (or one CTA). Partials go straight into the slots of every CTA's
-// shared memory, where its warp 0 polls them: one trip through the cluster's network a sum. The
-// number's two bits work as in the grid team, over the team's whole life.
-template <class TV, int CL>
+// `size` consecutive CTAs of a thread-block cluster from rank `base` (size 1: a CTA by itself).
+// Partials go straight into the slots of every member's shared memory, where its warp 0 polls them:
+// one trip through the cluster's network a sum. The number's two bits work as in the grid team. A
+// team may split into smaller ones between two sums: its members have counted the same sums, and a
+// slot's last partial is of the sum two before, so it is told from the next one.
+template <class TV>
 struct ClusterTeam
 {
-	static constexpr bool kManyCtas = CL > 1;
 	SolveSh* sh;
-	int rank;
+	int cta;          // rank in the cluster
+	int rank, base, ctas;
 	unsigned sums;
 	int ok;
 	TV ratio;
-	static constexpr int ctas = CL;
 
-	// (the caller synchronises the cluster after this)
-	__device__ __forceinline__ explicit ClusterTeam(SolveSh* s) : sh(s), rank(0), sums(0), ok(1), ratio((TV)0)
+	// (the caller synchronises the cluster after this, and again before a CTA leaves the kernel)
+	__device__ __forceinline__ explicit ClusterTeam(SolveSh* s)
+	    : sh(s), cta((int)cooperative_groups::this_cluster().block_rank()), rank(0), base(0), ctas(1), sums(0), ok(1), ratio((TV)0)
 	{
-		if (CL > 1) rank = (int)cooperative_groups::this_cluster().block_rank();
 		if (threadIdx.x < 2 * kMaxTeamCtas) (&sh->slot[0][0])[threadIdx.x] = 0ull;
 		if (threadIdx.x == 0) sh->lost = 0;
+	}
+	__device__ __forceinline__ void form(int size)
+	{
+		ctas = size;
+		base = cta / size * size;
+		rank = cta - base;
 	}
 	template <bool FENCE, class F, class R>
 	__device__ __forceinline__ double sum(Fixed v, F between, R ratio_of)
@@ -367,33 +374,37 @@ struct ClusterTeam
 		if (warp == 0)
 		{
 			total = cta_total(sh, buf, v);
-			if (CL > 1 && lane < CL)
+			if (ctas > 1)
 			{
-				const unsigned long long bits = ((unsigned long long)__double_as_longlong(total) & ~3ull) | tag;
-				unsigned remote;
-				asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-				             : "=r"(remote)
-				             : "r"((unsigned)__cvta_generic_to_shared(&sh->slot[buf][rank])), "r"(lane));
-				asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(bits) : "memory");
+				if (FENCE) __threadfence();
+				if (lane < ctas)
+				{
+					const unsigned long long bits = ((unsigned long long)__double_as_longlong(total) & ~3ull) | tag;
+					unsigned remote;
+					asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+					             : "=r"(remote)
+					             : "r"((unsigned)__cvta_generic_to_shared(&sh->slot[buf][rank])), "r"(base + lane));
+					asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(bits) : "memory");
+				}
 			}
 		}
 		between();
-		if (FENCE && CL > 1) cooperative_groups::this_cluster().sync();
 		if (warp == 0)
 		{
 			bool there = true;
-			if (CL > 1)
+			if (ctas > 1)
 			{
 				unsigned long long u = tag;
-				const unsigned mine = (unsigned)__cvta_generic_to_shared(&sh->slot[buf][lane < CL ? lane : 0]);
+				const unsigned mine = (unsigned)__cvta_generic_to_shared(&sh->slot[buf][lane < ctas ? lane : 0]);
 				for (int polls = 0;;)
 				{
-					if (lane < CL)
+					if (lane < ctas)
 						asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(u) : "r"(mine) : "memory");
 					there = __all_sync(0xffffffffu, (u & 3ull) == tag) != 0;
 					if (there || ++polls > 16 * kPollLimit) break;
 				}
 				total = fixed_value(fixed_warp_sum(to_fixed(__longlong_as_double((long long)(u & ~3ull)))));
+				if (FENCE) __threadfence();
 			}
 			const TV r = ratio_of(total);
 			if (lane == 0)
@@ -416,8 +427,26 @@ struct ClusterTeam
 	}
 	__device__ __forceinline__ void publish()
 	{
-		if (CL > 1) cooperative_groups::this_cluster().sync();
-		else __syncthreads();
+		Fixed z;
+		z.m = 0;
+		z.e = kFixedZero;
+		sum<true>(z);
+	}
+	// the first member's thread 0 evaluates next() (an integer below 2^30), the team returns it
+	template <class N>
+	__device__ __forceinline__ int agree(N next)
+	{
+		Fixed z;
+		z.m = 0;
+		z.e = kFixedZero;
+		if (rank == 0 && threadIdx.x < 32)
+		{
+			int item = threadIdx.x == 0 ? next() : 0;
+			item = __shfl_sync(0xffffffffu, item, 0);
+			z.m = (long long)item << 20;
+			z.e = item ? -20 : kFixedZero;
+		}
+		return (int)sum<false>(z);
 	}
 };
 
@@ -432,6 +461,26 @@ __device__ __forceinline__ float4 ld_version(const float* s, int i)
 	             : "memory");
 	return make_float4(__uint_as_float((unsigned)lo), __uint_as_float((unsigned)(lo >> 32)), __uint_as_float((unsigned)hi),
 	                   __uint_as_float((unsigned)(hi >> 32)));
+}
+// The same through the SM's L1, which may hold an older version (the caller reads that again). A sweep
+// whose matrix comes from L2 shares the L2-to-SM network with its gathers, a fourth of its bytes, and
+// a vertex is gathered about 15 times, mostly by one SM: the sweep of a large body goes through
+// the L1, which a fence empties of the last version between the sweeps, and the launch leaves it kL1Room
+// of the SM's memory. 64^3 block 11.7 -> 9.6 ms a step, PCG launch of 160 blocks 9.4 -> 7.9. On bodies that
+// shared memory holds, the extra reads of old lines cost 8-17 %.
+__device__ __forceinline__ float4 ld_version_l1(const float* s, int i)
+{
+	unsigned long long lo, hi;
+	asm volatile("{ .reg .b128 t; ld.relaxed.cta.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
+	             : "=l"(lo), "=l"(hi)
+	             : "l"(s + 4 * (size_t)i)
+	             : "memory");
+	return make_float4(__uint_as_float((unsigned)lo), __uint_as_float((unsigned)(lo >> 32)), __uint_as_float((unsigned)hi),
+	                   __uint_as_float((unsigned)(hi >> 32)));
+}
+__device__ __forceinline__ void empty_l1()
+{
+	if (threadIdx.x == blockDim.x - 32) asm volatile("fence.acq_rel.gpu;" ::: "memory");
 }
 __device__ __forceinline__ void st_version(float* s, int i, const float o[3], unsigned version)
 {
@@ -512,7 +561,7 @@ __device__ __forceinline__ void team_spmv_row(const M& m, int w, int lane, const
 			for (int g = 0; g < DEPTH; ++g)
 				if (g == 0 || k0 + g * kGroup < w)
 #pragma unroll
-					for (int u = 0; u < 4; ++u) r[g][u] = ld_version(s, jj[g][u]);
+					for (int u = 0; u < 4; ++u) r[g][u] = DEPTH == 1 ? ld_version_l1(s, jj[g][u]) : ld_version(s, jj[g][u]);
 			if (DEPTH == 1 && k0 + kGroup < w) ahead = m.cols(32 * (k0 + kGroup) + 4 * lane);
 			for (int polls = 0;; ++polls)
 			{
@@ -930,7 +979,7 @@ __device__ __forceinline__ void team_solve(Team& T, const DevBody& B, const Solv
 	                      solve_vec_bytes<TV, FF>(), P.keep, T.rank, T.ctas);
 	const TV* sv = (const TV*)B.s;
 	// FP32 vectors: s carries its version, 0 as the assembly leaves it; FP64: every new s is fenced
-	constexpr bool kVersions = sizeof(TV) == 4 && Team::kManyCtas;
+	constexpr bool kVersions = sizeof(TV) == 4;
 	constexpr bool kFence = !kVersions;
 	// BF16 blocks: the refresh uses the FP32 ones, and a residual that met the tolerance is confirmed
 	// by a refresh before the solve ends
@@ -970,7 +1019,7 @@ __device__ __forceinline__ void team_solve(Team& T, const DevBody& B, const Solv
 				else
 				{
 					TV q[3], own[3];
-					team_spmv_row<typename std::conditional<kConfirm, float, TA>::type, TV, DEPTH, false>(m, w, lane, (const TV*)B.py, 0u, T.sh, q, own);
+					team_spmv_row<typename std::conditional<kConfirm, float, TA>::type, TV, 1, false>(m, w, lane, (const TV*)B.py, 0u, T.sh, q, own);
 #pragma unroll
 					for (int c = 0; c < 3; ++c) rr[c] = b[c] - q[c];
 				}
@@ -1093,6 +1142,7 @@ __device__ __forceinline__ void team_solve(Team& T, const DevBody& B, const Solv
 			break;
 		}
 		const TV alpha = T.ratio;
+		if (kVersions && DEPTH == 1) empty_l1();
 		const Divisor<TV> by_delta(S.delta);
 		auto beta_of = [&](double t) { return by_delta.divide(t); };
 		double dn;
@@ -1164,6 +1214,27 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
 	    T, B, P, smem,
 	    [&](int i, float3 dv, bool finish) { return final_vertex_dv<LdPlain, FILTER>(B, i, P.h, P.newton == 0, finish, dv); },
 	    [](int) {});
+}
+
+// The same by one cluster, for a body whose slices fit a few CTAs: sums through distributed shared
+// memory instead of L2.
+template <class TA, class TV, bool FF, bool FILTER>
+__global__ void __launch_bounds__(256, 1) k_solve_cluster(DevBody B, SolveArgs P)
+{
+	extern __shared__ __align__(16) unsigned char smem[];
+	__shared__ SolveSh sh;
+	ClusterTeam<TV> T(&sh);
+	cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
+	cl.sync();
+	if (P.newton <= 0 || !B.sc->newton_done)
+	{
+		T.form((int)cl.num_blocks());
+		team_solve<TA, TV, FF, sizeof(TV) == 8 ? 2 : 4>(
+		    T, B, P, smem,
+		    [&](int i, float3 dv, bool finish) { return final_vertex_dv<LdPlain, FILTER>(B, i, P.h, P.newton == 0, finish, dv); },
+		    [](int) {});
+	}
+	cl.sync();
 }
 
 // The BF16 mode's solve: a flexible CG (Notay's, one stored direction) on the FP32 blocks, with
@@ -1290,6 +1361,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 				const double dq = T.sum<false>(part, [] {}, [&](double t) { return Divisor<float>(t).divide(delta); });
 				if (!T.ok || !bits_finite(dq) || !bits_positive(dq)) break;
 				const float alpha = T.ratio;
+				if (kDepth == 1) empty_l1();
 				const Divisor<float> by_delta(delta);
 				++version;
 				part = O.row_sum<float>([&](int j, int i) {
