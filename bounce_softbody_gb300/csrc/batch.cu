@@ -41,6 +41,7 @@ struct BatchCache
 	int threshold = 1 << 30;
 	int per = 0;                 // slices a CTA of a body's team should have (0: teams by threshold)
 	int tier_end[kTiers] = {};
+	int helper = 0;              // CTAs of a cluster of the second solve launch (0: none)
 	int nbig = 0;
 	int ctas = 0;
 	bool tuned = false;
@@ -92,6 +93,7 @@ BatchArgs make_args(BatchCache* c, float h, int steps, const b3g_solver_config& 
 	A.nsmall = (int)c->order.size() - c->nbig;
 	A.queue = c->d_queue;
 	std::copy(c->tier_end, c->tier_end + kTiers, A.tier_end);
+	A.helper = c->helper;
 	A.steps = steps;
 	A.h = h;
 	A.newton = (int)std::max<uint32_t>(1u, cfg.force_iterations);
@@ -144,12 +146,14 @@ double est_time(const BatchCache* c, int k, int width)
 // a width the queue runs largest first, or with lpt longest estimated solve first
 // (longest-processing-time order), so that a small body with many PCG iterations does not start
 // last and trail the launch; the autotuner tries both.
-void set_schedule(BatchCache* c, int cluster, int threshold, int sms, cudaStream_t st, int lpt = 0, int per = 0)
+void set_schedule(BatchCache* c, int cluster, int threshold, int sms, cudaStream_t st, int lpt = 0, int per = 0,
+                  int helper = 0)
 {
 	c->cluster = cluster;
 	c->threshold = threshold;
 	c->lpt = lpt;
 	c->per = per;
+	c->helper = helper;
 	const int count = (int)c->bodies.size();
 	std::vector<int> width(count);
 	std::vector<double> t(count);
@@ -232,6 +236,22 @@ std::vector<Snapshot> snapshot_list(BatchCache* c, char* store, size_t* total)
 	return L;
 }
 
+// The second stream of a single-Newton step (split assembly, helper solve launch) and its fork / join
+// events, made once per context
+int use_side_stream(b3g_context* ctx, BatchArgs* A)
+{
+	if (A->newton != 1) return B3G_OK;
+	cudaError_t e = cudaSuccess;
+	if (!ctx->side_stream) e = cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking);
+	if (e == cudaSuccess && !ctx->ev_fork) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
+	if (e == cudaSuccess && !ctx->ev_join) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
+	if (e != cudaSuccess) return cuda_fail(e, "batch side stream");
+	A->side = ctx->side_stream;
+	A->ev_fork = ctx->ev_fork;
+	A->ev_join = ctx->ev_join;
+	return B3G_OK;
+}
+
 cudaError_t run_once(BatchCache* c, const BatchArgs& A, cudaStream_t st) { return op_batch(A, st); }
 
 int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& cfg)
@@ -252,7 +272,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 	// candidates: (cluster size, slices per CTA of a team, queue order)
 	struct Cand
 	{
-		int cl, per, lpt;
+		int cl, per, lpt, helper;
 	};
 	std::vector<Cand> cands;
 	const int clusters[] = {16, 8, 4};
@@ -260,17 +280,20 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 	for (int cl : clusters)
 		if (batch_max_clusters(c->prec, cl) > 0)  // 16-CTA clusters need hardware support
 			for (int p : pers)
-				for (int o = 0; o < 2; ++o) cands.push_back({cl, p, o});
+				for (int o = 0; o < 2; ++o) cands.push_back({cl, p, o, 0});
 	cudaEvent_t e0, e1;
 	cudaEventCreate(&e0);
 	cudaEventCreate(&e1);
 	float best = 1e30f;
-	Cand best_c = {0, 0, 0};
-	for (const Cand& cd : cands)
+	Cand best_c = {0, 0, 0, 0};
+	const size_t plain = cands.size();
+	for (size_t n = 0; n < cands.size(); ++n)
 	{
-		set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per);
+		const Cand cd = cands[n];
+		set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per, cd.helper);
 		BatchArgs A = make_args(c, h, 1, cfg);
-		e = run_once(c, A, st);  // warm-up
+		if (use_side_stream(ctx, &A) != B3G_OK) e = cudaErrorUnknown;
+		if (e == cudaSuccess) e = run_once(c, A, st);  // warm-up
 		if (e == cudaSuccess && c->iters.empty())
 		{
 			// the first warm-up step gives every body's iteration count, which the estimated
@@ -281,8 +304,9 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 				e = cudaErrorUnknown;
 				break;
 			}
-			set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per);
+			set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per, cd.helper);
 			A = make_args(c, h, 1, cfg);
+			use_side_stream(ctx, &A);
 		}
 		for (const Snapshot& s : L) cudaMemcpyAsync((void*)s.src, s.dst, s.bytes, cudaMemcpyDeviceToDevice, st);
 		cudaEventRecord(e0, st);
@@ -293,11 +317,17 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 		if (e != cudaSuccess) break;
 		float ms = 0.0f;
 		cudaEventElapsedTime(&ms, e0, e1);
-		c->tune_log.push_back({cd.lpt * 100000000 + cd.cl * 1000000 + cd.per, (double)ms});
+		c->tune_log.push_back({cd.lpt * 100000000 + cd.cl * 1000000 + cd.helper * 1000 + cd.per, (double)ms});
 		if (ms < best)
 		{
 			best = ms;
 			best_c = cd;
+		}
+		if (n + 1 == plain && cfg.force_iterations <= 1)
+		{
+			// the best of those with a helper launch, and with wider teams for it to take from
+			for (int hw : {8, 4, 2})
+				for (int f : {1, 2, 4}) cands.push_back({best_c.cl, f * best_c.per, best_c.lpt, hw});
 		}
 	}
 	cudaStreamSynchronize(st);
@@ -305,7 +335,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 	cudaEventDestroy(e1);
 	cudaFree(store);
 	if (e != cudaSuccess) return cuda_fail(e, "batch autotune");
-	if (best_c.cl > 0) set_schedule(c, best_c.cl, 0, ctx->sm_count, st, best_c.lpt, best_c.per);
+	if (best_c.cl > 0) set_schedule(c, best_c.cl, 0, ctx->sm_count, st, best_c.lpt, best_c.per, best_c.helper);
 	c->tuned = true;
 	return B3G_OK;
 }
@@ -329,7 +359,7 @@ int build_cache(b3g_context* ctx, b3g_body* const* bodies, uint32_t count, int p
 	std::iota(c->order.begin(), c->order.end(), 0);
 	cudaError_t e = cudaMalloc(&c->d_bodies, std::max<size_t>(1, count) * sizeof(DevBody));
 	if (e == cudaSuccess) e = cudaMalloc(&c->d_order, std::max<size_t>(1, count) * sizeof(int));
-	if (e == cudaSuccess) e = cudaMalloc(&c->d_queue, kQueueCounters * sizeof(unsigned));
+	if (e == cudaSuccess) e = cudaMalloc(&c->d_queue, (kQueueCounters + 1) * sizeof(unsigned));
 	// flat numbering of all bodies' elements and row slices (count + 1 offsets each)
 	std::vector<unsigned> off(2 * (size_t)(count + 1), 0);
 	uint64_t ne = 0, nsl = 0;
@@ -498,18 +528,8 @@ extern "C" int b3g_step_batch(b3g_context* ctx, b3g_body* const* bodies, uint32_
 		}
 	}
 	BatchArgs A = make_args(c, dt, 1, cfg);
-	if (c->elem_mid > 0 && A.newton == 1)
-	{
-		// the split assembly's second stream and fork / join events, made once per context
-		cudaError_t e = cudaSuccess;
-		if (!ctx->side_stream) e = cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking);
-		if (e == cudaSuccess && !ctx->ev_fork) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
-		if (e == cudaSuccess && !ctx->ev_join) e = cudaEventCreateWithFlags(&ctx->ev_join, cudaEventDisableTiming);
-		if (e != cudaSuccess) return cuda_fail(e, "split assembly stream");
-		A.side = ctx->side_stream;
-		A.ev_fork = ctx->ev_fork;
-		A.ev_join = ctx->ev_join;
-	}
+	rc = use_side_stream(ctx, &A);
+	if (rc != B3G_OK) return rc;
 	if (ctx->launch_timing && A.newton == 1)
 	{
 		// timed steps: the two launches of each step bracketed by events, no graph

@@ -151,6 +151,9 @@ struct BatchArgs
 	// of the element and row launches (0: their defaults).
 	cudaStream_t side = nullptr;
 	cudaEvent_t ev_fork = nullptr, ev_join = nullptr;
+	// A second solve launch on `side` (0: none): clusters of `helper` CTAs on the SMs that the first one's
+	// clusters leave free, taking the bodies of teams at most that wide from the same counters.
+	int helper = 0;
 	unsigned elem_mid = 0, slice_mid = 0;
 	int split_elem_per_sm = 0, split_rows_per_sm = 0;
 };

@@ -77,6 +77,19 @@ int elem_grid(unsigned nelem, int per_sm)
 	return (int)(g < cap ? (g > 0 ? g : 1) : cap);
 }
 
+// CTAs of the helper's clusters that the SMs left by the solve launch's clusters can hold
+int helper_room(int prec, int cluster, int helper)
+{
+	static const int sms = [] {
+		int dev = 0, n = 0;
+		cudaGetDevice(&dev);
+		cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+		return n;
+	}();
+	const int m = prec == kP64 ? solve_clusters_f64(cluster) : (prec == kPBF ? solve_clusters_bf16(cluster) : solve_clusters_f32(cluster));
+	return m > 0 ? (sms - m * cluster) / helper * helper : 0;
+}
+
 } // namespace
 
 int batch_max_clusters(int prec, int cluster)
@@ -95,6 +108,7 @@ cudaError_t op_batch(const BatchArgs& A, cudaStream_t st)
 	P.small = A.small;
 	P.nsmall = A.nsmall;
 	P.queue = A.queue;
+	P.solve_ctas = 0;
 	for (int t = 0; t < kTiers; ++t) P.tier_end[t] = A.tier_end[t];
 	P.steps = A.steps;
 	P.h = A.h;
@@ -167,9 +181,24 @@ cudaError_t op_batch(const BatchArgs& A, cudaStream_t st)
 			if (e != cudaSuccess || A.part == 1) return e;
 		}
 	}
-	if (A.prec == kP64) return launch_batch_f64(P, A.cluster, A.ctas, A.part, st);
-	if (A.prec == kPBF) return launch_batch_bf16(P, A.cluster, A.ctas, A.part, st);
-	return launch_batch_f32(P, A.cluster, A.ctas, A.part, st);
+	auto solve = [&](const BatchParams& Q, int cluster, int part, cudaStream_t s) -> cudaError_t {
+		if (A.prec == kP64) return launch_batch_f64(Q, cluster, A.ctas, part, s);
+		if (A.prec == kPBF) return launch_batch_bf16(Q, cluster, A.ctas, part, s);
+		return launch_batch_f32(Q, cluster, A.ctas, part, s);
+	};
+	const int helper_ctas = P.flat && A.side && A.helper > 0 ? helper_room(A.prec, A.cluster, A.helper) : 0;
+	if (helper_ctas <= 0) return solve(P, A.cluster, A.part, st);
+	cudaError_t e = cudaEventRecord(A.ev_fork, st);
+	if (e == cudaSuccess) e = solve(P, A.cluster, A.part, st);
+	if (e == cudaSuccess) e = cudaStreamWaitEvent(A.side, A.ev_fork, 0);
+	// (one more node ahead of the helper: the wide clusters, which need whole GPCs, are placed first)
+	if (e == cudaSuccess) e = cudaMemsetAsync(A.queue + kQueueCounters, 0, sizeof(unsigned), A.side);
+	BatchParams H = P;
+	H.solve_ctas = helper_ctas;
+	if (e == cudaSuccess) e = solve(H, A.helper, 2, A.side);
+	if (e == cudaSuccess) e = cudaEventRecord(A.ev_join, A.side);
+	if (e == cudaSuccess) e = cudaStreamWaitEvent(st, A.ev_join, 0);
+	return e;
 }
 
 } // namespace b3g

@@ -38,6 +38,7 @@ struct BatchParams
 	const int* small;
 	int nsmall;
 	unsigned* queue;
+	int solve_ctas;        // CTAs of the solve launch (0: as many clusters as fit)
 	int tier_end[kTiers];  // of the order `big` (which runs on into `small`): the solve launch's teams
 	int steps;
 	float h;
@@ -770,7 +771,7 @@ cudaError_t launch_cl(const BatchParams& P, int ctas, int bf16, int part, cudaSt
 	const int m = solve_clusters<TA, TV>(CL);
 	cudaLaunchConfig_t cfg;
 	cudaLaunchAttribute attr;
-	cudaError_t e = solve_config<TA, TV>(&cfg, &attr, CL, m > 0 ? m * CL : CL, st);
+	cudaError_t e = solve_config<TA, TV>(&cfg, &attr, CL, P.solve_ctas > 0 ? P.solve_ctas : (m > 0 ? m * CL : CL), st);
 	if (e != cudaSuccess) return e;
 	return cudaLaunchKernelEx(&cfg, k_batch_solve<TA, TV>, P, solve_room());
 }
@@ -908,6 +909,10 @@ cudaError_t launch_batch_bf16(const BatchParams& P, int cluster, int ctas, int p
 cudaError_t launch_rows_f32(const BatchParams& P, cudaStream_t st);
 cudaError_t launch_rows_f64(const BatchParams& P, cudaStream_t st);
 cudaError_t launch_rows_bf16(const BatchParams& P, cudaStream_t st);
+// co-resident clusters of the solve launch
+int solve_clusters_f32(int cluster);
+int solve_clusters_f64(int cluster);
+int solve_clusters_bf16(int cluster);
 int max_clusters_f32(int cluster);
 int max_clusters_f64(int cluster);
 int max_clusters_bf16(int cluster);
