@@ -1,12 +1,14 @@
-// Batched stepping of many independent bodies (b3g_step_batch): one persistent launch
-// (persistent.cu) per call, captured once into a CUDA graph and replayed.
+// Batched stepping of many independent bodies (b3g_step_batch): a step's launches (persistent.cu)
+// captured once into a CUDA graph and replayed.
 //
-// Schedule: bodies are sorted by vertex count, largest first. Bodies with at least `threshold`
-// vertices are stepped by clusters of `cluster` CTAs, the rest by single CTAs. The schedule
-// (cluster size, threshold) is chosen per batch by an autotuner on the first call: it snapshots
-// the mutable state of every body, times one step of each candidate schedule with CUDA events,
-// restores the snapshot and keeps the fastest. Set B3G_AUTOTUNE=0 to use the size heuristic, or
-// B3G_BATCH_SCHEDULE="cluster,threshold" to force a schedule.
+// Schedule: the solve launch runs clusters of `cluster` CTAs, and a body's team is a cluster or the
+// half, quarter, ... of one that gives each CTA about `per` row slices; a second launch of
+// `helper`-CTA clusters can run beside it on the SMs that its clusters leave free. The schedule
+// (cluster, per, helper, queue order) is chosen per batch by an autotuner on the first call: it
+// snapshots the mutable state of every body, times one step of each candidate schedule with CUDA
+// events, restores the snapshot and keeps the fastest. Set B3G_AUTOTUNE=0 to use a fixed rule, or
+// B3G_BATCH_SCHEDULE="cluster,threshold[,lpt[,per[,helper]]]" to force a schedule (without `per`,
+// bodies of `threshold` vertices or more take a whole cluster and the others one CTA).
 #include "api_internal.h"
 
 #include <algorithm>
@@ -32,7 +34,7 @@ struct BatchCache
 	std::vector<b3g_body*> bodies;
 	int prec = 0, precond = 0;
 	DevBody* d_bodies = nullptr;
-	int* d_order = nullptr;      // cluster-stepped bodies, then the others, each longest first
+	int* d_order = nullptr;      // bodies by team width, widest first; within a width longest first
 	unsigned* d_queue = nullptr;
 	std::vector<int> order;
 	std::vector<int> iters;      // PCG iterations of each body's last step (0 = not known yet)
@@ -252,8 +254,6 @@ int use_side_stream(b3g_context* ctx, BatchArgs* A)
 	return B3G_OK;
 }
 
-cudaError_t run_once(BatchCache* c, const BatchArgs& A, cudaStream_t st) { return op_batch(A, st); }
-
 int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& cfg)
 {
 	cudaStream_t st = ctx->stream;
@@ -269,7 +269,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 	std::vector<Snapshot> L = snapshot_list(c, store, &total);
 	for (const Snapshot& s : L) cudaMemcpyAsync(s.dst, s.src, s.bytes, cudaMemcpyDeviceToDevice, st);
 
-	// candidates: (cluster size, slices per CTA of a team, queue order)
+	// candidates: (cluster size, slices per CTA of a team, queue order, cluster size of a helper launch)
 	struct Cand
 	{
 		int cl, per, lpt, helper;
@@ -293,7 +293,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 		set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per, cd.helper);
 		BatchArgs A = make_args(c, h, 1, cfg);
 		if (use_side_stream(ctx, &A) != B3G_OK) e = cudaErrorUnknown;
-		if (e == cudaSuccess) e = run_once(c, A, st);  // warm-up
+		if (e == cudaSuccess) e = op_batch(A, st);  // warm-up
 		if (e == cudaSuccess && c->iters.empty())
 		{
 			// the first warm-up step gives every body's iteration count, which the estimated
@@ -310,7 +310,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 		}
 		for (const Snapshot& s : L) cudaMemcpyAsync((void*)s.src, s.dst, s.bytes, cudaMemcpyDeviceToDevice, st);
 		cudaEventRecord(e0, st);
-		if (e == cudaSuccess) e = run_once(c, A, st);
+		if (e == cudaSuccess) e = op_batch(A, st);
 		cudaEventRecord(e1, st);
 		for (const Snapshot& s : L) cudaMemcpyAsync((void*)s.src, s.dst, s.bytes, cudaMemcpyDeviceToDevice, st);
 		if (e == cudaSuccess) e = cudaEventSynchronize(e1);
@@ -516,11 +516,12 @@ extern "C" int b3g_step_batch(b3g_context* ctx, b3g_body* const* bodies, uint32_
 		if (rc != B3G_OK) return rc;
 		ctx->batch = c;
 		const char* env = std::getenv("B3G_AUTOTUNE");
-		const char* forced = std::getenv("B3G_BATCH_SCHEDULE");  // "cluster,threshold[,lpt]"
-		int fc = 0, ft = 0, fo = 0;
-		if (forced && std::sscanf(forced, "%d,%d,%d", &fc, &ft, &fo) >= 2 &&
-		    (fc == 1 || fc == 2 || fc == 4 || fc == 8 || fc == 16))
-			set_schedule(c, fc, ft > 0 ? ft : (1 << 30), ctx->sm_count, ctx->stream, fo ? 1 : 0);
+		const char* forced = std::getenv("B3G_BATCH_SCHEDULE");  // "cluster,threshold[,lpt[,per[,helper]]]"
+		int fc = 0, ft = 0, fo = 0, fp = 0, fh = 0;
+		auto size = [](int x) { return x == 1 || x == 2 || x == 4 || x == 8 || x == 16; };
+		if (forced && std::sscanf(forced, "%d,%d,%d,%d,%d", &fc, &ft, &fo, &fp, &fh) >= 2 && size(fc))
+			set_schedule(c, fc, ft > 0 ? ft : (1 << 30), ctx->sm_count, ctx->stream, fo ? 1 : 0, std::max(fp, 0),
+			             size(fh) && fh > 1 && fh < fc ? fh : 0);
 		else if (!(env && env[0] == '0'))
 		{
 			rc = autotune(ctx, c, dt, cfg);
@@ -539,7 +540,7 @@ extern "C" int b3g_step_batch(b3g_context* ctx, b3g_body* const* bodies, uint32_
 		{
 			cudaError_t e = cudaEventRecord(ctx->tev[0], st);
 			A.part = 1;
-			A.ev_rows = A.side ? nullptr : ctx->tev[3];  // no single element/row boundary when split
+			A.ev_rows = A.elem_mid > 0 ? nullptr : ctx->tev[3];  // no single element/row boundary when split
 			if (e == cudaSuccess) e = op_batch(A, st);
 			A.ev_rows = nullptr;
 			if (e == cudaSuccess) e = cudaEventRecord(ctx->tev[1], st);
@@ -551,7 +552,7 @@ extern "C" int b3g_step_batch(b3g_context* ctx, b3g_body* const* bodies, uint32_
 			float m1 = 0.0f, m2 = 0.0f, m3 = 0.0f;
 			cudaEventElapsedTime(&m1, ctx->tev[0], ctx->tev[1]);
 			cudaEventElapsedTime(&m2, ctx->tev[1], ctx->tev[2]);
-			if (!A.side) cudaEventElapsedTime(&m3, ctx->tev[0], ctx->tev[3]);
+			if (A.elem_mid == 0) cudaEventElapsedTime(&m3, ctx->tev[0], ctx->tev[3]);
 			ctx->t_assembly_ms += m1;
 			ctx->t_elements_ms += m3;
 			ctx->t_pcg_ms += m2;
