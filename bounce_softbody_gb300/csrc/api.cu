@@ -1,5 +1,5 @@
-// C ABI of b3g (include/b3g.h): contexts, bodies, the single-body step (per-op kernels) and
-// state transfer. The batch entry point lives in batch.cu.
+// C ABI of b3g (include/b3g.h): contexts, bodies, the single-body step (elements, rows and
+// one solve launch per Newton iteration) and state transfer. The batch entry point lives in batch.cu.
 #include "api_internal.h"
 #include "forces.h"
 #include "shapes.h"

@@ -79,7 +79,7 @@ struct PrecBuffers
 	void* minv = nullptr;
 	void* alo = nullptr;
 	float* xff = nullptr;  // float-float solution (FP32 and BF16 modes), 8 floats per vertex
-	// BF16 mode of the per-op step: the inner solve's z, r, d, q (4-wide), used where the solve's
+	// BF16 mode of the single-body step: the inner solve's z, r, d, q (4-wide), used where the solve's
 	// shared memory has no room for them
 	void* fcg_vec[4] = {};
 };
@@ -119,7 +119,7 @@ int cuda_fail(cudaError_t e, const char* where);
 void reset_mass(b3g_body* b);
 int upload_masses(b3g_body* b);
 int ensure_precision(b3g_body* b, int prec);
-// refine: the per-op path's iterative refinement (float-float solution and refresh residual)
+// refine: the single-body step's iterative refinement (float-float solution and refresh residual)
 DevBody dev_for(const b3g_body* b, int prec, int precond, bool refine = false);
 int prec_of(const b3g_solver_config* c);
 // filter_ok: the caller steps filtered contacts (b3g_body_step, b3g_step_batch)

@@ -50,7 +50,7 @@ struct BatchCache
 	// graph of (memset queue, batch launch) for one step with the current parameters
 	cudaGraphExec_t graph = nullptr;
 	float g_h = 0.0f;
-	int g_steps = 0, g_newton = 0, g_max_iter = 0, g_refresh = 0;
+	int g_newton = 0, g_max_iter = 0, g_refresh = 0;
 	double g_tol2 = 0.0, g_ntol2 = 0.0;
 	std::vector<std::pair<int, double>> tune_log;  // (cluster * 1e6 + threshold, ms)
 	unsigned long long* d_prof = nullptr;          // phase cycle counters when B3G_PHASE_PROFILE=1

@@ -1,5 +1,5 @@
-// Device building blocks of the implicit step, shared by the per-op kernels (kernels.cu) and
-// the persistent batch kernel (persistent.cu). Matrices in registers are row-major float[9].
+// Device building blocks of the implicit step, shared by the single-body kernels (kernels.cu,
+// solve.cu) and the batch kernels (persistent.cu). Matrices in registers are row-major float[9].
 #pragma once
 
 #include "internal.h"
@@ -29,17 +29,10 @@ struct LdCG
 	template <class T> static __device__ __forceinline__ T ld(const T* p) { return __ldcg(p); }
 };
 
-// Matrix streams of the SpMV. MatNC: for a large body stepped by the per-op kernels, whose
-// matrix (larger than L2) is read once per product: read-only path with an L2 evict-first policy,
-// so the vector the SpMV gathers from stays in L2 while the matrix streams past it. MatCG: the
-// same policy through L2-coherent loads (for a kernel that assembles the matrix earlier in the
-// same launch). MatVia<L>: the loads of policy L without a cache hint, for the persistent batch
-// kernel, where a small body's matrix is re-read from L2 by every PCG iteration (evict-first
-// measured 6% slower on the 512-body batch).
+// Matrix streams of the SpMV. MatNC: read-only path past L1 with an L2 eviction policy of the
+// caller's, for a matrix that earlier launches wrote. MatVia<L>: the loads of policy L without a
+// hint, for the persistent batch kernel, which assembles the matrix in the same launch.
 struct MatNC
-{
-};
-struct MatCG
 {
 };
 template <class L>
@@ -78,15 +71,6 @@ __device__ __forceinline__ uint4 mat_ld16<MatNC>(const void* p, unsigned long lo
 	    : "l"(p), "l"(pol));
 	return r;
 }
-template <>
-__device__ __forceinline__ uint4 mat_ld16<MatCG>(const void* p, unsigned long long pol)
-{
-	uint4 r;
-	asm volatile("ld.global.cg.L2::cache_hint.v4.u32 {%0, %1, %2, %3}, [%4], %5;"
-	             : "=r"(r.x), "=r"(r.y), "=r"(r.z), "=r"(r.w)
-	             : "l"(p), "l"(pol));
-	return r;
-}
 template <class M>
 __device__ __forceinline__ uint2 mat_ld8(const void* p, unsigned long long pol);
 template <>
@@ -94,13 +78,6 @@ __device__ __forceinline__ uint2 mat_ld8<MatNC>(const void* p, unsigned long lon
 {
 	uint2 r;
 	asm("ld.global.nc.L1::no_allocate.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(r.x), "=r"(r.y) : "l"(p), "l"(pol));
-	return r;
-}
-template <>
-__device__ __forceinline__ uint2 mat_ld8<MatCG>(const void* p, unsigned long long pol)
-{
-	uint2 r;
-	asm volatile("ld.global.cg.L2::cache_hint.v2.u32 {%0, %1}, [%2], %3;" : "=r"(r.x), "=r"(r.y) : "l"(p), "l"(pol));
 	return r;
 }
 
@@ -252,11 +229,6 @@ __device__ __forceinline__ float3 mv9(const float* M, float3 v)
 {
 	return f3(M[0] * v.x + M[1] * v.y + M[2] * v.z, M[3] * v.x + M[4] * v.y + M[5] * v.z,
 	          M[6] * v.x + M[7] * v.y + M[8] * v.z);
-}
-__device__ __forceinline__ float3 mtv9(const float* M, float3 v)
-{
-	return f3(M[0] * v.x + M[3] * v.y + M[6] * v.z, M[1] * v.x + M[4] * v.y + M[7] * v.z,
-	          M[2] * v.x + M[5] * v.y + M[8] * v.z);
 }
 
 // quat.h:133 GetRotationMatrix, row-major
@@ -1752,18 +1724,12 @@ __device__ __forceinline__ void mat_load4(const TA* p, AT o[4], unsigned long lo
 {
 	hinted_load4<MatNC>(p, o, pol);
 }
-template <class TA, class AT>
-__device__ __forceinline__ void mat_load4(const TA* p, AT o[4], unsigned long long pol, MatCG*)
-{
-	hinted_load4<MatCG>(p, o, pol);
-}
 template <class L>
 __device__ __forceinline__ int4 mat_cols(const int* p, unsigned long long, MatVia<L>*)
 {
 	return __ldg((const int4*)p);  // column ids never change after creation
 }
 __device__ __forceinline__ int4 mat_cols(const int* p, unsigned long long pol, MatNC*) { return hinted_cols<MatNC>(p, pol); }
-__device__ __forceinline__ int4 mat_cols(const int* p, unsigned long long pol, MatCG*) { return hinted_cols<MatCG>(p, pol); }
 
 // q_i = (A x)_i for row i = 32 s + lane of a slice of width w (a multiple of 4). Per group of
 // four blocks a lane issues one 16-byte load of column ids, one vector load per value plane and
@@ -1802,108 +1768,12 @@ __device__ __forceinline__ void spmv_row(const TA* A, const int* __restrict__ co
 	out[2] = (TV)o2;
 }
 
-// (A x)_i in float-float for the refinement residual: FP32 blocks times the float-float
-// solution, every product split into its float value and rounding error, summed in
-// float-float. Returns hi + lo per component.
-__device__ __forceinline__ void spmv_row_ff(const float* A, const int* __restrict__ col, int nslots, int base, int w,
-                                            int lane, const float* xff, float ohi[3], float olo[3])
-{
-	float h0 = 0, h1 = 0, h2 = 0, l0 = 0, l1 = 0, l2 = 0;
-	const size_t ns = (size_t)nslots;
-	const unsigned long long pol = evict_first_policy();
-	for (int k = 0; k < w; k += kGroup)
-	{
-		const size_t off = block_slot((size_t)base, k, lane);
-		const int4 jj = mat_cols(col + off, pol, (MatNC*)nullptr);
-		float a[9][4];
-#pragma unroll
-		for (int p = 0; p < 9; ++p) mat_load4(A + p * ns + off, a[p], pol, (MatNC*)nullptr);
-		const int js[4] = {jj.x, jj.y, jj.z, jj.w};
-#pragma unroll
-		for (int u = 0; u < 4; ++u)
-		{
-			float xh[3], xl[3];
-			ff_ld(xff, js[u], xh, xl);
-#pragma unroll
-			for (int c = 0; c < 3; ++c)
-			{
-				const float a0 = a[3 * 0 + c][u], a1 = a[3 * 1 + c][u], a2 = a[3 * 2 + c][u];
-				// row 0, 1, 2 of the block times component c of x_j
-				float p = __fmul_rn(a0, xh[c]);
-				ff_add(h0, l0, p, fmaf(a0, xh[c], -p) + a0 * xl[c]);
-				p = __fmul_rn(a1, xh[c]);
-				ff_add(h1, l1, p, fmaf(a1, xh[c], -p) + a1 * xl[c]);
-				p = __fmul_rn(a2, xh[c]);
-				ff_add(h2, l2, p, fmaf(a2, xh[c], -p) + a2 * xl[c]);
-			}
-		}
-	}
-	ohi[0] = h0; ohi[1] = h1; ohi[2] = h2;
-	olo[0] = l0; olo[1] = l1; olo[2] = l2;
-}
-
 // b - (hi + lo), rounded once to float
 __device__ __forceinline__ float ff_residual(float b, float hi, float lo)
 {
 	float t, e;
 	two_sum(b, -hi, t, e);
 	return __fadd_rn(t, __fsub_rn(e, lo));
-}
-
-// The SpMV of a PCG iteration with the direction update folded in: q_i = (A d')_i with
-// d' = s + beta d, the new direction, formed from the gathered s and d of every column
-// (first iteration of a solve: d' = s). The diagonal block leads every row, so the first gathered
-// column is the row itself and its d'_i is returned in dn. Every lane forms d'_j with the same
-// expression as the owner of row j, so all copies of a value agree bitwise.
-template <class TV, class L = LdPlain>
-__device__ __forceinline__ void gather_dir(const TV* s, const TV* d, TV beta, bool first, int j, TV o[3])
-{
-	vld<TV, L>(s, j, o);
-	if (first) return;
-	TV dj[3];
-	vld<TV, L>(d, j, dj);
-#pragma unroll
-	for (int c = 0; c < 3; ++c) o[c] = o[c] + beta * dj[c];
-}
-
-template <class TA, class TV, class L = LdPlain, class M = MatNC>
-__device__ __forceinline__ void spmv_row_dir(const TA* A, const int* __restrict__ col, int nslots, int base, int w,
-                                             int lane, const TV* s, const TV* d, TV beta, bool first, TV out[3],
-                                             TV dn[3])
-{
-	typedef typename Acc<TA>::type AT;
-	AT o0 = 0, o1 = 0, o2 = 0;
-	const size_t ns = (size_t)nslots;
-	const unsigned long long pol = evict_first_policy();
-	for (int k = 0; k < w; k += kGroup)
-	{
-		const size_t off = block_slot((size_t)base, k, lane);
-		const int4 jj = mat_cols(col + off, pol, (M*)nullptr);
-		AT a[9][4];
-#pragma unroll
-		for (int p = 0; p < 9; ++p) mat_load4(A + p * ns + off, a[p], pol, (M*)nullptr);
-		TV xv[4][3];
-		gather_dir<TV, L>(s, d, beta, first, jj.x, xv[0]);
-		gather_dir<TV, L>(s, d, beta, first, jj.y, xv[1]);
-		gather_dir<TV, L>(s, d, beta, first, jj.z, xv[2]);
-		gather_dir<TV, L>(s, d, beta, first, jj.w, xv[3]);
-		if (k == 0)
-		{
-#pragma unroll
-			for (int c = 0; c < 3; ++c) dn[c] = xv[0][c];
-		}
-#pragma unroll
-		for (int u = 0; u < 4; ++u)
-		{
-			const AT x0 = (AT)xv[u][0], x1 = (AT)xv[u][1], x2 = (AT)xv[u][2];
-			o0 += a[0][u] * x0 + a[1][u] * x1 + a[2][u] * x2;
-			o1 += a[3][u] * x0 + a[4][u] * x1 + a[5][u] * x2;
-			o2 += a[6][u] * x0 + a[7][u] * x1 + a[8][u] * x2;
-		}
-	}
-	out[0] = (TV)o0;
-	out[1] = (TV)o1;
-	out[2] = (TV)o2;
 }
 
 // M^-1 r for one row (scalar or block Jacobi)

@@ -52,8 +52,6 @@ struct Scalars
 {
 	double delta;      // r.s of the current residual
 	double delta0;     // r0.s0
-	double dq;         // d.q
-	double alpha, beta;
 	double tol2;       // pcg_tolerance^2
 	double newton_err, newton_err0;
 	double newton_tol2;
@@ -65,8 +63,6 @@ struct Scalars
 	int newton_done;
 	int min_it, max_it;
 	int refresh;       // refresh period
-	unsigned counter;  // arrival counter of the deterministic grid reduction (plain path)
-	int pending_check; // bf16 mode: recursive residual met the tolerance, confirm with a refresh
 	int fault;         // a bounded device wait expired (the step's results are not valid)
 	unsigned long long total_iters;  // PCG iterations of every step since creation
 	unsigned long long total_steps;
@@ -116,7 +112,7 @@ struct TeamMemory
 	unsigned long long tagged[2][kTeamReplicas][kTeamMax];
 };
 
-// Everything a kernel needs about one body. Passed by value to the per-op kernels and read
+// Everything a kernel needs about one body. Passed by value to the single-body kernels and read
 // from a device array by the persistent batch kernel.
 struct DevBody
 {
@@ -206,7 +202,7 @@ struct DevBody
 	uint8_t* c_apply;
 	float* c_nf;                // accumulated normal force
 	float* c_normal;            // 3 per contact
-	// filtered contacts (B3G_CONTACT_FILTER, per-op step only; null otherwise): per vertex the
+	// filtered contacts (B3G_CONTACT_FILTER; null otherwise): per vertex the
 	// constrained normal n (zero when free) and the normal velocity change zn of z = zn n
 	float4* filt;
 
@@ -218,7 +214,7 @@ struct DevBody
 	void* q;
 	void* s;
 	void* py;
-	float* xff;                 // float-float solution for iterative refinement (per-op path, FP32
+	float* xff;                 // float-float solution for iterative refinement (single-body step, FP32
 	                            // and BF16 modes): 8 floats per vertex, (hi x, y, z, 0) then
 	                            // (lo x, y, z, 0); null = the solution is py
 

@@ -1,6 +1,5 @@
-// Per-op kernels of the single-body ("plain") path: one kernel per phase, grid-wide
-// deterministic reductions (per-CTA partials summed in a fixed order by the last CTA to
-// arrive), solver decisions taken on the device in Scalars.
+// Single-body kernels other than the solve (solve.cu): elements, row assembly, contact filter,
+// state transfer, ray casts.
 #include "device.cuh"
 #include "ops.h"
 
@@ -352,11 +351,8 @@ StepParams dev_params(const StepParamsHost& P)
 
 int slice_grid(const DevBody& B) { return grid_for(B.nslices, kWarps); }
 
-// Grid of the per-vertex kernels (vector update, final update): at most two CTAs per SM, each
-// thread striding over several vertices. One vertex per thread (1024 CTAs on the 64³ block) made
-// the vector update 1.6x slower: every CTA pays the reduction's fence and its atomic on one
-// counter. Measured per 64³ step: 17.9 ms (one vertex a thread), 17.3 (4 CTAs/SM), 16.7 (2),
-// 17.3 (1). B3G_VERTEX_CTAS overrides the cap (tuning knob, read once).
+// Grid of the per-vertex kernels (contact filter, steps without a solve, types): at most two CTAs
+// per SM, each thread striding over several vertices. B3G_VERTEX_CTAS overrides the cap (read once).
 int vertex_grid(const DevBody& B)
 {
 	static const int cap = [] {

@@ -1,15 +1,13 @@
-// Host-callable launchers of the per-op kernels (kernels.cu) and of the persistent batch
-// kernel (persistent.cu).
+// Host-callable launchers of the single-body kernels (kernels.cu, solve.cu) and of the batch kernels
+// (persistent.cu).
 #pragma once
 
 #include "internal.h"
 
 #include <cuda_runtime.h>
 
-// Threads per CTA of the batch kernel's team launches (the PCG launch and the team assembly).
-// On the 512-body batch with every body on a cluster, 256-thread CTAs at 4 per SM (clusters of
-// 8) measured 1 % faster than 512-thread CTAs at 2 per SM (clusters of 4); with small bodies on
-// single CTAs it was the other way round.
+// Threads per CTA of the whole-step launch (several Newton iterations) and of the team assembly; the
+// single-Newton solve launch sets its own (kSolveMaxThreads).
 #ifndef B3G_PCG_THREADS
 #define B3G_PCG_THREADS 256
 #endif

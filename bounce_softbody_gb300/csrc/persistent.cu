@@ -1,4 +1,4 @@
-// Dispatch of the persistent batch kernel (persistent.cuh) to its per-precision instantiations.
+// Dispatch of the batch kernels (persistent.cuh) to their per-precision instantiations.
 #include "persistent.cuh"
 
 namespace b3g {

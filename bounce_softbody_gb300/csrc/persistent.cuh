@@ -1,6 +1,7 @@
-// Persistent batch kernel: many independent bodies step in one launch.
+// Batch kernels: many independent bodies step in one launch (k_batch, several Newton iterations) or in
+// an element, a row and a solve launch (k_batch_solve, one Newton iteration).
 //
-// A body is owned by a team: either a thread-block cluster of CL CTAs (large bodies) or a
+// k_batch: a body is owned by a team: either a thread-block cluster of CL CTAs (large bodies) or a
 // single CTA (small bodies). The team runs the whole implicit step of its body without leaving
 // the kernel: element phase, row assembly, PCG, final update. Team-wide synchronisation is the
 // hardware cluster barrier (or __syncthreads for one CTA); dot products are reduced per warp by
@@ -12,6 +13,9 @@
 //
 // Work distribution: bodies are sorted by size (largest first). Clusters first take large bodies
 // from a global counter; when those run out every CTA takes small bodies on its own.
+//
+// k_batch_solve: the solve of solve.cuh by teams of a cluster or of the half, quarter, ... of one, each
+// width taking its bodies from its own counter, widest first.
 //
 // This header holds the kernel templates; persistent_{f32,f64,bf16}.cu instantiate one
 // precision each (compiled in parallel) and persistent.cu dispatches.
@@ -449,8 +453,7 @@ __device__ void team_finish(Team<CL>& T, const DevBody& B, const BatchParams& P,
 }
 
 // The whole implicit step of one body by one team (any number of Newton iterations); mirrors
-// the per-op path of kernels.cu phase for phase (same device functions, same reduction
-// decisions).
+// the single-body step phase for phase (same device functions, same solver decisions).
 template <int CL, class TA, class TV>
 __device__ void team_step(Team<CL>& T, const DevBody& B, const BatchParams& P, bool bf16)
 {

@@ -1,5 +1,5 @@
-// Serving loop: step requests for many bodies, continuously batched into the persistent batch
-// kernel (persistent.cu).
+// Serving loop: step requests for many bodies, continuously batched into the batch kernels
+// (persistent.cu).
 //
 // A client registers bodies (host copies of their descriptions) and submits requests "step body
 // b n times". A worker thread repeats: admit waiting requests (a body must be resident on the

@@ -9,8 +9,8 @@
 // only when a write names a new (i, j) or an operation needs the union of two patterns; values
 // live on the device only. Writes queued by the add / set calls are applied on the device in
 // call order per entry (one thread per written block, its writes in order), so results do not
-// depend on thread scheduling. The CG reuses the per-op PCG kernels of the body step
-// (kernels.cu) on this layout.
+// depend on thread scheduling. The CG is the solve launch of the body step (solve.cu)
+// on this layout.
 #include "api_internal.h"
 #include "device.cuh"
 #include "../../include/b3g_sparse.h"

@@ -249,8 +249,8 @@ B3G_API int b3g_body_device_bytes(const b3g_body* body, uint64_t* bytes);
  * in which case the call waits and fills stats. dt <= 0 skips the solve like the reference. */
 B3G_API int b3g_body_step(b3g_body* body, float dt, const b3g_solver_config* config, b3g_step_stats* stats);
 
-/* `steps` steps of `count` independent bodies of one context in one persistent launch per
- * size bucket (captured once in a CUDA graph and replayed). stats, if non-NULL, receives the
+/* `steps` steps of `count` independent bodies of one context in a few launches per step
+ * (captured once in a CUDA graph and replayed). stats, if non-NULL, receives the
  * last step's statistics of each body (count entries) and makes the call wait. */
 B3G_API int b3g_step_batch(b3g_context* ctx, b3g_body* const* bodies, uint32_t count, float dt,
                    const b3g_solver_config* config, uint32_t steps, b3g_step_stats* stats);
@@ -264,8 +264,8 @@ B3G_API int b3g_step_batch(b3g_context* ctx, b3g_body* const* bodies, uint32_t c
  * fails with B3G_ERROR_UNSUPPORTED). Differences from b3g_step_batch: each body must already have
  * solver buffers for the requested precision (FP32 always does; FP64 / BF16 after a first step in
  * that precision), where b3g_step_batch creates them; dt must be > 0 (b3g_step_batch steps each
- * body alone for dt <= 0); the schedule is a fixed size rule (clusters of 4 CTAs of 256 threads
- * for bodies of 4096 vertices or more, single CTAs below), not autotuned. The first call on a device looks the
+ * body alone for dt <= 0); the schedule is a fixed size rule (clusters of 4 CTAs for bodies
+ * of 4096 vertices or more, single CTAs below), not autotuned. The first call on a device looks the
  * array up and clears it (set-up): make that first call before any stream capture. Each call
  * copies the body descriptors to the device from static host arrays of the library, which the
  * next call rewrites. Every call reuses the same device array, so calls whose work overlaps on the
@@ -292,7 +292,7 @@ B3G_API int b3g_batch_assembly_split(b3g_context* ctx, uint32_t out[4]);
 B3G_API int b3g_batch_phase_cycles(b3g_context* ctx, uint64_t out[8], int reset);
 
 /* Launch timing of batched steps (measurement aid, no reference counterpart). While on, a
- * single-Newton b3g_step_batch launches its two kernels (elements + assembly, then PCG + final
+ * single-Newton b3g_step_batch launches its kernels (elements + assembly, then PCG + final
  * update) directly instead of replaying its graph, records CUDA events around each and waits
  * for them; b3g_batch_launch_times returns the accumulated device milliseconds of the assembly
  * launches and of the PCG launches and the number of timed steps (out[0..2]). */
