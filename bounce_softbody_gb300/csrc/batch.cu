@@ -238,11 +238,11 @@ std::vector<Snapshot> snapshot_list(BatchCache* c, char* store, size_t* total)
 	return L;
 }
 
-// The second stream of a single-Newton step (split assembly, helper solve launch) and its fork / join
+// The second stream of a step in flat launches (split assembly, helper solve launch) and its fork / join
 // events, made once per context
 int use_side_stream(b3g_context* ctx, BatchArgs* A)
 {
-	if (A->newton != 1) return B3G_OK;
+	if (A->newton > kFlatNewton) return B3G_OK;
 	cudaError_t e = cudaSuccess;
 	if (!ctx->side_stream) e = cudaStreamCreateWithFlags(&ctx->side_stream, cudaStreamNonBlocking);
 	if (e == cudaSuccess && !ctx->ev_fork) e = cudaEventCreateWithFlags(&ctx->ev_fork, cudaEventDisableTiming);
@@ -323,7 +323,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 			best = ms;
 			best_c = cd;
 		}
-		if (n + 1 == plain && cfg.force_iterations <= 1)
+		if (n + 1 == plain && cfg.force_iterations <= (uint32_t)kFlatNewton)
 		{
 			// the best of those with a helper launch, and with wider teams for it to take from
 			for (int hw : {8, 4, 2})

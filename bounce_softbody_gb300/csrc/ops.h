@@ -128,12 +128,12 @@ struct BatchArgs
 	int cluster;             // CTAs per cluster: 1, 2, 4 or 8
 	int ctas;                // CTAs of the launch (multiple of cluster)
 	unsigned long long* prof; // optional phase cycle counters (8 per CTA), null = off
-	int part = 0;            // single-Newton steps: 0 both launches, 1 assembly only, 2 PCG only
+	int part = 0;            // single-Newton steps: 0 every launch, 1 assembly only, 2 PCG only
 	cudaEvent_t ev_rows = nullptr;  // if set, recorded between the element and the row launches
-	// single-Newton steps: the elements, then the rows, of all bodies in two flat launches before
+	// up to kFlatNewton iterations: the elements, then the rows, of all bodies in two flat launches before
 	// the PCG launch. elem_off[k] / slice_off[k]: first element / row slice of bodies[k] in the
 	// flat numbering (count + 1 entries each; elements of a body: tetrahedra, triangles, springs,
-	// stretch/shear triangles, mouse springs). Null = the team launches do both, as for several
+	// stretch/shear triangles, mouse springs). Null = the team launches do both, as for many
 	// Newton iterations.
 	const unsigned* elem_off = nullptr;
 	const unsigned* slice_off = nullptr;
@@ -160,6 +160,12 @@ inline void two_tiers(BatchArgs* A, int cluster, int nbig, int count)
 {
 	for (int t = 0; t < kTiers; ++t) A->tier_end[t] = t == kTiers - 1 ? count : ((kMaxTeamCtas >> t) <= cluster ? nbig : 0);
 }
+// Newton iterations of a batched step that take launches of their own (elements, rows, solve), ms a step
+// in one launch -> in launches of their own: 12 uneven blocks x 3 iterations 3.3 -> 1.4, 160 blocks 9.5 ->
+// 4.6, 24 blocks and cloths 33.8 -> 11.8; 16 allowed and two or three taken 2.3 -> 1.3, 6.1 -> 3.8. An
+// allowed iteration that no body takes costs its launches some 10 us, so a step that may take more is
+// one launch of the whole-step kernel, which stops at each body's last iteration.
+constexpr int kFlatNewton = 16;
 cudaError_t op_batch(const BatchArgs& A, cudaStream_t st);
 // Co-resident clusters of the batch kernel for this precision and cluster size (0 on error).
 int batch_max_clusters(int prec, int cluster);

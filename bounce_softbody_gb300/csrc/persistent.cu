@@ -10,7 +10,7 @@ constexpr int kElemThreads = 256;
 // The elements of every body of a batch (tetrahedra, triangles, springs, stretch / shear
 // triangles, mouse springs, then the vertices of bodies with filtered contacts; first Newton
 // iteration of a step), one per thread over a flat
-// numbering (elem_off: first element of each body). Its own launch runs at its own register
+// numbering (elem_off: first element of each body; LATER: a Newton iteration after the first). Its own launch runs at its own register
 // budget (3 CTAs per SM) instead of the 128 registers the row assembly needs: the tetrahedra's
 // rotation extraction, a dependent chain, wants the extra warps. The state it reads was written
 // by earlier launches, so plain (L1) loads. TETS: every body has tetrahedra only (and no filtered
@@ -18,16 +18,17 @@ constexpr int kElemThreads = 256;
 #ifndef B3G_ELEM_TETS_MIN_BLOCKS
 #define B3G_ELEM_TETS_MIN_BLOCKS 4
 #endif
-template <bool TETS>
+template <bool TETS, bool LATER>
 __global__ void __launch_bounds__(kElemThreads, TETS ? B3G_ELEM_TETS_MIN_BLOCKS : 3) k_batch_elements(BatchParams P)
 {
 	StepParams sp;
 	sp.h = P.h;
-	sp.first_newton = 1;
+	sp.first_newton = LATER ? 0 : 1;
 	for (unsigned g = P.g_begin + blockIdx.x * blockDim.x + threadIdx.x; g < P.nelem; g += gridDim.x * blockDim.x)
 	{
 		const int b = flat_body(P.elem_off, P.nbodies, g);
 		const DevBody& B = P.bodies[b];
+		if (LATER && B.sc->newton_done) continue;
 		int e = (int)(g - __ldg(P.elem_off + b));
 		if (TETS || e < B.nt)
 		{
@@ -60,7 +61,7 @@ __global__ void __launch_bounds__(kElemThreads, TETS ? B3G_ELEM_TETS_MIN_BLOCKS 
 		}
 		// filtered contacts: the body's vertices follow its elements in the numbering; the
 		// contact update and each vertex's constraint at the step's start (no element reads them)
-		contact_filter_vertex(B, e - B.nms, P.h);
+		if (!LATER) contact_filter_vertex(B, e - B.nms, P.h);
 	}
 }
 
@@ -90,47 +91,9 @@ int helper_room(int prec, int cluster, int helper)
 	return m > 0 ? (sms - m * cluster) / helper * helper : 0;
 }
 
-} // namespace
-
-int batch_max_clusters(int prec, int cluster)
+// The launches of Newton iteration P.k (the whole step when P.flat is not set)
+cudaError_t launch_iteration(const BatchArgs& A, const BatchParams& P, cudaStream_t st)
 {
-	if (prec == kP64) return max_clusters_f64(cluster);
-	if (prec == kPBF) return max_clusters_bf16(cluster);
-	return max_clusters_f32(cluster);
-}
-
-cudaError_t op_batch(const BatchArgs& A, cudaStream_t st)
-{
-	BatchParams P;
-	P.bodies = A.bodies;
-	P.big = A.big;
-	P.nbig = A.nbig;
-	P.small = A.small;
-	P.nsmall = A.nsmall;
-	P.queue = A.queue;
-	P.solve_ctas = 0;
-	for (int t = 0; t < kTiers; ++t) P.tier_end[t] = A.tier_end[t];
-	P.steps = A.steps;
-	P.h = A.h;
-	P.newton = A.newton < 1 ? 1 : A.newton;
-	P.max_iter = A.max_iter;
-	P.tol2 = A.tol2;
-	P.refresh = A.refresh;
-	P.newton_tol2 = A.newton_tol2;
-	P.prof = A.prof;
-	P.elem_off = A.elem_off;
-	P.slice_off = A.slice_off;
-	P.nelem = A.nelem;
-	P.nslices = A.nslices;
-	P.nbodies = A.nbodies;
-	P.tets_only = A.tets_only;
-	P.filter = A.filter;
-	P.g_begin = 0;
-	P.s_begin = 0;
-	P.rows_per_sm = 0;
-	// a single Newton iteration with the flat numbering: elements and rows in two flat launches,
-	// then the PCG launch (which knows from `flat` to sum delta0 itself)
-	P.flat = (P.newton == 1 && A.elem_off && A.slice_off && A.nslices > 0) ? 1 : 0;
 	if (A.part != 2)
 	{
 		// the solve-only part reuses what the assembly part cleared
@@ -143,10 +106,17 @@ cudaError_t op_batch(const BatchArgs& A, cudaStream_t st)
 			auto elements = [&](const BatchParams& Q, int per_sm, cudaStream_t s) -> cudaError_t {
 				const unsigned count = Q.nelem - Q.g_begin;
 				if (count == 0) return cudaSuccess;
+				const int grid = elem_grid(count, per_sm > 0 ? per_sm : (Q.tets_only ? B3G_ELEM_TETS_MIN_BLOCKS : 3));
 				if (Q.tets_only)
-					k_batch_elements<true><<<elem_grid(count, per_sm > 0 ? per_sm : B3G_ELEM_TETS_MIN_BLOCKS), kElemThreads, 0, s>>>(Q);
+				{
+					if (Q.k > 0) k_batch_elements<true, true><<<grid, kElemThreads, 0, s>>>(Q);
+					else k_batch_elements<true, false><<<grid, kElemThreads, 0, s>>>(Q);
+				}
 				else
-					k_batch_elements<false><<<elem_grid(count, per_sm > 0 ? per_sm : 3), kElemThreads, 0, s>>>(Q);
+				{
+					if (Q.k > 0) k_batch_elements<false, true><<<grid, kElemThreads, 0, s>>>(Q);
+					else k_batch_elements<false, false><<<grid, kElemThreads, 0, s>>>(Q);
+				}
 				return cudaGetLastError();
 			};
 			auto rows = [&](const BatchParams& Q, cudaStream_t s) -> cudaError_t {
@@ -198,6 +168,57 @@ cudaError_t op_batch(const BatchArgs& A, cudaStream_t st)
 	if (e == cudaSuccess) e = solve(H, A.helper, 2, A.side);
 	if (e == cudaSuccess) e = cudaEventRecord(A.ev_join, A.side);
 	if (e == cudaSuccess) e = cudaStreamWaitEvent(st, A.ev_join, 0);
+	return e;
+}
+
+} // namespace
+
+int batch_max_clusters(int prec, int cluster)
+{
+	if (prec == kP64) return max_clusters_f64(cluster);
+	if (prec == kPBF) return max_clusters_bf16(cluster);
+	return max_clusters_f32(cluster);
+}
+
+cudaError_t op_batch(const BatchArgs& A, cudaStream_t st)
+{
+	BatchParams P;
+	P.bodies = A.bodies;
+	P.big = A.big;
+	P.nbig = A.nbig;
+	P.small = A.small;
+	P.nsmall = A.nsmall;
+	P.queue = A.queue;
+	P.solve_ctas = 0;
+	for (int t = 0; t < kTiers; ++t) P.tier_end[t] = A.tier_end[t];
+	P.steps = A.steps;
+	P.h = A.h;
+	P.newton = A.newton < 1 ? 1 : A.newton;
+	P.max_iter = A.max_iter;
+	P.tol2 = A.tol2;
+	P.refresh = A.refresh;
+	P.newton_tol2 = A.newton_tol2;
+	P.prof = A.prof;
+	P.elem_off = A.elem_off;
+	P.slice_off = A.slice_off;
+	P.nelem = A.nelem;
+	P.nslices = A.nslices;
+	P.nbodies = A.nbodies;
+	P.tets_only = A.tets_only;
+	P.filter = A.filter;
+	P.g_begin = 0;
+	P.s_begin = 0;
+	P.rows_per_sm = 0;
+	// with the flat numbering each Newton iteration is an element launch, a row launch and a PCG launch
+	// (which knows from `flat` to sum delta0 itself)
+	P.flat = (P.newton <= kFlatNewton && A.elem_off && A.slice_off && A.nslices > 0) ? 1 : 0;
+	P.k = 0;
+	cudaError_t e = launch_iteration(A, P, st);
+	for (int k = 1; P.flat && k < P.newton && e == cudaSuccess; ++k)
+	{
+		P.k = k;
+		e = launch_iteration(A, P, st);
+	}
 	return e;
 }
 

@@ -1,5 +1,6 @@
-// Batch kernels: many independent bodies step in one launch (k_batch, several Newton iterations) or in
-// an element, a row and a solve launch (k_batch_solve, one Newton iteration).
+// Batch kernels: many independent bodies step in an element, a row and a solve launch per Newton
+// iteration (k_batch_elements, k_batch_rows, k_batch_solve) or, with more than kFlatNewton of them, in
+// one launch (k_batch).
 //
 // k_batch: a body is owned by a team: either a thread-block cluster of CL CTAs (large bodies) or a
 // single CTA (small bodies). The team runs the whole implicit step of its body without leaving
@@ -47,13 +48,14 @@ struct BatchParams
 	int steps;
 	float h;
 	int newton;
+	int k;                 // flat: the Newton iteration of these launches
 	int max_iter;
 	double tol2;
 	int refresh;
 	double newton_tol2;
 	unsigned long long* prof;  // optional: kPhases cycle counters per CTA
-	// flat: the single Newton iteration's elements and rows ran in the flat launches (their
-	// numbering below); the PCG launch then starts by summing delta0 = r.s itself
+	// flat: a Newton iteration's elements and rows ran in the flat launches (their numbering below);
+	// the PCG launch then starts by summing delta0 = r.s itself
 	int flat;
 	const unsigned* elem_off;
 	const unsigned* slice_off;
@@ -589,7 +591,7 @@ __global__ void __launch_bounds__(kPThreads, B3G_BATCH_MIN_BLOCKS) k_batch(Batch
 	}
 }
 
-// The PCG, the final update and the statistics of every body of a batch (single-Newton steps). A body's
+// The PCG, the final update and the statistics of every body of a batch, one Newton iteration. A body's
 // team is a cluster or an aligned half, quarter ... of one (its tier); each body is solved by
 // team_solve with its rows' vectors and as much of its matrix as fits in shared memory.
 // One CTA of 512 threads per SM (128 registers a thread, the SM's shared memory to itself). Measured
@@ -597,9 +599,9 @@ __global__ void __launch_bounds__(kPThreads, B3G_BATCH_MIN_BLOCKS) k_batch(Batch
 // 12.2 / 1.59 / 6.6, 768 x 1 14.4 / 1.68 / 7.4 (spills), 320 x 2 12.9 / 1.90 / 8.8, 256 x 2 14.5 /
 // 1.97 / 10.8; the launch before (256 x 4, every vector and matrix through L2 and HBM) 14.0 / 2.99 / 12.1.
 
-__device__ __noinline__ double final_vertex_dv_filtered(const DevBody& B, int i, float h, bool finish, float3 dv)
+__device__ __noinline__ double final_vertex_dv_filtered(const DevBody& B, int i, float h, bool first, bool finish, float3 dv)
 {
-	return final_vertex_dv<LdPlain, true>(B, i, h, true, finish, dv);
+	return final_vertex_dv<LdPlain, true>(B, i, h, first, finish, dv);
 }
 
 template <class TA, class TV, class Team>
@@ -613,16 +615,17 @@ __device__ __forceinline__ void batch_solve_body(Team& T, const DevBody& B, cons
 	A.max_iter = P.max_iter;
 	A.refresh = P.refresh;
 	A.h = P.h;
-	A.newton = 0;
-	A.newton_max = 1;
-	A.forces_left = 0;
-	A.warm = 0;
+	A.newton = P.k;
+	A.newton_max = P.newton;
+	A.forces_left = P.k + 1 < P.newton ? 1 : 0;
+	A.warm = P.k > 0 ? 1 : 0;
 	A.smem = room;
 	A.keep = 1024;
 	team_solve<TA, TV, false, 1>(
 	    T, B, A, smem,
 	    [&](int i, float3 dv, bool finish) {
-		    return B.filt ? final_vertex_dv_filtered(B, i, A.h, finish, dv) : final_vertex_dv<LdPlain, false>(B, i, A.h, true, finish, dv);
+		    return B.filt ? final_vertex_dv_filtered(B, i, A.h, A.newton == 0, finish, dv)
+		                  : final_vertex_dv<LdPlain, false>(B, i, A.h, A.newton == 0, finish, dv);
 	    },
 	    [&](int phase) { pc.tick(phase); });
 }
@@ -650,6 +653,7 @@ __global__ void __launch_bounds__(kSolveMaxThreads, 1) k_batch_solve(BatchParams
 				if (item >= end || !T.ok) break;
 				load_body(&sb, P.bodies + P.big[item]);
 				__syncthreads();
+				if (P.k > 0 && sb.sc->newton_done) continue;  // its Newton loop ended (every CTA agrees)
 				batch_solve_body<TA, TV>(T, sb, P, smem, room);
 			}
 		}
@@ -759,13 +763,13 @@ int solve_clusters(int cluster)
 	return m;
 }
 
-// One step: the whole-step kernel for several Newton iterations, else the assembly launch
+// One step: the whole-step kernel for many Newton iterations, else the assembly launch
 // (`ctas` CTAs) followed by the solve launch (as many CTAs as fit). part 1 / 2 issues only the
 // assembly / solve launch of a single-Newton step (timed separately), 0 both.
 template <int CL, class TA, class TV>
 cudaError_t launch_cl(const BatchParams& P, int ctas, int bf16, int part, cudaStream_t st)
 {
-	if (P.newton > 1) return launch_ph<CL, TA, TV, kPhaseWhole>(P, ctas, bf16, st);
+	if (P.newton > 1 && !P.flat) return launch_ph<CL, TA, TV, kPhaseWhole>(P, ctas, bf16, st);
 	if (part != 2 && !P.flat)
 	{
 		cudaError_t e = launch_ph<CL, TA, TV, kPhaseAssemble>(P, ctas, bf16, st);
@@ -809,8 +813,9 @@ constexpr int kRowsWarps = B3G_ROWS_THREADS / 32;
 #define B3G_ROWS_TETS_MIN_BLOCKS 3  // the tetrahedra-only row assembly fits more CTAs per SM
 #endif
 
-// FILT: some bodies have filtered contacts (their filt buffer set); each body takes its own form
-template <class TA, class TV, bool TETS, bool FILT = false>
+// FILT: some bodies have filtered contacts (their filt buffer set); each body takes its own form.
+// LATER: a Newton iteration after the first (a form of its own keeps the first one's registers).
+template <class TA, class TV, bool TETS, bool FILT, bool LATER>
 __global__ void __launch_bounds__(B3G_ROWS_THREADS, TETS ? B3G_ROWS_TETS_MIN_BLOCKS : B3G_ROWS_MIN_BLOCKS)
 k_batch_rows(BatchParams P)
 {
@@ -822,7 +827,8 @@ k_batch_rows(BatchParams P)
 	DevBody& B = s_body[threadIdx.x >> 5];
 	StepParams sp;
 	sp.h = P.h;
-	sp.first_newton = 1;
+	sp.first_newton = LATER ? 0 : 1;
+	const int init = LATER ? kInitNone : kInitTeam;
 	const unsigned nw = gridDim.x * kRowsWarps;
 	for (unsigned g = P.s_begin + blockIdx.x * kRowsWarps + (threadIdx.x >> 5); g < P.nslices; g += nw)
 	{
@@ -834,36 +840,43 @@ k_batch_rows(BatchParams P)
 			for (int w = lane; w < (int)(sizeof(DevBody) / 8); w += 32) dst[w] = __ldg(src + w);
 		}
 		__syncwarp();
+		if (LATER && B.sc->newton_done) continue;
 		const int sl = (int)(g - __ldg(P.slice_off + b));
-		if (FILT && B.filt) assemble_row_filtered<TA, TV, LdPlain>(B, sl, lane, sp, kInitTeam);
-		else assemble_row<TA, TV, LdPlain, false, TETS>(B, sl, lane, sp, kInitTeam);
+		if (FILT && B.filt) assemble_row_filtered<TA, TV, LdPlain>(B, sl, lane, sp, init);
+		else assemble_row<TA, TV, LdPlain, false, TETS>(B, sl, lane, sp, init);
 	}
 }
 
-template <class TA, class TV, bool TETS, bool FILT>
+template <class TA, class TV, bool TETS, bool FILT, bool LATER>
 cudaError_t launch_rows_t(const BatchParams& P, cudaStream_t st)
 {
 	static const std::pair<int, int> resident = [] {  // SMs, resident CTAs per SM
 		int dev = 0, sms = 0, per_sm = 0;
 		cudaGetDevice(&dev);
 		cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_rows<TA, TV, TETS, FILT>, B3G_ROWS_THREADS, 0);
+		cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_batch_rows<TA, TV, TETS, FILT, LATER>, B3G_ROWS_THREADS, 0);
 		return std::make_pair(std::max(1, sms), std::max(per_sm, 1));
 	}();
 	const int cap = resident.first * (P.rows_per_sm > 0 ? std::min(P.rows_per_sm, resident.second) : resident.second);
 	const unsigned need = (P.nslices - P.s_begin + kRowsWarps - 1) / kRowsWarps;
 	const int grid = (int)std::max(1u, std::min(need, (unsigned)cap));
-	k_batch_rows<TA, TV, TETS, FILT><<<grid, B3G_ROWS_THREADS, 0, st>>>(P);
+	k_batch_rows<TA, TV, TETS, FILT, LATER><<<grid, B3G_ROWS_THREADS, 0, st>>>(P);
 	return cudaGetLastError();
 }
 
 // the tetrahedra-only kernel when every body of the batch qualifies (P.tets_only), the kernel
 // with both row forms when some body has filtered contacts (P.filter)
+template <class TA, class TV, bool LATER>
+cudaError_t launch_rows_k(const BatchParams& P, cudaStream_t st)
+{
+	if (P.filter) return launch_rows_t<TA, TV, false, true, LATER>(P, st);
+	return P.tets_only ? launch_rows_t<TA, TV, true, false, LATER>(P, st) : launch_rows_t<TA, TV, false, false, LATER>(P, st);
+}
+
 template <class TA, class TV>
 cudaError_t launch_rows(const BatchParams& P, cudaStream_t st)
 {
-	if (P.filter) return launch_rows_t<TA, TV, false, true>(P, st);
-	return P.tets_only ? launch_rows_t<TA, TV, true, false>(P, st) : launch_rows_t<TA, TV, false, false>(P, st);
+	return P.k > 0 ? launch_rows_k<TA, TV, true>(P, st) : launch_rows_k<TA, TV, false>(P, st);
 }
 
 template <class TA, class TV>

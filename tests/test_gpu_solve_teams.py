@@ -135,3 +135,43 @@ def test_rows_longer_than_a_pass_match_oracle(ctx, spokes):
     assert st["solve_status"] == "converged"
     assert np.linalg.norm(v - vr) <= TOL * np.linalg.norm(vr)
     assert np.linalg.norm(x - xr) <= TOL * np.linalg.norm(xr - d.x)
+
+
+# up to 16 Newton iterations a batched step takes launches of their own, one whole-step launch above
+@pytest.mark.parametrize("newton", [2, 3, 16, 17])
+@pytest.mark.parametrize("precision", ["fp32", "fp64"])
+def test_batched_newton_iterations_match_oracle(ctx, precision, newton, monkeypatch):
+    monkeypatch.setenv("B3G_BATCH_SCHEDULE", "16,1,0,4,4")
+    mixes = [[block((2, 2, 2)), block((9, 8, 8)), block((16, 16, 17))]]  # the rows' short form
+    if newton <= 3:  # a cloth at rest is on springs' slack edge: FP32 and FP64 oracles part with every iteration
+        mixes.append([block((9, 8, 8)), meshes.cloth_grid(16)])
+    for descs in mixes:
+        bodies = [b3g.Body(ctx, d) for d in descs]
+        cfg = b3g.solver_config(force_iterations=newton, max_pcg_iterations=500, pcg_tolerance=1e-5,
+                                precision=PRECISIONS[precision])
+        b3g.step_batch(ctx, bodies, DT, 1, cfg)
+        for d, b in zip(descs, bodies):
+            x, v = b.state()
+            xr, vr, _, _ = oracle.simulate(d, 1, dt=DT, newton_iters=newton, max_sub=500, sub_tol=1e-5, bits=64)
+            assert np.linalg.norm(v - vr) <= TOL * np.linalg.norm(vr)
+            assert np.linalg.norm(x - xr) <= TOL * np.linalg.norm(xr - d.x)
+            b.close()
+
+
+def test_batched_newton_loops_end_at_their_own_iteration(ctx, monkeypatch):
+    """Bodies whose loops end early, by tolerance, beside one that goes on; 16 and 17 as above."""
+    monkeypatch.setenv("B3G_BATCH_SCHEDULE", "8,1,0,4")
+    descs = [block((4, 4, 3)), meshes.tet_grid(6, 6, 6, seed=2, E=2e3, nu=0.3, pin="y0"), block((16, 16, 17))]
+    runs = []
+    for newton in (16, 17):
+        bodies = [b3g.Body(ctx, d) for d in descs]
+        cfg = b3g.solver_config(force_iterations=newton, max_pcg_iterations=500, pcg_tolerance=1e-5, newton_tolerance=1e-2)
+        for _ in range(3):
+            stats = b3g.step_batch(ctx, bodies, DT, 1, cfg)
+        runs.append([(b.state(), s) for b, s in zip(bodies, stats)])
+        for b in bodies:
+            b.close()
+    for ((xa, va), sa), ((xb, vb), sb) in zip(*runs):
+        assert sa["newton_iterations"] == sb["newton_iterations"] < 16
+        assert sa["total_steps"] == sb["total_steps"] == 3
+        assert np.linalg.norm(va - vb) <= TOL * np.linalg.norm(vb)
