@@ -37,8 +37,9 @@ DT = 1.0 / 60.0
 PCG_TOL = 1e-5
 PCG_MAX = 200
 # DRAM traffic / algorithmic bytes of the batch PCG launch, from the ncu capture of the
-# 128-body case (profiles/k_batch_batch512.md)
-PCG_TRAFFIC_RATIO = 1.072
+# 128-body case (profiles/k_batch_solve_batch128.md): most of a body's matrix and vectors stay in
+# shared memory and L2 between its iterations
+PCG_TRAFFIC_RATIO = 0.25
 # steps of the CPU-baseline run and of the parity check, from the bodies' initial state
 PARITY_STEPS = 3
 
@@ -57,7 +58,7 @@ def parse():
     p.add_argument("--precision", default="fp32", choices=["fp32", "fp64", "bf16"])
     p.add_argument("--no-extras", action="store_true", help="skip e2e, plain path and CPU baseline")
     p.add_argument("--path", default="plain", choices=["plain", "batch"],
-                   help="single-body workloads: the per-op kernels (plain) or the persistent kernel with one body")
+                   help="single-body workloads: the single-body step (plain) or a batch of one body")
     # serving (--workload serve): Poisson arrivals over a pool of bodies
     p.add_argument("--serve-rate", type=float, default=2000.0, help="requests per second")
     p.add_argument("--serve-seconds", type=float, default=60.0, help="length of the arrival stream")
@@ -176,7 +177,7 @@ def workload(args, rank, world=1):
 
 
 def bf16_inner():
-    """Inner BF16 iterations per outer iteration of the per-op BF16 mode (the library's default)."""
+    """Inner BF16 iterations per outer iteration of the single-body BF16 mode (the library's default)."""
     return int(os.environ.get("B3G_BF16_INNER", "20"))
 
 
@@ -346,7 +347,7 @@ def ours(args, world, rank, local, pg):
 
     def step_once():
         if per_op:
-            # one body: the per-op kernels of the single-body path (grid-wide SpMV / reductions)
+            # one body: the single-body step (one solve launch over the GPU)
             bodies[0].step(dt, scfg, stats=False)
         else:
             b3g.step_batch(ctx, bodies, dt, 1, scfg, stats=False)
@@ -392,13 +393,13 @@ def ours(args, world, rank, local, pg):
                                         "ms_per_step": total_ms / args.steps}, world)
 
     # rooflines. Whole step: every kernel of the timed region. Persistent path: the PCG launch
-    # (the dominant kernel, 78 % of a step) and the assembly launch, each timed live with CUDA
+    # (the dominant kernel, 77 % of a step) and the assembly launch, each timed live with CUDA
     # events around its own launch on the context's stream (b3g_batch_set_launch_timing) over
     # extra steps run after the timed region.
     bs, vsz = {"fp32": (36, 4), "fp64": (72, 8), "bf16": (18, 4)}[args.precision]
     alg_asm = sum(args.steps * assembly_bytes(i) for i in infos)
     if per_op and args.precision == "bf16":
-        # the per-op BF16 mode counts outer iterations of its flexible CG: each is BF16_INNER inner
+        # the single-body BF16 mode counts outer iterations of its flexible CG: each is BF16_INNER inner
         # iterations with the bf16 blocks, one FP32 product with its update, and z.q_prev
         m = bf16_inner()
         alg_pcg = sum(it * (m * iteration_bytes(i, 4, 18) + iteration_bytes(i, 4, 36) + 32 * i["vertices"])
@@ -427,11 +428,11 @@ def ours(args, world, rank, local, pg):
         asm_b = sum(assembly_bytes(i) for i in infos)
         pcg_ms, asm_ms = lt["pcg_ms"] / lt["steps"], lt["assembly_ms"] / lt["steps"]
         ach = pcg_b / (pcg_ms / 1e3) / 1e9
-        roof.update({"achieved": ach, "frac": ach / peak, "kernel": "k_batch PCG launch (PCG + final update)",
+        roof.update({"achieved": ach, "frac": ach / peak, "kernel": "k_batch_solve launch (PCG + final update)",
                      "algorithmic_bytes_per_launch": pcg_b, "launch_ms": pcg_ms, "launches_timed": lt["steps"]})
-        # DRAM traffic of the PCG launch: ncu on the 128-body case measured 39.55 GB for
-        # 36.90 GB of algorithmic bytes with 256-thread CTAs (PCG_TRAFFIC_RATIO; 1.093 with
-        # 512-thread CTAs); traffic grows with the work, so the ratio scales it to this launch
+        # DRAM traffic of the PCG launch: ncu on the 128-body case (PCG_TRAFFIC_RATIO); traffic
+        # grows with the work, so the ratio scales it to this launch. The algorithmic bytes count
+        # every iteration's operands, so `achieved` can pass the HBM peak
         if args.precision == "fp32":
             roof["traffic"] = PCG_TRAFFIC_RATIO * pcg_b
         roof["assembly_launch"] = {"achieved": asm_b / (asm_ms / 1e3) / 1e9, "frac": asm_b / (asm_ms / 1e3) / 1e9 / peak,
@@ -490,7 +491,7 @@ def ours(args, world, rank, local, pg):
                          "h2d_bytes_per_step": 12 * nverts, "d2h_bytes_per_step": 24 * nverts,
                          "upload": "upload stream, overlapping the step before",
                          "read_back": "second stream, overlapping the next step", "host_arrays_match": e2e_ok}
-        # plain one-body-at-a-time GPU path (per-op kernels) on a size-stratified sample
+        # plain one-body-at-a-time GPU path (b3g_body_step) on a size-stratified sample
         sample = sorted(range(len(bodies)), key=lambda k: -infos[k]["vertices"])[::16] if len(bodies) > 16 else list(
             range(len(bodies)))
         for k in sample[:2]:
@@ -543,39 +544,24 @@ def ours(args, world, rank, local, pg):
             "residual_ratio_max": max(float(s["residual_ratio"]) for s in last),
             "solver_outcome": "last timed step of every body: solves not converged, largest sqrt(delta/delta0)"}
 
-    # persistent path: two launches per step (elements + assembly, then PCG + final update), plus
-    # a 16-byte memset of the work counters that is not a kernel. Per-op path per step: begin,
-    # one element kernel per element kind, assembly, then per PCG iteration the fused
-    # direction/SpMV/dot kernel and the update kernel (launched in chunks of 8 iterations between
-    # convergence checks), the true-residual refresh when due, and the final update; in bf16 mode
-    # the outer iterations of the flexible CG instead (counted below).
+    # Per Newton iteration. Single body: one element kernel per element kind, the row assembly and
+    # the solve (PCG, final update and statistics, in every precision). Batch: the flat element and
+    # row launches and the solve, plus memsets of the work counters that are not kernels.
+    newton = max(1, int(scfg.force_iterations))
     if per_op:
         i0 = infos[0]
-        per_step = 1 + (1 if i0["tets"] else 0) + (1 if i0["tris"] else 0) + (1 if i0["springs"] else 0) + 1 + 1
-        launches = per_step * args.steps
-        refresh = scfg.refresh_period
-        for it in iters:  # total over the timed steps; every step of a run takes about the same
-            per = int(it) / max(args.steps, 1)
-            if args.precision == "bf16":
-                # per outer iteration: inner begin (2), 2 per inner iteration, z.q_prev (not on the
-                # first), direction / product, update, refresh check
-                outer = int(round(per))
-                launches += args.steps * (outer * (2 + 2 * bf16_inner() + 4) - 1)
-                continue
-            launched = min(-(-int(round(per)) // 8) * 8, mx)
-            resid = sum(1 for j in range(launched) if refresh > 0 and j % refresh == 0)
-            launches += args.steps * (2 * launched + resid)
-        roof["kernel"] = "per-op step: k_dir_spmv_dot (70 % of the kernel time) + k_update + refresh"
+        kinds = (1 if i0["tets"] else 0) + (1 if i0["tris"] else 0) + (1 if i0["springs"] else 0)
+        launches = (kinds + 2) * newton * args.steps
+        roof["kernel"] = "single-body step: k_solve (PCG + final update, one launch) after elements and rows"
     else:
-        # single Newton iteration: the flat element launch, the flat row launch and the PCG
-        # launch; several: one whole-step launch
-        if scfg.force_iterations > 1:
-            launches = args.steps
-        else:
-            has_elements = any(i["tets"] or i["tris"] or i["springs"] for i in infos)
-            # the split assembly launches elements and rows twice each (two body groups)
-            per_step = (3 if has_elements else 2) + (2 if b3g.batch_assembly_split(ctx)["elem_mid"] else 0)
-            launches = per_step * args.steps
+        has_elements = any(i["tets"] or i["tris"] or i["springs"] for i in infos)
+        # the split assembly launches elements and rows twice each (two body groups)
+        per_step = (3 if has_elements else 2) + (2 if b3g.batch_assembly_split(ctx)["elem_mid"] else 0)
+        # the chosen schedule's second solve launch, on the SMs that the wide clusters leave free
+        best = min(sched["candidates_ms"], key=lambda c: c[3]) if sched["candidates_ms"] else None
+        if best and best[1] >= 1000:
+            per_step += 1
+        launches = per_step * newton * args.steps
     line = {"metric": METRIC, "value": value, "unit": "vertex-steps/s", "n_gpus": world, "steps": args.steps,
             "warmup": max(args.warmup, 3), "ms_per_step": t_max * 1e3 / args.steps, "higher_is_better": True,
             "scaling": "strong" if args.split else "weak", "vs_baseline": None,
@@ -590,7 +576,19 @@ def ours(args, world, rank, local, pg):
     if sched:
         line["schedule"] = {k: sched[k] for k in ("cluster", "threshold", "cluster_bodies", "ctas", "autotuned", "order")}
         line["schedule"]["candidates_timed"] = len(sched["candidates_ms"])
-        # the chosen schedule per size bucket: which team steps the bucket's bodies
+        # the chosen schedule per size bucket: the teams of the bucket's bodies (parts of a cluster)
+        best = min(sched["candidates_ms"], key=lambda c: c[3]) if sched["candidates_ms"] else None
+        per, helper = (best[1] % 1000, best[1] // 1000) if best else (0, 0)
+        line["schedule"].update(slices_per_cta=per, second_launch_cluster=helper)
+
+        def team(n):
+            if per <= 0:
+                return sched["cluster"] if 0 <= sched["threshold"] <= n else 1
+            w = 1
+            while w < sched["cluster"] and -(-n // 32) > per * w:
+                w *= 2
+            return w
+
         edges = [0, 1024, 2048, 4096, 8192, 16384, 32768, 1 << 31]
         iters_all = [b.stats()["pcg_iterations"] for b in bodies] if not per_op else []
         buckets = []
@@ -598,9 +596,9 @@ def ours(args, world, rank, local, pg):
             ks = [k for k, i in enumerate(infos) if lo <= i["vertices"] < hi]
             if not ks:
                 continue
-            clustered = sched["threshold"] >= 0 and sched["cluster"] > 1 and lo >= sched["threshold"]
+            w = sorted({team(infos[k]["vertices"]) for k in ks})
             buckets.append({"vertices": f"[{lo},{hi})" if hi < (1 << 31) else f"[{lo},)", "bodies": len(ks),
-                            "team": f"cluster of {sched['cluster']} CTAs" if clustered else "one CTA",
+                            "team": f"{w[0]} CTAs" if len(w) == 1 else f"{w[0]} to {w[-1]} CTAs",
                             "mean_pcg_iterations": float(np.mean([iters_all[k] for k in ks])) if iters_all else None})
         line["schedule"]["buckets"] = buckets
     line.update(extras)
