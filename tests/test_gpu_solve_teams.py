@@ -82,7 +82,8 @@ def test_batched_teams_match_oracle(ctx, precision, schedule, monkeypatch):
     if precision != "bf16":  # a batched BF16 solve is one with the rounded blocks
         for s, (x, v), st in zip(sizes, states, stats):
             check(s, x, v, st, False)
-    # team sums are exact and a row's order is fixed: a body's result does not depend on its team
+    # a row's order is fixed and sums are integers with at least FP64's bits: on these bodies the result
+    # does not depend on the team
     alone, alone_stats = run("4,1,0,100000")
     for s, (x, v), st, (xa, va), sa in zip(sizes, states, stats, alone, alone_stats):
         assert st["pcg_iterations"] == sa["pcg_iterations"], s
