@@ -36,6 +36,10 @@ const Device& device()
 // kL2Keep bytes of it all stay there. Beyond, a cyclic sweep under LRU would find nothing left, so
 // kL2Keep bytes are kept (evict last) and the rest streams past them (evict first). 64^3 block,
 // 165 MB: 0 / 25 / 37 / 50 / 62 / 75 / 100 % kept 12.8 / 12.4 / 12.0 / 11.7 / 12.7 / 13.6 / 14.1 ms.
+// Row vectors that shared memory does not hold are read and written every iteration, so their bytes come
+// off kL2Keep first: matrix kept beside them pushed them out. BF16 62^3 3.51 -> 3.15 ms a step, 75x74x73
+// 6.08 -> 5.45, 97x89x83 10.9 -> 9.3 (10.2 kernel by kernel); FP32 97x89x83 11.1 -> 10.5 ms per 100 iterations,
+// 62^3, whose vectors fit, the same.
 constexpr size_t kL2Keep = (size_t)80 << 20;
 
 struct Geometry
@@ -58,7 +62,9 @@ Geometry geometry(const DevBody& B, size_t vec_bytes, size_t slot_bytes, int lea
 	const size_t total = (size_t)B.nslots * slot_bytes;
 	const size_t held = (size_t)g.ctas * (size_t)std::max(0, g.smem - (int)std::min<size_t>(slices * vec_bytes, g.smem));
 	const size_t stream = total > held ? total - held : 0;
-	g.keep = stream <= kL2Keep ? 1024 : (int)(1024 * kL2Keep / stream);
+	const size_t outside = (size_t)g.ctas * (slices * vec_bytes - std::min<size_t>(slices * vec_bytes, g.smem));
+	const size_t keep = kL2Keep > outside ? kL2Keep - outside : 0;
+	g.keep = stream <= keep ? 1024 : (int)(1024 * keep / stream);
 	return g;
 }
 
