@@ -116,6 +116,7 @@ SIGNATURES = {
     "b3g_context_destroy": (C.c_int, [C.c_void_p]),
     "b3g_context_stream": (C.c_int, [C.c_void_p, C.POINTER(C.c_void_p)]),
     "b3g_context_synchronize": (C.c_int, [C.c_void_p]),
+    "b3g_context_set_poll_limit": (C.c_int, [C.c_void_p, C.c_uint32]),
     "b3g_body_create": (C.c_int, [C.c_void_p, C.POINTER(BodyDescC), C.POINTER(C.c_void_p)]),
     "b3g_body_destroy": (C.c_int, [C.c_void_p]),
     "b3g_body_info": (C.c_int, [C.c_void_p, C.POINTER(C.c_uint64)]),
@@ -231,6 +232,10 @@ class Context:
 
     def synchronize(self):
         _check(load_library().b3g_context_synchronize(self.handle), "b3g_context_synchronize")
+
+    def set_poll_limit(self, polls: int):
+        """b3g_context_set_poll_limit: polls after which a device wait gives up (0: the default)."""
+        _check(load_library().b3g_context_set_poll_limit(self.handle, polls), "b3g_context_set_poll_limit")
 
     def close(self):
         if self.handle:

@@ -331,7 +331,7 @@ void stats_from(const Scalars& sc, b3g_step_stats* st)
 	st->newton_iterations = (uint32_t)sc.newton_iter;
 	st->pcg_iterations = (uint32_t)sc.max_it;
 	st->min_pcg_iterations = sc.min_it == 0x7fffffff ? 0u : (uint32_t)sc.min_it;
-	st->solve_status = sc.fault ? B3G_SOLVE_DEVICE_TIMEOUT : sc.status;
+	st->solve_status = timed_out(sc) ? B3G_SOLVE_DEVICE_TIMEOUT : sc.status;
 	st->residual_ratio = sc.delta0 > 0.0 ? std::sqrt(std::max(0.0, sc.delta / sc.delta0)) : 0.0;
 	st->newton_error = sc.newton_err;
 	st->total_pcg_iterations = sc.total_iters;
@@ -446,6 +446,13 @@ int b3g_context_stream(b3g_context* c, void** stream)
 {
 	if (!c || !stream) return fail(B3G_ERROR_INVALID_ARGUMENT, "null argument");
 	*stream = (void*)c->stream;
+	return B3G_OK;
+}
+
+int b3g_context_set_poll_limit(b3g_context* c, uint32_t polls)
+{
+	if (!c) return fail(B3G_ERROR_INVALID_ARGUMENT, "null context");
+	c->polls = (int)std::min<uint32_t>(polls, 0x7fffffffu);
 	return B3G_OK;
 }
 
@@ -893,6 +900,7 @@ int b3g_body_step(b3g_body* b, float dt, const b3g_solver_config* cfg_in, b3g_st
 		A.forces_left = k + 1 < newton ? 1 : 0;
 		A.warm = k > 0 ? 1 : 0;
 		A.smem = 0;
+		A.polls = b->ctx->polls;
 		if (prec == kPBF)
 		{
 			const PrecBuffers& pb = b->prec[kPBF];

@@ -6,6 +6,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <mutex>
 #include <vector>
 
@@ -19,6 +20,7 @@ struct b3g_context
 {
 	int device = 0;
 	int sm_count = 0;
+	std::atomic<int> polls{0};           // of a device wait before it gives up, 0: the default
 	cudaStream_t stream = nullptr;
 	b3g::Scalars* h_scalars = nullptr;   // pinned, 1024 entries
 	b3g_ray_hit* h_hits = nullptr;       // pinned, kRayPick entries; one ray cast at a time (ray_mutex)

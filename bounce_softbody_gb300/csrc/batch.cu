@@ -50,7 +50,7 @@ struct BatchCache
 	// graph of (memset queue, batch launch) for one step with the current parameters
 	cudaGraphExec_t graph = nullptr;
 	float g_h = 0.0f;
-	int g_newton = 0, g_max_iter = 0, g_refresh = 0;
+	int g_newton = 0, g_max_iter = 0, g_refresh = 0, g_polls = 0;
 	double g_tol2 = 0.0, g_ntol2 = 0.0;
 	std::vector<std::pair<int, double>> tune_log;  // (cluster * 1e6 + threshold, ms)
 	unsigned long long* d_prof = nullptr;          // phase cycle counters when B3G_PHASE_PROFILE=1
@@ -85,7 +85,7 @@ int schedule_ctas(int prec, int cluster, int sms)
 	return m * cluster;
 }
 
-BatchArgs make_args(BatchCache* c, float h, int steps, const b3g_solver_config& cfg)
+BatchArgs make_args(const b3g_context* ctx, BatchCache* c, float h, int steps, const b3g_solver_config& cfg)
 {
 	BatchArgs A;
 	A.bodies = c->d_bodies;
@@ -96,6 +96,7 @@ BatchArgs make_args(BatchCache* c, float h, int steps, const b3g_solver_config& 
 	A.queue = c->d_queue;
 	std::copy(c->tier_end, c->tier_end + kTiers, A.tier_end);
 	A.helper = c->helper;
+	A.polls = ctx->polls;
 	A.steps = steps;
 	A.h = h;
 	A.newton = (int)std::max<uint32_t>(1u, cfg.force_iterations);
@@ -291,7 +292,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 	{
 		const Cand cd = cands[n];
 		set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per, cd.helper);
-		BatchArgs A = make_args(c, h, 1, cfg);
+		BatchArgs A = make_args(ctx, c, h, 1, cfg);
 		if (use_side_stream(ctx, &A) != B3G_OK) e = cudaErrorUnknown;
 		if (e == cudaSuccess) e = op_batch(A, st);  // warm-up
 		if (e == cudaSuccess && c->iters.empty())
@@ -305,7 +306,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 				break;
 			}
 			set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per, cd.helper);
-			A = make_args(c, h, 1, cfg);
+			A = make_args(ctx, c, h, 1, cfg);
 			use_side_stream(ctx, &A);
 		}
 		for (const Snapshot& s : L) cudaMemcpyAsync((void*)s.src, s.dst, s.bytes, cudaMemcpyDeviceToDevice, st);
@@ -528,7 +529,7 @@ extern "C" int b3g_step_batch(b3g_context* ctx, b3g_body* const* bodies, uint32_
 			if (rc != B3G_OK) return rc;
 		}
 	}
-	BatchArgs A = make_args(c, dt, 1, cfg);
+	BatchArgs A = make_args(ctx, c, dt, 1, cfg);
 	rc = use_side_stream(ctx, &A);
 	if (rc != B3G_OK) return rc;
 	if (ctx->launch_timing && A.newton == 1)
@@ -562,7 +563,7 @@ extern "C" int b3g_step_batch(b3g_context* ctx, b3g_body* const* bodies, uint32_
 		return stats ? read_batch_stats(ctx, bodies, count, stats) : B3G_OK;
 	}
 	const bool graph_ok = c->graph && c->g_h == dt && c->g_newton == A.newton && c->g_max_iter == A.max_iter &&
-	                      c->g_tol2 == A.tol2 && c->g_refresh == A.refresh && c->g_ntol2 == A.newton_tol2;
+	                      c->g_tol2 == A.tol2 && c->g_refresh == A.refresh && c->g_ntol2 == A.newton_tol2 && c->g_polls == A.polls;
 	cudaError_t e = cudaSuccess;
 	if (!graph_ok)
 	{
@@ -588,6 +589,7 @@ extern "C" int b3g_step_batch(b3g_context* ctx, b3g_body* const* bodies, uint32_
 		c->g_tol2 = A.tol2;
 		c->g_refresh = A.refresh;
 		c->g_ntol2 = A.newton_tol2;
+		c->g_polls = A.polls;
 	}
 	for (uint32_t s = 0; s < steps && e == cudaSuccess; ++s) e = cudaGraphLaunch(c->graph, st);
 	if (e != cudaSuccess) return cuda_fail(e, "batch launch");
@@ -1007,6 +1009,7 @@ extern "C" int b3g_step_batch_noalloc(b3g_context* ctx, b3g_body* const* bodies,
 	A.cluster = cluster;
 	A.ctas = m * cluster;
 	A.prof = nullptr;
+	A.polls = ctx->polls;
 	for (uint32_t s = 0; s < steps && e == cudaSuccess; ++s) e = op_batch(A, st);
 	if (e != cudaSuccess) return cuda_fail(e, "b3g_step_batch_noalloc launch");
 	if (stats)

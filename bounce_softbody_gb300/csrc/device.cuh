@@ -1189,6 +1189,20 @@ __device__ __forceinline__ void contact_filter_vertex(const DevBody& B, int i, f
 
 __device__ __forceinline__ bool filt_on(float4 f) { return f.x != 0.0f || f.y != 0.0f || f.z != 0.0f; }
 
+// A body whose rows are being assembled: its solve is outstanding. A step's first one starts without
+// a fault; a later one finds the solve before it finished, or the step is lost.
+__device__ __forceinline__ void solve_pending(const DevBody& B, bool first_newton)
+{
+	if (first_newton)
+	{
+		if (timed_out(*B.sc)) B.sc->lost_steps += 1ull;
+		B.sc->fault = 0;
+	}
+	else if (B.sc->pending)
+		B.sc->fault = B.sc->newton_done = 1;
+	B.sc->pending = 1;
+}
+
 // The end of row i's assembly once its right-hand side bi and diagonal block are final: pb,
 // the Jacobi preconditioner and, for init_pcg = kInitAll, r = pb, s = d = M^-1 r and the zero
 // initial guess; returns r.s (0 otherwise). kInitTeam: only s = M^-1 pb.

@@ -57,7 +57,7 @@ struct Scalars
 	double newton_tol2;
 	int iter;          // PCG iteration of the current solve
 	int max_iter;
-	int done;          // current PCG solve finished
+	int pending;       // rows assembled, solve not finished: set by the assembly, cleared by the solve
 	int status;        // b3g_solve_status
 	int newton_iter;
 	int newton_done;
@@ -66,7 +66,11 @@ struct Scalars
 	int fault;         // a bounded device wait expired (the step's results are not valid)
 	unsigned long long total_iters;  // PCG iterations of every step since creation
 	unsigned long long total_steps;
+	unsigned long long lost_steps;   // steps before the last one whose waits ran out
 };
+// Whether the last step's device waits ran out (its results are not valid): a member of the body's
+// team gave up, or no team took the body.
+B3G_HD bool timed_out(const Scalars& s) { return s.fault || s.pending; }
 
 // One static world shape (b3WorldFixture + b3Shape) on the device. Geometry is in world space
 // except where the shape keeps a frame (box, sdf: rotation q, translation t; mesh triangles are

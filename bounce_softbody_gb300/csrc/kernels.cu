@@ -212,6 +212,7 @@ __global__ void __launch_bounds__(kThreads) k_assemble(DevBody B, StepParams P, 
 	// the grid team's reduction memory starts at zero
 	for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < (int)(sizeof(TeamMemory) / 4); k += gridDim.x * blockDim.x)
 		((unsigned*)B.team)[k] = 0u;
+	if (blockIdx.x == 0 && threadIdx.x == 0) solve_pending(B, P.first_newton);
 	const int lane = threadIdx.x & 31;
 	for (int s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; s < B.nslices; s += (gridDim.x * blockDim.x) >> 5)
 		assemble_row<TA, TV, LdPlain, FILTER>(B, s, lane, P, init);
@@ -230,6 +231,7 @@ __global__ void __launch_bounds__(32 * kSlotWarps) k_assemble_slots(DevBody B, S
 	if (newton_over(B, P)) return;
 	for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < (int)(sizeof(TeamMemory) / 4); k += gridDim.x * blockDim.x)
 		((unsigned*)B.team)[k] = 0u;
+	if (blockIdx.x == 0 && threadIdx.x == 0) solve_pending(B, P.first_newton);
 	__shared__ float sb[3][32], sk[9][32], sd[32];
 	const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, slots = (int)(blockDim.x >> 5) - 1;
 	const int i = blockIdx.x * kSlice + lane;

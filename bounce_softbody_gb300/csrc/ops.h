@@ -51,10 +51,10 @@ struct SolveArgs
 	int warm;          // start from the solution at hand (r = b - A x) instead of zero
 	int smem;          // bytes of shared memory of a CTA (set by op_solve)
 	int keep;          // 1/1024 of a CTA's slices whose matrix stays in L2 (set by op_solve)
+	int polls;         // of a team's wait before it gives up, 0: the default
 };
+// The team's reduction memory starts cleared, and the scalars without a fault (op_assemble does both).
 cudaError_t op_solve(const DevBody& B, const SolveArgs& P, int prec, cudaStream_t st);
-// the team's reduction slots cleared before a solve (op_assemble does it for a body step)
-cudaError_t op_solve_clear(const DevBody& B, cudaStream_t st);
 // The BF16 mode's solve (flexible CG on the FP32 blocks around `inner` PCG iterations with the BF16
 // blocks) and what follows it. W: the inner solve's vectors, 4-wide, where shared memory has no
 // room for them.
@@ -152,6 +152,7 @@ struct BatchArgs
 	// A second solve launch on `side` (0: none): clusters of `helper` CTAs on the SMs that the first one's
 	// clusters leave free, taking the bodies of teams at most that wide from the same counters.
 	int helper = 0;
+	int polls = 0;           // of a solve team's wait before it gives up, 0: the default
 	unsigned elem_mid = 0, slice_mid = 0;
 	int split_elem_per_sm = 0, split_rows_per_sm = 0;
 };

@@ -190,6 +190,7 @@ cudaError_t op_batch(const BatchArgs& A, cudaStream_t st)
 	P.nsmall = A.nsmall;
 	P.queue = A.queue;
 	P.solve_ctas = 0;
+	P.polls = A.polls;
 	for (int t = 0; t < kTiers; ++t) P.tier_end[t] = A.tier_end[t];
 	P.steps = A.steps;
 	P.h = A.h;

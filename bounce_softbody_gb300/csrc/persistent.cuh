@@ -44,6 +44,7 @@ struct BatchParams
 	int nsmall;
 	unsigned* queue;
 	int solve_ctas;        // CTAs of the solve launch (0: as many clusters as fit)
+	int polls;             // of a solve team's wait before it gives up, 0: the default
 	int tier_end[kTiers];  // of the order `big` (which runs on into `small`): the solve launch's teams
 	int steps;
 	float h;
@@ -447,7 +448,7 @@ __device__ void team_finish(Team<CL>& T, const DevBody& B, const BatchParams& P,
 		sc->max_it = max_it;
 		sc->newton_iter = newton_iters;
 		sc->newton_err = err;
-		sc->done = 1;
+		sc->pending = 0;
 		if (sc->fault) sc->status = B3G_SOLVE_DEVICE_TIMEOUT;
 		sc->total_iters += iters_all;
 		sc->total_steps += 1ull;
@@ -522,7 +523,7 @@ __device__ void team_step_assemble(Team<CL>& T, const DevBody& B, const BatchPar
 	typedef typename std::conditional<CL == 1, LdPlain, LdCG>::type LD;
 	PhaseClock pc;
 	pc.start(P.prof);
-	if (T.tid() == 0) B.sc->fault = 0;
+	if (T.tid() == 0) solve_pending(B, true);
 	const double delta0 = team_assemble<CL, TA, TV, LD>(T, B, P, bf16, 0, pc);
 	if (T.tid() == 0) B.sc->delta0 = delta0;
 }
@@ -621,6 +622,7 @@ __device__ __forceinline__ void batch_solve_body(Team& T, const DevBody& B, cons
 	A.warm = P.k > 0 ? 1 : 0;
 	A.smem = room;
 	A.keep = 1024;
+	A.polls = P.polls;
 	team_solve<TA, TV, false, 1>(
 	    T, B, A, smem,
 	    [&](int i, float3 dv, bool finish) {
@@ -637,11 +639,13 @@ __global__ void __launch_bounds__(kSolveMaxThreads, 1) k_batch_solve(BatchParams
 	__shared__ SolveSh sh;
 	__shared__ __align__(16) DevBody sb;
 	cg::cluster_group cl = cg::this_cluster();
-	ClusterTeam<TV> T(&sh);
+	ClusterTeam<TV> T(&sh, P.polls);
 	cl.sync();
-	// widest teams first; a cluster whose wider teams find no more bodies splits into narrower ones
+	// widest teams first; a cluster whose wider teams find no more bodies splits into narrower ones.
+	// A CTA one of whose waits ran out takes part in no further sum: its teammates run out at their next
+	// one, so no partial of one sum is taken for another's, and the bodies they leave are reported.
 	int begin = 0;
-	for (int t = 0; t < kTiers; ++t)
+	for (int t = 0; t < kTiers && T.ok; ++t)
 	{
 		const int end = P.tier_end[t], width = kMaxTeamCtas >> t;
 		if (end > begin && width <= (int)cl.num_blocks())
@@ -649,12 +653,21 @@ __global__ void __launch_bounds__(kSolveMaxThreads, 1) k_batch_solve(BatchParams
 			T.form(width);
 			for (;;)
 			{
-				const int item = begin + T.agree([&] { return (int)min(atomicAdd(P.queue + 2 + t, 1u), 1u << 29); });
-				if (item >= end || !T.ok) break;
+				// the next body whose Newton loop goes on (the team's first thread decides for all)
+				int taken = end;
+				const int item = begin + T.agree([&] {
+					do
+					{
+						taken = begin + (int)min(atomicAdd(P.queue + 2 + t, 1u), 1u << 28);
+					} while (taken < end && P.k > 0 && P.bodies[P.big[taken]].sc->newton_done);
+					return taken - begin;
+				});
+				if (!T.ok && taken < end) team_fault(P.bodies[P.big[taken]]);
+				if (!T.ok || item < begin || item >= end) break;
 				load_body(&sb, P.bodies + P.big[item]);
 				__syncthreads();
-				if (P.k > 0 && sb.sc->newton_done) continue;  // its Newton loop ended (every CTA agrees)
 				batch_solve_body<TA, TV>(T, sb, P, smem, room);
+				if (!T.ok) break;
 			}
 		}
 		begin = end;
@@ -842,6 +855,7 @@ k_batch_rows(BatchParams P)
 		__syncwarp();
 		if (LATER && B.sc->newton_done) continue;
 		const int sl = (int)(g - __ldg(P.slice_off + b));
+		if (sl == 0 && lane == 0) solve_pending(B, !LATER);
 		if (FILT && B.filt) assemble_row_filtered<TA, TV, LdPlain>(B, sl, lane, sp, init);
 		else assemble_row<TA, TV, LdPlain, false, TETS>(B, sl, lane, sp, init);
 	}

@@ -232,6 +232,7 @@ struct Request
 	int32_t status = 0;
 	uint64_t pcg_iterations = 0;
 	uint64_t iters0 = 0;         // the body's PCG iteration total when the request started
+	uint64_t lost0 = 0;          // and its steps whose waits ran out
 };
 
 struct SBody
@@ -427,6 +428,7 @@ void admit(b3g_server* s)
 			return;
 		}
 		r.iters0 = sc.total_iters;
+		r.lost0 = sc.lost_steps + timed_out(sc);
 		B.active = true;
 		r.t_start = now_s();
 		s->admitted++;
@@ -516,6 +518,7 @@ int step_active(b3g_server* s, int count, int nbig)
 	A.nelem = s->h_flat_off[count];
 	A.nslices = s->h_flat_off[2 * count + 1];
 	A.nbodies = count;
+	A.polls = s->ctx->polls;
 	cudaEventRecord(s->ev0, st);
 	e = op_batch(A, st);
 	cudaEventRecord(s->ev1, st);
@@ -582,7 +585,7 @@ void worker_loop(b3g_server* s)
 					return;
 				}
 				r.pcg_iterations = sc.total_iters - r.iters0;
-				r.status = sc.fault ? B3G_REQUEST_DEVICE_TIMEOUT : B3G_REQUEST_DONE;
+				r.status = sc.lost_steps + timed_out(sc) > r.lost0 ? B3G_REQUEST_DEVICE_TIMEOUT : B3G_REQUEST_DONE;
 				r.t_finish = t;
 				s->done.push_back(r.id);
 				s->completed++;

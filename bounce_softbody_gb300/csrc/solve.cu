@@ -162,9 +162,4 @@ cudaError_t op_solve_fcg(const DevBody& B, const FcgVecs& W, const SolveArgs& P,
 	return B.filt ? launch_fcg<true>(B, W, P, inner, st) : launch_fcg<false>(B, W, P, inner, st);
 }
 
-cudaError_t op_solve_clear(const DevBody& B, cudaStream_t st)
-{
-	return cudaMemsetAsync(B.team, 0, sizeof(TeamMemory), st);
-}
-
 } // namespace b3g

@@ -22,7 +22,9 @@
 // older version reads again. What does not fit one access (FP64 vectors, x of a refresh) is
 // published by a release atomic on an arrival counter that the CTAs poll, behind the sum's slots: the
 // fence alone costs 900 clocks.
-// All polls are bounded; a wait that runs out sets Scalars::fault and ends the launch.
+// All polls are bounded. A wait that runs out is final for its CTA: it sets Scalars::fault, posts no
+// further partial and leaves the launch, so that its teammates' next wait runs out too. What a team
+// leaves unsolved keeps Scalars::pending.
 // FP64 is slow on this GPU: an FP64 instruction occupies the SM's pipe for 16 clocks a warp and its
 // result takes about 100; a division takes about 1000. Measured per iteration of a small body with
 // FP64 trees and divisions: 1500 clocks of the update and 1000 of each sum. So sums are exact integer sums of
@@ -44,7 +46,8 @@ namespace {
 
 constexpr int kSolveMaxThreads = 512;
 constexpr int kL1Room = 32 << 10;             // shared memory left to the L1 where it serves the gathers
-constexpr int kPollLimit = 1 << 20;           // polls before a warp gives up (about a second)
+constexpr int kPollLimit = 1 << 20;           // polls of L2 before a warp gives up (about a second)
+constexpr int kSmemPollLimit = 16 * kPollLimit;  // of its shared memory
 constexpr int kTeamWarpSlots = kTeamMax / 32; // slots a lane of the polling warp reads
 
 
@@ -204,6 +207,7 @@ struct SolveSh
 	Fixed w[2][32];
 	double total, ratio;
 	int ok, lost;
+	int polls;  // of a gather that waits for a version
 	unsigned long long slot[2][kMaxTeamCtas];  // a cluster's partials
 };
 
@@ -229,16 +233,20 @@ struct GridTeam
 	SolveSh* sh;
 	TeamMemory* mem;
 	int ctas, rank;
-	int replicas;
+	int replicas, polls;
 	unsigned sums, fences;  // so far
 	int ok;
 	TV ratio;
 
-	__device__ __forceinline__ GridTeam(SolveSh* s, TeamMemory* m)
-	    : sh(s), mem(m), ctas(gridDim.x), rank(blockIdx.x), replicas(gridDim.x > 16 ? kTeamReplicas : 1), sums(0), fences(0),
-	      ok(1), ratio((TV)0)
+	__device__ __forceinline__ GridTeam(SolveSh* s, TeamMemory* m, int limit)
+	    : sh(s), mem(m), ctas(gridDim.x), rank(blockIdx.x), replicas(gridDim.x > 16 ? kTeamReplicas : 1),
+	      polls(limit > 0 ? limit : kPollLimit), sums(0), fences(0), ok(1), ratio((TV)0)
 	{
-		if (threadIdx.x == 0) sh->lost = 0;
+		if (threadIdx.x == 0)
+		{
+			sh->lost = 0;
+			sh->polls = polls;
+		}
 	}
 
 	// This warp's value v (the same in all lanes) summed over the team. `between` runs after this
@@ -264,7 +272,7 @@ struct GridTeam
 		{
 			const unsigned long long* mine = all[rank & (replicas - 1)];
 			unsigned long long u[kTeamWarpSlots];
-			int polls = 0;
+			int tries = 0;
 			bool there;
 			for (;;)
 			{
@@ -276,7 +284,7 @@ struct GridTeam
 					there = there && (u[q] & 3ull) == tag;
 				}
 				there = __all_sync(0xffffffffu, there) != 0;
-				if (there || ++polls > kPollLimit) break;
+				if (there || ++tries > polls) break;
 			}
 			// a lane's slots aligned to their largest exponent: 53-bit mantissas, so five of them
 			// stay below 2^58
@@ -298,7 +306,7 @@ struct GridTeam
 			{
 				const unsigned want = (fences + 1) * (unsigned)ctas;
 				while (ld_acquire(&mem->arrived) < want)
-					if (++polls > kPollLimit)
+					if (++tries > polls)
 					{
 						there = false;
 						break;
@@ -310,6 +318,7 @@ struct GridTeam
 				sh->total = total;
 				*(TV*)&sh->ratio = r;
 				sh->ok = there && !sh->lost ? 1 : 0;
+				if (!there) sh->lost = 1;
 			}
 		}
 		++sums;
@@ -345,16 +354,22 @@ struct ClusterTeam
 	SolveSh* sh;
 	int cta;          // rank in the cluster
 	int rank, base, ctas;
+	int polls;
 	unsigned sums;
 	int ok;
 	TV ratio;
 
 	// (the caller synchronises the cluster after this, and again before a CTA leaves the kernel)
-	__device__ __forceinline__ explicit ClusterTeam(SolveSh* s)
-	    : sh(s), cta((int)cooperative_groups::this_cluster().block_rank()), rank(0), base(0), ctas(1), sums(0), ok(1), ratio((TV)0)
+	__device__ __forceinline__ ClusterTeam(SolveSh* s, int limit)
+	    : sh(s), cta((int)cooperative_groups::this_cluster().block_rank()), rank(0), base(0), ctas(1),
+	      polls(limit > 0 ? limit : kSmemPollLimit), sums(0), ok(1), ratio((TV)0)
 	{
 		if (threadIdx.x < 2 * kMaxTeamCtas) (&sh->slot[0][0])[threadIdx.x] = 0ull;
-		if (threadIdx.x == 0) sh->lost = 0;
+		if (threadIdx.x == 0)
+		{
+			sh->lost = 0;
+			sh->polls = limit > 0 ? limit : kPollLimit;
+		}
 	}
 	__device__ __forceinline__ void form(int size)
 	{
@@ -396,12 +411,12 @@ struct ClusterTeam
 			{
 				unsigned long long u = tag;
 				const unsigned mine = (unsigned)__cvta_generic_to_shared(&sh->slot[buf][lane < ctas ? lane : 0]);
-				for (int polls = 0;;)
+				for (int tries = 0;;)
 				{
 					if (lane < ctas)
 						asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(u) : "r"(mine) : "memory");
 					there = __all_sync(0xffffffffu, (u & 3ull) == tag) != 0;
-					if (there || ++polls > 16 * kPollLimit) break;
+					if (there || ++tries > polls) break;
 				}
 				total = fixed_value(fixed_warp_sum(to_fixed(__longlong_as_double((long long)(u & ~3ull)))));
 				if (FENCE) __threadfence();
@@ -412,6 +427,7 @@ struct ClusterTeam
 				sh->total = total;
 				*(TV*)&sh->ratio = r;
 				sh->ok = there && !sh->lost ? 1 : 0;
+				if (!there) sh->lost = 1;
 			}
 		}
 		++sums;
@@ -577,7 +593,7 @@ __device__ __forceinline__ void team_spmv_row(const M& m, int w, int lane, const
 								old = true;
 							}
 				if (!old) break;
-				if (polls > kPollLimit || *(volatile int*)&sh->lost)
+				if (polls > sh->polls || *(volatile int*)&sh->lost)
 				{
 					sh->lost = 1;
 					break;
@@ -940,7 +956,7 @@ __device__ __forceinline__ void team_end(G& T, const DevBody& B, const SolveArgs
 		sc->delta = S.delta;
 		sc->delta0 = S.delta0;
 		sc->status = S.status;
-		sc->done = 1;
+		sc->pending = 0;
 	}
 	if (!T.ok && threadIdx.x == 0) sc->fault = 1;
 }
@@ -990,7 +1006,6 @@ __device__ __forceinline__ void team_solve(Team& T, const DevBody& B, const Solv
 		if constexpr (kVersions) st_version((float*)B.s, i, o, version);
 		else vst((TV*)B.s, i, o);
 	};
-	if (T.rank == 0 && threadIdx.x == 0 && P.newton <= 0) B.sc->fault = 0;
 	auto row = [&](int j, int i) { return Row(B, O.vec, j, O.vec_slices, lane, i); };
 
 	auto refresh_matrix = [&](int j, auto f) {
@@ -1209,7 +1224,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve(DevBody B, SolveArgs P)
 	__shared__ SolveSh sh;
 	if (P.newton > 0 && B.sc->newton_done) return;
 	constexpr int kDepth = THREADS <= 256 ? (sizeof(TV) == 8 ? 2 : 4) : 1;
-	GridTeam<TV> T(&sh, B.team);
+	GridTeam<TV> T(&sh, B.team, P.polls);
 	team_solve<TA, TV, FF, kDepth>(
 	    T, B, P, smem,
 	    [&](int i, float3 dv, bool finish) { return final_vertex_dv<LdPlain, FILTER>(B, i, P.h, P.newton == 0, finish, dv); },
@@ -1223,7 +1238,7 @@ __global__ void __launch_bounds__(256, 1) k_solve_cluster(DevBody B, SolveArgs P
 {
 	extern __shared__ __align__(16) unsigned char smem[];
 	__shared__ SolveSh sh;
-	ClusterTeam<TV> T(&sh);
+	ClusterTeam<TV> T(&sh, P.polls);
 	cooperative_groups::cluster_group cl = cooperative_groups::this_cluster();
 	cl.sync();
 	if (P.newton <= 0 || !B.sc->newton_done)
@@ -1252,12 +1267,11 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 	constexpr int kDepth = THREADS <= 256 ? 4 : 1;
 	typedef __nv_bfloat16 TA;
 	const int lane = threadIdx.x & 31;
-	GridTeam<float> T(&sh, B.team);
+	GridTeam<float> T(&sh, B.team, P.polls);
 	const OwnSlices<TA> O(B, (const TA*)B.Alo, smem, P.smem, kFcgVecBytes, P.keep, T.rank, T.ctas);
 	const float* sv = (const float*)B.s;
 	unsigned version = 0;  // of s
 	const float* pv = (const float*)B.d2;
-	if (blockIdx.x == 0 && threadIdx.x == 0 && P.newton <= 0) B.sc->fault = 0;
 	auto row = [&](int j, int i) { return Row(B, W, O.vec, j, O.vec_slices, lane, i); };
 	auto matrix32 = [&](int j, auto f) {
 		const int base = B.slice_ptr[O.s0 + j];

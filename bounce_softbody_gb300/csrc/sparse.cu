@@ -1133,7 +1133,6 @@ void release_sparse(b3g_context* c)
 		w->pA.release();
 		w->maps.release();
 		w->sys.reset();
-		if (w->sc) cudaFree(w->sc);
 		if (w->partials) cudaFree(w->partials);
 		if (w->team) cudaFree(w->team);
 		delete w;
@@ -1848,14 +1847,18 @@ int work_for(b3g_context* ctx, uint32_t n, SparseWork** out)
 	if (!ctx->sparse_work) ctx->sparse_work = new SparseWork();
 	SparseWork* w = ctx->sparse_work;
 	cudaError_t e = w->vecs.ensure(9 * 4 * std::max<size_t>(n, 1) * sizeof(float));
-	if (e == cudaSuccess && !w->sc) e = cudaMalloc(&w->sc, sizeof(Scalars));
 	if (e == cudaSuccess && !w->partials)
 	{
 		e = cudaMalloc(&w->partials, (kMaxPartials + 1) * sizeof(double));
 		if (e == cudaSuccess) e = cudaMemset(w->partials, 0, (kMaxPartials + 1) * sizeof(double));
 		w->sum = w->partials + kMaxPartials;
 	}
-	if (e == cudaSuccess && !w->team) e = cudaMalloc(&w->team, sizeof(TeamMemory));
+	if (e == cudaSuccess && !w->team)
+	{
+		// with the scalars behind it: both are cleared before a solve
+		e = cudaMalloc(&w->team, sizeof(TeamMemory) + sizeof(Scalars));
+		if (e == cudaSuccess) w->sc = (Scalars*)(w->team + 1);
+	}
 	if (e != cudaSuccess) return cuda_fail(e, "sparse solver workspace");
 	*out = w;
 	return B3G_OK;
@@ -1897,13 +1900,14 @@ int run_cg(b3g_context* ctx, SparseWork* w, const SpPattern* P, const float* A, 
 	S.refresh = 50;  // sparse_solver.cpp:83
 	S.newton = -1;
 	S.warm = 1;
-	cudaError_t e = op_solve_clear(D, st);
+	S.polls = ctx->polls;
+	cudaError_t e = cudaMemsetAsync(w->team, 0, sizeof(TeamMemory) + sizeof(Scalars), st);
 	if (e == cudaSuccess) e = op_solve(D, S, kP32, st);
 	if (e == cudaSuccess) e = cudaMemcpyAsync(ctx->h_scalars, w->sc, sizeof(Scalars), cudaMemcpyDeviceToHost, st);
 	if (e == cudaSuccess) e = cudaStreamSynchronize(st);
 	if (e != cudaSuccess) return cuda_fail(e, "sparse CG");
 	*out = *ctx->h_scalars;
-	if (out->fault) out->status = B3G_SOLVE_DEVICE_TIMEOUT;
+	if (timed_out(*out)) out->status = B3G_SOLVE_DEVICE_TIMEOUT;
 	return B3G_OK;
 }
 

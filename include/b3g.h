@@ -237,6 +237,10 @@ B3G_API int b3g_context_destroy(b3g_context* ctx);
 /* The CUDA stream (cudaStream_t) every call of this context is ordered on. */
 B3G_API int b3g_context_stream(b3g_context* ctx, void** stream);
 B3G_API int b3g_context_synchronize(b3g_context* ctx);
+/* The CTAs that solve a body together wait for one another. A wait gives up after this many polls;
+ * the step then ends without a valid result and reports B3G_SOLVE_DEVICE_TIMEOUT. 0 (the default):
+ * about a second. Applies to the calls that follow. */
+B3G_API int b3g_context_set_poll_limit(b3g_context* ctx, uint32_t polls);
 
 B3G_API int b3g_body_create(b3g_context* ctx, const b3g_body_desc* desc, b3g_body** out);
 B3G_API int b3g_body_destroy(b3g_body* body);
