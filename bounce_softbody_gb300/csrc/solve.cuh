@@ -17,11 +17,12 @@
 // sixteen 0.9 / 0.95 / 1.6. Two slot arrays alternate: a CTA can only overwrite its slot of sum e
 // with that of sum e + 2 after every CTA has arrived at sum e + 1, and so has read sum e. The same
 // holds for s, rewritten only after the sum that follows the sweep which gathers it.
-// s itself needs no barrier in the FP32 and BF16 modes: its fourth component carries the number of
-// its version, a vertex's 16 bytes are written and read as one access, and a gather that meets an
-// older version reads again. What does not fit one access (FP64 vectors, x of a refresh) is
-// published by a release atomic on an arrival counter that the CTAs poll, behind the sum's slots: the
-// fence alone costs 900 clocks.
+// s itself needs no barrier in the FP32 and BF16 modes on small bodies: its fourth component carries the
+// number of its version, a vertex's 16 bytes are written and read as one access at GPU scope, and a
+// gather that meets an older version reads again. What does not fit one access (FP64 vectors, x of a
+// refresh), and the s that a large body gathers through the L1, is published by a fence of the CTA's
+// first warp and a flag behind it that the team polls with the sum's slots: the fence alone costs 900
+// clocks, most of them beside the sum and the update of x.
 // All polls are bounded. A wait that runs out is final for its CTA: it sets Scalars::fault, posts no
 // further partial and leaves the launch, so that its teammates' next wait runs out too. What a team
 // leaves unsolved keeps Scalars::pending.
@@ -67,6 +68,7 @@ __device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
 	asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
 	return v;
 }
+__device__ __forceinline__ void fence_gpu() { asm volatile("fence.acq_rel.gpu;" ::: "memory"); }
 __device__ __forceinline__ void red_release(unsigned* p)
 {
 	asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
@@ -209,6 +211,7 @@ struct SolveSh
 	int ok, lost;
 	int polls;  // of a gather that waits for a version
 	unsigned long long slot[2][kMaxTeamCtas];  // a cluster's partials
+	unsigned fenced[kMaxTeamCtas];             // the last sum before which a cluster's CTA has fenced
 };
 
 // The sum of a CTA's warps, in warp 0 (v is each warp's value, already in sh->w[buf])
@@ -265,8 +268,8 @@ struct GridTeam
 		{
 			const unsigned long long bits = (unsigned long long)__double_as_longlong(cta_total(sh, buf, v));
 			if (lane < replicas) st_relaxed(all[lane] + rank, (bits & ~3ull) | tag);
-			if (FENCE && lane == 0) red_release(&mem->arrived);
 		}
+		if (FENCE && threadIdx.x == 0) red_release(&mem->arrived);
 		between();
 		if (warp == 0)
 		{
@@ -365,11 +368,21 @@ struct ClusterTeam
 	      polls(limit > 0 ? limit : kSmemPollLimit), sums(0), ok(1), ratio((TV)0)
 	{
 		if (threadIdx.x < 2 * kMaxTeamCtas) (&sh->slot[0][0])[threadIdx.x] = 0ull;
+		if (threadIdx.x < kMaxTeamCtas) sh->fenced[threadIdx.x] = 0u;
 		if (threadIdx.x == 0)
 		{
 			sh->lost = 0;
 			sh->polls = limit > 0 ? limit : kPollLimit;
 		}
+	}
+	// the address of a member's copy of a shared variable
+	__device__ __forceinline__ unsigned peer(const void* p, int member) const
+	{
+		unsigned remote;
+		asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+		             : "=r"(remote)
+		             : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(base + member));
+		return remote;
 	}
 	__device__ __forceinline__ void form(int size)
 	{
@@ -389,19 +402,17 @@ struct ClusterTeam
 		if (warp == 0)
 		{
 			total = cta_total(sh, buf, v);
-			if (ctas > 1)
+			if (lane < ctas && ctas > 1)
 			{
-				if (FENCE) __threadfence();
-				if (lane < ctas)
-				{
-					const unsigned long long bits = ((unsigned long long)__double_as_longlong(total) & ~3ull) | tag;
-					unsigned remote;
-					asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
-					             : "=r"(remote)
-					             : "r"((unsigned)__cvta_generic_to_shared(&sh->slot[buf][rank])), "r"(base + lane));
-					asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(remote), "l"(bits) : "memory");
-				}
+				const unsigned long long bits = ((unsigned long long)__double_as_longlong(total) & ~3ull) | tag;
+				asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(peer(&sh->slot[buf][rank], lane)), "l"(bits) : "memory");
 			}
+		}
+		if (FENCE && ctas > 1 && threadIdx.x >= blockDim.x - 32)
+		{
+			fence_gpu();
+			if (lane < ctas)
+				asm volatile("st.relaxed.cluster.shared::cluster.u32 [%0], %1;" ::"r"(peer(&sh->fenced[rank], lane)), "r"(sums + 1) : "memory");
 		}
 		between();
 		if (warp == 0)
@@ -410,16 +421,21 @@ struct ClusterTeam
 			if (ctas > 1)
 			{
 				unsigned long long u = tag;
+				unsigned fenced = sums + 1;
 				const unsigned mine = (unsigned)__cvta_generic_to_shared(&sh->slot[buf][lane < ctas ? lane : 0]);
+				const unsigned flag = (unsigned)__cvta_generic_to_shared(&sh->fenced[lane < ctas ? lane : 0]);
 				for (int tries = 0;;)
 				{
 					if (lane < ctas)
+					{
 						asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(u) : "r"(mine) : "memory");
-					there = __all_sync(0xffffffffu, (u & 3ull) == tag) != 0;
+						if (FENCE) asm volatile("ld.relaxed.cluster.shared::cta.u32 %0, [%1];" : "=r"(fenced) : "r"(flag) : "memory");
+					}
+					there = __all_sync(0xffffffffu, (u & 3ull) == tag && (int)(fenced - (sums + 1)) >= 0) != 0;
 					if (there || ++tries > polls) break;
 				}
 				total = fixed_value(fixed_warp_sum(to_fixed(__longlong_as_double((long long)(u & ~3ull)))));
-				if (FENCE) __threadfence();
+				if (FENCE) fence_gpu();
 			}
 			const TV r = ratio_of(total);
 			if (lane == 0)
@@ -478,26 +494,6 @@ __device__ __forceinline__ float4 ld_version(const float* s, int i)
 	return make_float4(__uint_as_float((unsigned)lo), __uint_as_float((unsigned)(lo >> 32)), __uint_as_float((unsigned)hi),
 	                   __uint_as_float((unsigned)(hi >> 32)));
 }
-// The same through the SM's L1, which may hold an older version (the caller reads that again). A sweep
-// whose matrix comes from L2 shares the L2-to-SM network with its gathers, a fourth of its bytes, and
-// a vertex is gathered about 15 times, mostly by one SM: the sweep of a large body goes through
-// the L1, which a fence empties of the last version between the sweeps, and the launch leaves it kL1Room
-// of the SM's memory. 64^3 block 11.7 -> 9.6 ms a step, PCG launch of 160 blocks 9.4 -> 7.9. On bodies that
-// shared memory holds, the extra reads of old lines cost 8-17 %.
-__device__ __forceinline__ float4 ld_version_l1(const float* s, int i)
-{
-	unsigned long long lo, hi;
-	asm volatile("{ .reg .b128 t; ld.relaxed.cta.global.b128 t, [%2]; mov.b128 {%0, %1}, t; }"
-	             : "=l"(lo), "=l"(hi)
-	             : "l"(s + 4 * (size_t)i)
-	             : "memory");
-	return make_float4(__uint_as_float((unsigned)lo), __uint_as_float((unsigned)(lo >> 32)), __uint_as_float((unsigned)hi),
-	                   __uint_as_float((unsigned)(hi >> 32)));
-}
-__device__ __forceinline__ void empty_l1()
-{
-	if (threadIdx.x == blockDim.x - 32) asm volatile("fence.acq_rel.gpu;" ::: "memory");
-}
 __device__ __forceinline__ void st_version(float* s, int i, const float o[3], unsigned version)
 {
 	const unsigned long long lo = (unsigned long long)__float_as_uint(o[0]) | ((unsigned long long)__float_as_uint(o[1]) << 32);
@@ -506,6 +502,24 @@ __device__ __forceinline__ void st_version(float* s, int i, const float o[3], un
 	             "l"(s + 4 * (size_t)i)
 	             : "memory");
 }
+
+// How a sweep gathers s (team_spmv_row): by its versions, or with the loads of a policy from a vector
+// that a fenced sum has published.
+struct GatherVersions
+{
+};
+// A sweep whose matrix comes from L2 shares the L2-to-SM network with its gathers, a fourth of its
+// bytes, and a vertex is gathered about 15 times, mostly by one SM: with many warps (DEPTH 1) the FP32
+// sweep gathers through the L1, and the launch leaves it kL1Room of the SM's memory. Other SMs write what
+// it reads, so each new s is fenced. ms a step by versions from L2 / by versions through the L1, which is a
+// race (the loads' scope is not the stores') / behind fences: 64^3 block 9.6 / 9.4 / 9.3, BF16 block of
+// 47x41x37 3.55 / 3.40 / 3.26, 160 blocks 10.3 / 10.0 / 10.1, 16 blocks and cloths 5.87 / 5.58 / 5.61, 12
+// blocks 1.42 / 1.38 / 1.44.
+template <class TV, int DEPTH>
+struct GatherOf
+{
+	typedef typename std::conditional<sizeof(TV) == 8, LdCG, typename std::conditional<DEPTH == 1, LdPlain, GatherVersions>::type>::type type;
+};
 
 // Where a slice's matrix comes from: shared memory (a chunk of nine planes and the column ids of
 // its w x 32 slots) or global memory with an L2 policy.
@@ -536,13 +550,13 @@ struct GlobalMat
 };
 
 // o = (A s)_i and own = s_i (the diagonal block leads every row); the products are summed in slot
-// order, as spmv_row sums them. VERSIONED: s is a float vector whose entries carry their version;
-// entries older than `version` are read again (sh->lost: a wait ran out).
+// order, as spmv_row sums them. G: how s is gathered; of a vector with versions, entries older than
+// `version` are read again (sh->lost: a wait ran out).
 // DEPTH groups of four blocks have their columns' s in flight at a time: the gathers go to L2, and a
 // thread that waits for them group by group pays that trip four times a row (matrix in shared
 // memory, few warps). With DEPTH 1 (many warps, matrix from L2) the column ids are read a group
 // ahead, so that a group's planes and gathers are in flight together.
-template <class TA, class TV, int DEPTH, bool VERSIONED, class M>
+template <class TA, class TV, int DEPTH, class G, class M>
 __device__ __forceinline__ void team_spmv_row(const M& m, int w, int lane, const TV* s, unsigned version, SolveSh* sh,
                                               TV o[3], TV own[3])
 {
@@ -570,15 +584,14 @@ __device__ __forceinline__ void team_spmv_row(const M& m, int w, int lane, const
 				jj[g][3] = c.w;
 			}
 		TV xv[DEPTH][4][3];
-		if constexpr (VERSIONED)
+		if constexpr (std::is_same<G, GatherVersions>::value)
 		{
 			float4 r[DEPTH][4];
 #pragma unroll
 			for (int g = 0; g < DEPTH; ++g)
 				if (g == 0 || k0 + g * kGroup < w)
 #pragma unroll
-					for (int u = 0; u < 4; ++u) r[g][u] = DEPTH == 1 ? ld_version_l1(s, jj[g][u]) : ld_version(s, jj[g][u]);
-			if (DEPTH == 1 && k0 + kGroup < w) ahead = m.cols(32 * (k0 + kGroup) + 4 * lane);
+					for (int u = 0; u < 4; ++u) r[g][u] = ld_version(s, jj[g][u]);
 			for (int polls = 0;; ++polls)
 			{
 				bool old = false;
@@ -615,7 +628,7 @@ __device__ __forceinline__ void team_spmv_row(const M& m, int w, int lane, const
 			for (int g = 0; g < DEPTH; ++g)
 				if (g == 0 || k0 + g * kGroup < w)
 #pragma unroll
-					for (int u = 0; u < 4; ++u) vld<TV, LdCG>(s, jj[g][u], xv[g][u]);
+					for (int u = 0; u < 4; ++u) vld<TV, G>(s, jj[g][u], xv[g][u]);
 			if (DEPTH == 1 && k0 + kGroup < w) ahead = m.cols(32 * (k0 + kGroup) + 4 * lane);
 		}
 		if (k0 == 0)
@@ -994,8 +1007,9 @@ __device__ __forceinline__ void team_solve(Team& T, const DevBody& B, const Solv
 	const OwnSlices<TA> O(B, sizeof(TA) == sizeof(float) ? (const TA*)B.A32 : (const TA*)B.Alo, smem, P.smem,
 	                      solve_vec_bytes<TV, FF>(), P.keep, T.rank, T.ctas);
 	const TV* sv = (const TV*)B.s;
-	// FP32 vectors: s carries its version, 0 as the assembly leaves it; FP64: every new s is fenced
-	constexpr bool kVersions = sizeof(TV) == 4;
+	// s carries its version, 0 as the assembly leaves it, or every new s is fenced
+	typedef typename GatherOf<TV, DEPTH>::type Gather;
+	constexpr bool kVersions = std::is_same<Gather, GatherVersions>::value;
 	constexpr bool kFence = !kVersions;
 	// BF16 blocks: the refresh uses the FP32 ones, and a residual that met the tolerance is confirmed
 	// by a refresh before the solve ends
@@ -1034,7 +1048,7 @@ __device__ __forceinline__ void team_solve(Team& T, const DevBody& B, const Solv
 				else
 				{
 					TV q[3], own[3];
-					team_spmv_row<typename std::conditional<kConfirm, float, TA>::type, TV, 1, false>(m, w, lane, (const TV*)B.py, 0u, T.sh, q, own);
+					team_spmv_row<typename std::conditional<kConfirm, float, TA>::type, TV, 1, LdCG>(m, w, lane, (const TV*)B.py, 0u, T.sh, q, own);
 #pragma unroll
 					for (int c = 0; c < 3; ++c) rr[c] = b[c] - q[c];
 				}
@@ -1126,7 +1140,7 @@ __device__ __forceinline__ void team_solve(Team& T, const DevBody& B, const Solv
 		part = O.template row_sum<TV>([&](int j, int i) {
 			const Row v = row(j, i);
 			TV o[3], dn[3];
-			O.matrix(j, [&](const auto& m, int w) { team_spmv_row<TA, TV, DEPTH, kVersions>(m, w, lane, sv, version, T.sh, o, dn); });
+			O.matrix(j, [&](const auto& m, int w) { team_spmv_row<TA, TV, DEPTH, Gather>(m, w, lane, sv, version, T.sh, o, dn); });
 			if (!first)
 			{
 				TV dp[3], qp[3];
@@ -1157,7 +1171,6 @@ __device__ __forceinline__ void team_solve(Team& T, const DevBody& B, const Solv
 			break;
 		}
 		const TV alpha = T.ratio;
-		if (kVersions && DEPTH == 1) empty_l1();
 		const Divisor<TV> by_delta(S.delta);
 		auto beta_of = [&](double t) { return by_delta.divide(t); };
 		double dn;
@@ -1265,6 +1278,8 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 	if (P.newton > 0 && B.sc->newton_done) return;
 	typedef FcgRowVecs Row;
 	constexpr int kDepth = THREADS <= 256 ? 4 : 1;
+	typedef typename GatherOf<float, kDepth>::type Gather;
+	constexpr bool kVersions = std::is_same<Gather, GatherVersions>::value;
 	typedef __nv_bfloat16 TA;
 	const int lane = threadIdx.x & 31;
 	GridTeam<float> T(&sh, B.team, P.polls);
@@ -1272,6 +1287,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 	const float* sv = (const float*)B.s;
 	unsigned version = 0;  // of s
 	const float* pv = (const float*)B.d2;
+	auto store_s = [&](int i, const float* o) {
+		if constexpr (kVersions) st_version((float*)B.s, i, o, version);
+		else vst((float*)B.s, i, o);
+	};
 	auto row = [&](int j, int i) { return Row(B, W, O.vec, j, O.vec_slices, lane, i); };
 	auto matrix32 = [&](int j, auto f) {
 		const int base = B.slice_ptr[O.s0 + j];
@@ -1340,13 +1359,13 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 			vld<float, LdPlain>(v.r, 0, r);
 			row_precond<float>(B, v.m, i, r, s);
 			vst(v.ri, 0, r);
-			st_version((float*)B.s, i, s, version);
+			store_s(i, s);
 			vst(v.z, 0, zero);
 			return term3(r, s);
 		});
 		// a warm start finds an s of any version: fenced once
-		if (P.warm && S.iter == 0) T.publish();
-		double delta = T.sum<false>(part);
+		if (kVersions && P.warm && S.iter == 0) T.publish();
+		double delta = T.sum<!kVersions>(part);
 		if (!T.ok) break;
 		float beta = 0.0f;
 		if (isfinite(delta) && delta > 0.0)
@@ -1355,7 +1374,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 				part = O.row_sum<float>([&](int j, int i) {
 					const Row v = row(j, i);
 					float o[3], dn[3];
-					O.matrix(j, [&](const auto& m, int w) { team_spmv_row<TA, float, kDepth, true>(m, w, lane, sv, version, &sh, o, dn); });
+					O.matrix(j, [&](const auto& m, int w) { team_spmv_row<TA, float, kDepth, Gather>(m, w, lane, sv, version, &sh, o, dn); });
 					if (it > 0)
 					{
 						float dp[3], qp[3];
@@ -1375,7 +1394,6 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 				const double dq = T.sum<false>(part, [] {}, [&](double t) { return Divisor<float>(t).divide(delta); });
 				if (!T.ok || !bits_finite(dq) || !bits_positive(dq)) break;
 				const float alpha = T.ratio;
-				if (kDepth == 1) empty_l1();
 				const Divisor<float> by_delta(delta);
 				++version;
 				part = O.row_sum<float>([&](int j, int i) {
@@ -1387,10 +1405,10 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 					for (int c = 0; c < 3; ++c) r[c] -= alpha * q[c];
 					row_precond<float>(B, v.m, i, r, s);
 					vst(v.ri, 0, r);
-					st_version((float*)B.s, i, s, version);
+					store_s(i, s);
 					return term3(r, s);
 				});
-				const double dn = T.sum<false>(part, [&] {
+				const double dn = T.sum<!kVersions>(part, [&] {
 					O.rows([&](int j, int i) {
 						const Row v = row(j, i);
 						row_x_update<float, false>(v.z, v.di, alpha);
@@ -1436,7 +1454,7 @@ __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, 
 		part = O.row_sum<float>([&](int j, int i) {
 			const Row v = row(j, i);
 			float o[3], p[3];
-			matrix32(j, [&](const auto& m, int w) { team_spmv_row<float, float, kDepth, false>(m, w, lane, pv, 0u, &sh, o, p); });
+			matrix32(j, [&](const auto& m, int w) { team_spmv_row<float, float, kDepth, LdCG>(m, w, lane, pv, 0u, &sh, o, p); });
 			vst(v.q, 0, o);
 			return term3(p, o);
 		});
