@@ -113,7 +113,7 @@ struct TeamMemory
 {
 	unsigned arrived;
 	unsigned pad[31];
-	unsigned long long tagged[2][kTeamReplicas][kTeamMax];
+	unsigned long long tagged[2][kTeamReplicas][kTeamMax][2];
 };
 
 // Everything a kernel needs about one body. Passed by value to the single-body kernels and read

@@ -9,8 +9,8 @@
 // d.q after q = A s + beta q, d = s + beta d, and r.s after r -= alpha q, s = M^-1 r. x += alpha d
 // runs while the second sum is on its way.
 //
-// Team sums. Every CTA stores its partial in its slot with two bits of the sum's number in the
-// lowest mantissa bits (4e-16 of the partial); one warp of every CTA polls all slots and adds them
+// Team sums. Every CTA stores its partial in its slot as two words, mantissa and exponent (Fixed), each
+// with two bits of the sum's number; one warp of every CTA polls all slots and adds them
 // up, so every thread holds the same bits and takes the same decisions. No fence and no atomic is on
 // that path. Above 16 CTAs the slots exist 16 times, a replica for every 16th CTA: with one copy
 // the pollers' traffic on the same lines costs 0.4 / 1.4 / 3.8 us a sum for 4 / 32 / 152 CTAs, with
@@ -28,9 +28,10 @@
 // leaves unsolved keeps Scalars::pending.
 // FP64 is slow on this GPU: an FP64 instruction occupies the SM's pipe for 16 clocks a warp and its
 // result takes about 100; a division takes about 1000. Measured per iteration of a small body with
-// FP64 trees and divisions: 1500 clocks of the update and 1000 of each sum. So sums are exact integer sums of
-// aligned mantissas (Fixed, error at most that of FP64 additions), comparisons are made on the bits, and
-// alpha and beta of the FP32 modes, which are rounded to float, are divided in float-float.
+// FP64 trees and divisions: 1500 clocks of the update and 1000 of each sum. So sums are integer sums of
+// mantissas of 58 bits aligned to the largest (Fixed), rounded to FP64 once at the end, comparisons are
+// made on the bits, and alpha and beta of the FP32 modes, which are rounded to float, are divided in
+// float-float.
 //
 // The rows' arithmetic is that of the launches it replaces, in the same order.
 #pragma once
@@ -52,14 +53,14 @@ constexpr int kSmemPollLimit = 16 * kPollLimit;  // of its shared memory
 constexpr int kTeamWarpSlots = kTeamMax / 32; // slots a lane of the polling warp reads
 
 
-__device__ __forceinline__ void st_relaxed(unsigned long long* p, unsigned long long v)
+__device__ __forceinline__ void st_relaxed(unsigned long long p[2], ulonglong2 v)
 {
-	asm volatile("st.relaxed.gpu.global.u64 [%0], %1;" ::"l"(p), "l"(v) : "memory");
+	asm volatile("st.relaxed.gpu.global.v2.u64 [%0], {%1, %2};" ::"l"(p), "l"(v.x), "l"(v.y) : "memory");
 }
-__device__ __forceinline__ unsigned long long ld_relaxed(const unsigned long long* p)
+__device__ __forceinline__ ulonglong2 ld_relaxed(const unsigned long long p[2])
 {
-	unsigned long long v;
-	asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
+	ulonglong2 v;
+	asm volatile("ld.relaxed.gpu.global.v2.u64 {%0, %1}, [%2];" : "=l"(v.x), "=l"(v.y) : "l"(p) : "memory");
 	return v;
 }
 __device__ __forceinline__ unsigned ld_acquire(const unsigned* p)
@@ -74,14 +75,15 @@ __device__ __forceinline__ void red_release(unsigned* p)
 	asm volatile("red.release.gpu.global.add.u32 [%0], 1;" ::"l"(p) : "memory");
 }
 
-// m 2^e with |m| < 2^58: a float's or a double's value, or a sum of such values to 2^-53 of the
-// largest (the precision of FP64 additions). e >= kNotFinite: not finite.
+// m 2^e with |m| < 2^58: a float's or a double's value, or a sum of such values, of each of which 57 bits
+// below the largest one's first are kept. Infinities have e >= kNotFinite and m as if they were numbers,
+// a NaN's e is kNaN or above and swamps them.
 struct Fixed
 {
 	long long m;
 	int e;
 };
-constexpr int kNotFinite = 1 << 20, kFixedZero = -(1 << 20);
+constexpr int kNotFinite = 1 << 20, kNaN = kNotFinite + 4096, kFixedZero = -(1 << 20);
 
 __device__ __forceinline__ Fixed to_fixed(float t)
 {
@@ -90,7 +92,7 @@ __device__ __forceinline__ Fixed to_fixed(float t)
 	const long long m = (long long)((u & 0x7fffffu) | (e > 0 ? 0x800000u : 0u)) << 34;
 	Fixed f;
 	f.m = (u >> 31) ? -m : m;
-	f.e = e == 0xff ? kNotFinite : (m == 0 ? kFixedZero : max(e, 1) - 184);
+	f.e = e == 0xff ? ((u & 0x7fffffu) ? kNaN : kNotFinite) : (m == 0 ? kFixedZero : max(e, 1) - 184);
 	return f;
 }
 __device__ __forceinline__ Fixed to_fixed(double t)
@@ -100,7 +102,7 @@ __device__ __forceinline__ Fixed to_fixed(double t)
 	const long long m = (long long)((u & 0xfffffffffffffull) | (e > 0 ? 0x10000000000000ull : 0ull)) << 5;
 	Fixed f;
 	f.m = (u >> 63) ? -m : m;
-	f.e = e == 0x7ff ? kNotFinite : (m == 0 ? kFixedZero : max(e, 1) - 1080);
+	f.e = e == 0x7ff ? ((u & 0xfffffffffffffull) ? kNaN : kNotFinite) : (m == 0 ? kFixedZero : max(e, 1) - 1080);
 	return f;
 }
 // back below 2^58
@@ -130,18 +132,39 @@ __device__ __forceinline__ Fixed fixed_warp_sum(Fixed a)
 	t.m = (long long)l0 + ((long long)l1 << 20) + ((long long)l2 << 40);
 	return t;
 }
-// the nearest double towards zero (|m| < 2^63)
+// The nearest double (|m| < 2^63): a normal number in a line, what is not one apart
+__device__ __noinline__ double fixed_rare(Fixed a)
+{
+	const unsigned long long u = (unsigned long long)(a.m < 0 ? -a.m : a.m), sign = a.m < 0 ? 1ull << 63 : 0ull;
+	if (a.e >= kNotFinite)  // a sum with opposite infinities is what is left of their ms: about 0
+		return __longlong_as_double(a.e >= kNaN || u < (1ull << 40) ? 0x7ff8000000000000ll : (long long)(sign | 0x7ff0000000000000ull));
+	if (u == 0 || a.e < -1137) return 0.0;
+	if (a.e + 63 - __clzll((long long)u) > 1023) return __longlong_as_double((long long)(sign | 0x7ff0000000000000ull));
+	// below the normal numbers: a multiple of 2^-1074
+	const int drop = -1074 - a.e;
+	return __longlong_as_double((long long)(sign | (drop > 0 ? (u + (1ull << (drop - 1))) >> drop : u << -drop)));
+}
 __device__ __forceinline__ double fixed_value(Fixed a)
 {
 	const unsigned long long u = (unsigned long long)(a.m < 0 ? -a.m : a.m);
-	const int lead = 63 - __clzll((long long)u);  // u = 1.xxx 2^lead
-	const int ex = a.e + lead + 1023;
-	const unsigned long long frac = ((u << (63 - lead)) >> 11) & 0xfffffffffffffull;
-	const unsigned long long v = ((unsigned long long)ex << 52) | frac | (a.m < 0 ? 1ull << 63 : 0ull);
-	if (u == 0 && a.e < kNotFinite) return 0.0;
-	if (ex <= 0) return 0.0;
-	if (ex >= 0x7ff) return __longlong_as_double(0x7ff8000000000000ll);
-	return __longlong_as_double((long long)v);
+	const int lz = __clzll((long long)u);
+	const int ex = a.e - lz + 1085;  // the exponent field less the mantissa's leading bit
+	if (u == 0 || (unsigned)ex >= 0x7feu) return fixed_rare(a);
+	const unsigned long long r = (((u << lz) >> 10) + 1ull) >> 1;
+	return __longlong_as_double((long long)((((unsigned long long)ex << 52) + r) | ((unsigned long long)a.m & (1ull << 63))));
+}
+// A partial in a slot: mantissa and exponent, each with the sum's two-bit number
+__device__ __forceinline__ ulonglong2 fixed_words(Fixed a, unsigned long long tag)
+{
+	return make_ulonglong2(((unsigned long long)a.m << 2) | tag, ((unsigned long long)(long long)a.e << 2) | tag);
+}
+__device__ __forceinline__ bool tagged(ulonglong2 w, unsigned long long tag) { return (w.x & 3ull) == tag && (w.y & 3ull) == tag; }
+__device__ __forceinline__ Fixed fixed_of(ulonglong2 w)
+{
+	Fixed a;
+	a.m = (long long)w.x >> 2;
+	a.e = (int)((long long)w.y >> 2);
+	return a;
 }
 
 // Comparisons on the bits of doubles (an FP64 comparison waits for the FP64 pipe)
@@ -210,12 +233,12 @@ struct SolveSh
 	double total, ratio;
 	int ok, lost;
 	int polls;  // of a gather that waits for a version
-	unsigned long long slot[2][kMaxTeamCtas];  // a cluster's partials
-	unsigned fenced[kMaxTeamCtas];             // the last sum before which a cluster's CTA has fenced
+	ulonglong2 slot[2][kMaxTeamCtas];  // a cluster's partials
+	unsigned fenced[kMaxTeamCtas];     // the last sum before which a cluster's CTA has fenced
 };
 
 // The sum of a CTA's warps, in warp 0 (v is each warp's value, already in sh->w[buf])
-__device__ __forceinline__ double cta_total(const SolveSh* sh, int buf, Fixed v)
+__device__ __forceinline__ Fixed cta_total(const SolveSh* sh, int buf, Fixed v)
 {
 	const int lane = threadIdx.x & 31, nw = blockDim.x >> 5;
 	if (nw > 1)
@@ -224,9 +247,10 @@ __device__ __forceinline__ double cta_total(const SolveSh* sh, int buf, Fixed v)
 		z.m = 0;
 		z.e = kFixedZero;
 		if (lane < nw) z = sh->w[buf][lane];
-		v = fixed_warp_sum(z);
+		z = fixed_warp_sum(z);
+		v = fixed_norm(z.m, z.e);
 	}
-	return fixed_value(v);
+	return v;
 }
 
 // The reduction memory (cleared before the launch) and this CTA's place in the team.
@@ -263,18 +287,19 @@ struct GridTeam
 		if (lane == 0) sh->w[buf][warp] = v;
 		__syncthreads();
 		const unsigned long long tag = (unsigned long long)(((sums >> 1) + 1) & 3);
-		unsigned long long(*all)[kTeamMax] = mem->tagged[buf];
+		unsigned long long(*all)[kTeamMax][2] = mem->tagged[buf];
 		if (warp == 0)
 		{
-			const unsigned long long bits = (unsigned long long)__double_as_longlong(cta_total(sh, buf, v));
-			if (lane < replicas) st_relaxed(all[lane] + rank, (bits & ~3ull) | tag);
+			const ulonglong2 w = fixed_words(cta_total(sh, buf, v), tag);
+			if (lane < replicas) st_relaxed(all[lane][rank], w);
 		}
 		if (FENCE && threadIdx.x == 0) red_release(&mem->arrived);
 		between();
 		if (warp == 0)
 		{
-			const unsigned long long* mine = all[rank & (replicas - 1)];
-			unsigned long long u[kTeamWarpSlots];
+			unsigned long long(*mine)[2] = all[rank & (replicas - 1)];
+			ulonglong2 u[kTeamWarpSlots];
+			const ulonglong2 none = fixed_words(Fixed{0, kFixedZero}, tag);
 			int tries = 0;
 			bool there;
 			for (;;)
@@ -283,20 +308,20 @@ struct GridTeam
 #pragma unroll
 				for (int q = 0; q < kTeamWarpSlots; ++q)
 				{
-					u[q] = lane + 32 * q < ctas ? ld_relaxed(mine + lane + 32 * q) : tag;
-					there = there && (u[q] & 3ull) == tag;
+					u[q] = lane + 32 * q < ctas ? ld_relaxed(mine[lane + 32 * q]) : none;
+					there = there && tagged(u[q], tag);
 				}
 				there = __all_sync(0xffffffffu, there) != 0;
 				if (there || ++tries > polls) break;
 			}
-			// a lane's slots aligned to their largest exponent: 53-bit mantissas, so five of them
-			// stay below 2^58
+			// a lane's slots aligned to their largest exponent and to 55 bits, so that five of them stay
+			// below 2^58
 			Fixed f[kTeamWarpSlots], t;
 			t.e = kFixedZero;
 #pragma unroll
 			for (int q = 0; q < kTeamWarpSlots; ++q)
 			{
-				f[q] = to_fixed(__longlong_as_double((long long)(u[q] & ~3ull)));
+				f[q] = fixed_of(u[q]);
 				t.e = max(t.e, f[q].e);
 			}
 			t.m = 0;
@@ -367,7 +392,7 @@ struct ClusterTeam
 	    : sh(s), cta((int)cooperative_groups::this_cluster().block_rank()), rank(0), base(0), ctas(1),
 	      polls(limit > 0 ? limit : kSmemPollLimit), sums(0), ok(1), ratio((TV)0)
 	{
-		if (threadIdx.x < 2 * kMaxTeamCtas) (&sh->slot[0][0])[threadIdx.x] = 0ull;
+		if (threadIdx.x < 2 * kMaxTeamCtas) (&sh->slot[0][0])[threadIdx.x] = make_ulonglong2(0ull, 0ull);
 		if (threadIdx.x < kMaxTeamCtas) sh->fenced[threadIdx.x] = 0u;
 		if (threadIdx.x == 0)
 		{
@@ -398,14 +423,15 @@ struct ClusterTeam
 		if (lane == 0) sh->w[buf][warp] = v;
 		__syncthreads();
 		const unsigned long long tag = (unsigned long long)(((sums >> 1) + 1) & 3);
-		double total = 0.0;
+		Fixed t = v;
 		if (warp == 0)
 		{
-			total = cta_total(sh, buf, v);
+			t = cta_total(sh, buf, v);
 			if (lane < ctas && ctas > 1)
 			{
-				const unsigned long long bits = ((unsigned long long)__double_as_longlong(total) & ~3ull) | tag;
-				asm volatile("st.relaxed.cluster.shared::cluster.u64 [%0], %1;" ::"r"(peer(&sh->slot[buf][rank], lane)), "l"(bits) : "memory");
+				const ulonglong2 w = fixed_words(t, tag);
+				asm volatile("st.relaxed.cluster.shared::cluster.v2.u64 [%0], {%1, %2};" ::"r"(peer(&sh->slot[buf][rank], lane)), "l"(w.x), "l"(w.y)
+				             : "memory");
 			}
 		}
 		if (FENCE && ctas > 1 && threadIdx.x >= blockDim.x - 32)
@@ -420,7 +446,7 @@ struct ClusterTeam
 			bool there = true;
 			if (ctas > 1)
 			{
-				unsigned long long u = tag;
+				ulonglong2 u = fixed_words(Fixed{0, kFixedZero}, tag);
 				unsigned fenced = sums + 1;
 				const unsigned mine = (unsigned)__cvta_generic_to_shared(&sh->slot[buf][lane < ctas ? lane : 0]);
 				const unsigned flag = (unsigned)__cvta_generic_to_shared(&sh->fenced[lane < ctas ? lane : 0]);
@@ -428,15 +454,16 @@ struct ClusterTeam
 				{
 					if (lane < ctas)
 					{
-						asm volatile("ld.relaxed.cluster.shared::cta.u64 %0, [%1];" : "=l"(u) : "r"(mine) : "memory");
+						asm volatile("ld.relaxed.cluster.shared::cta.v2.u64 {%0, %1}, [%2];" : "=l"(u.x), "=l"(u.y) : "r"(mine) : "memory");
 						if (FENCE) asm volatile("ld.relaxed.cluster.shared::cta.u32 %0, [%1];" : "=r"(fenced) : "r"(flag) : "memory");
 					}
-					there = __all_sync(0xffffffffu, (u & 3ull) == tag && (int)(fenced - (sums + 1)) >= 0) != 0;
+					there = __all_sync(0xffffffffu, tagged(u, tag) && (int)(fenced - (sums + 1)) >= 0) != 0;
 					if (there || ++tries > polls) break;
 				}
-				total = fixed_value(fixed_warp_sum(to_fixed(__longlong_as_double((long long)(u & ~3ull)))));
+				t = fixed_warp_sum(fixed_of(u));
 				if (FENCE) fence_gpu();
 			}
+			const double total = fixed_value(t);
 			const TV r = ratio_of(total);
 			if (lane == 0)
 			{
