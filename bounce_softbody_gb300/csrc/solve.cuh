@@ -175,10 +175,14 @@ __device__ __forceinline__ bool bits_at_most(double x, double y) { return __doub
 
 // a / b rounded to the vector type. For float, in double-single arithmetic (Dekker, A floating-point
 // technique for extending the available precision, 1971): each mantissa as two floats, the
-// denominator's reciprocal as an estimate and its correction, good to about 2^-44 before the rounding
-// to 24 bits. The reciprocal is formed ahead where the denominator is known ahead.
+// denominator's reciprocal as an estimate and its correction. The quotient is good to 2^-42, 2^-18 of
+// half a float's unit in the last place; one that close to the midpoint of two floats, or beside a power
+// of two, takes the FP64 division (once in about 2^13), so the result is always its result. The
+// reciprocal is formed ahead where the denominator is known ahead.
 template <class TV>
 struct Divisor;
+// (a call, so that no part of it is on the way of the others)
+__device__ __noinline__ float divide_fp64(double a, double b) { return (float)(a / b); }
 template <>
 struct Divisor<double>
 {
@@ -211,11 +215,16 @@ struct Divisor<float>
 		const float ah = __uint_as_float(0x3f800000u | (unsigned)((u >> 29) & 0x7fffffu));
 		const float al = (float)(unsigned)(u & 0x1fffffffu) * 0x1p-52f;
 		const float q0 = ah * hi;
-		const float q = q0 + (fmaf(ah, hi, -q0) + fmaf(ah, lo, al * hi));
+		const float c = fmaf(ah, hi, -q0) + fmaf(ah, lo, al * hi);
+		const float q = q0 + c;
 		const unsigned qb = __float_as_uint(q);
+		// what the rounding to q left (exact), against half a unit in the last place
+		const float left = fabsf((q0 - q) + c), half = __uint_as_float((qb & 0x7f800000u) - (24u << 23));
 		const int ex = (int)(qb >> 23) + (ea - e);
-		// a zero, a denormal, a value that is not finite, or a quotient outside the normal floats
-		if (ea == 0 || ea == 0x7ff || e == 0 || e == 0x7ff || ex <= 0 || ex >= 0xff) return (float)(a / b);
+		// or a zero, a denormal, a value that is not finite, or a quotient outside the normal floats
+		if (left > half * (1.0f - 0x1p-13f) || !(qb & 0x7fffffu) || ea == 0 || ea == 0x7ff || e == 0 || e == 0x7ff || ex <= 0 ||
+		    ex >= 0xff)
+			return divide_fp64(a, b);
 		return __uint_as_float((qb & 0x7fffffu) | ((unsigned)ex << 23) | (((u >> 63) != 0) != neg ? 0x80000000u : 0u));
 	}
 };

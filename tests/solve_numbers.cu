@@ -1,4 +1,5 @@
-// Team sums of the solve launches on given values: the grid's and a cluster's, fenced and not.
+// Team sums of the solve launches on given values, the grid's and a cluster's, fenced and not, and their
+// divisions.
 #include "solve.cuh"
 
 #include <cmath>
@@ -42,6 +43,12 @@ __global__ void cluster_sums(const double* in, double* out)
 	cooperative_groups::this_cluster().sync();
 }
 
+__global__ void divisions(const double* in, double* out, int count)
+{
+	const int k = blockIdx.x * blockDim.x + threadIdx.x;
+	if (k < count) out[k] = (double)Divisor<float>(in[2 * k + 1]).divide(in[2 * k]);
+}
+
 bool ok(cudaError_t e)
 {
 	if (e != cudaSuccess) std::fprintf(stderr, "%s\n", cudaGetErrorString(e));
@@ -50,7 +57,8 @@ bool ok(cudaError_t e)
 
 } // namespace numbers
 
-// stdin: ctas, warps, cluster (0: the grid), then ctas * warps * kRounds doubles; stdout: ctas * kRounds
+// stdin: ctas, warps, cluster (0: the grid), then ctas * warps * kRounds doubles; stdout: ctas * kRounds.
+// Or: count, 0, -1, then count pairs of doubles; stdout: count quotients.
 int main()
 {
 	using namespace numbers;
@@ -58,6 +66,23 @@ int main()
 	while (std::fread(shape, sizeof(int), 3, stdin) == 3)
 	{
 		const int ctas = shape[0], warps = shape[1], cluster = shape[2];
+		if (cluster < 0)
+		{
+			const int count = ctas;
+			if (count < 1 || count > 1 << 24) return 2;
+			std::vector<double> in(2 * (size_t)count), out(count);
+			if (std::fread(in.data(), sizeof(double), in.size(), stdin) != in.size()) return 2;
+			double *din = nullptr, *dout = nullptr;
+			if (!ok(cudaMalloc(&din, in.size() * sizeof(double))) || !ok(cudaMalloc(&dout, out.size() * sizeof(double))) ||
+			    !ok(cudaMemcpy(din, in.data(), in.size() * sizeof(double), cudaMemcpyHostToDevice)))
+				return 3;
+			divisions<<<(count + 255) / 256, 256>>>(din, dout, count);
+			if (!ok(cudaGetLastError()) || !ok(cudaMemcpy(out.data(), dout, out.size() * sizeof(double), cudaMemcpyDeviceToHost))) return 3;
+			cudaFree(din);
+			cudaFree(dout);
+			std::fwrite(out.data(), sizeof(double), out.size(), stdout);
+			continue;
+		}
 		if (ctas < 1 || ctas > kTeamMax || warps < 1 || warps > kWarpsMax || (cluster && cluster != ctas) || cluster > kMaxTeamCtas) return 2;
 		std::vector<double> in((size_t)ctas * warps * kRounds), out((size_t)ctas * kRounds);
 		if (std::fread(in.data(), sizeof(double), in.size(), stdin) != in.size()) return 2;

@@ -1,5 +1,6 @@
 """The team sums of the solve launches against exactly rounded sums (math.fsum): as accurate as FP64
-additions, for every team, and a sum of infinities and NaN what IEEE arithmetic gives."""
+additions, for every team, and a sum of infinities and NaN what IEEE arithmetic gives. Their divisions
+against FP64 ones rounded to float."""
 import math
 import os
 import subprocess
@@ -81,3 +82,30 @@ def test_sums_that_are_not_finite(program, team):
         v[0, r], v[-1, r], want[r] = a, b, c
     got = team_sums(program, team, v)
     assert np.array_equal(got, want, equal_nan=True)
+
+
+def test_divisions_are_fp64_ones_rounded_to_float(program):
+    rng = np.random.default_rng(7)
+    n = 1 << 20
+    b = np.ldexp(rng.uniform(1.0, 2.0, n), rng.integers(-60, 60, n)) * rng.choice([-1.0, 1.0], n)
+    # quotients anywhere
+    a = np.ldexp(rng.uniform(1.0, 2.0, n), rng.integers(-60, 60, n))
+    # quotients at the midpoint of two floats, to a few units in the last place of a double
+    q = rng.uniform(1.0, 2.0, n).astype(np.float32)
+    q[: n // 16] = np.float32(1.0)
+    q[n // 16: n // 8] = np.nextafter(np.float32(2.0), np.float32(0.0))
+    mid = q.astype(np.float64) + 2.0 ** -24 * rng.choice([-1.0, -0.5, 1.0], n)
+    near = (mid * b).view(np.int64) + rng.integers(-6, 7, n)
+    special = np.array([0.0, -0.0, 1.0, -3.0, 5e-324, 2.0 ** -1022, np.finfo(float).max, np.inf, -np.inf, np.nan, 1e-30,
+                        1e30, 2.0 ** 127, 2.0 ** -126, 2.0 ** -149])
+    sa, sb = (x.ravel() for x in np.meshgrid(special, special))
+    num, den = np.concatenate([a, near.view(np.float64), sa]), np.concatenate([b, b, sb])
+    with np.errstate(all="ignore"):
+        want = (num / den).astype(np.float32)
+    pairs = np.ascontiguousarray(np.stack([num, den], 1))
+    out = subprocess.run([program], input=np.array([len(num), 0, -1], np.int32).tobytes() + pairs.tobytes(),
+                         stdout=subprocess.PIPE, check=True, timeout=120).stdout
+    got = np.frombuffer(out).astype(np.float32)
+    nan = np.isnan(want)
+    assert np.isnan(got[nan]).all()
+    assert np.array_equal(got[~nan].view(np.uint32), want[~nan].view(np.uint32))
