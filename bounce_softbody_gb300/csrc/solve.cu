@@ -1,7 +1,9 @@
 // Launch of the grid team's PCG (solve.cuh).
 #include "solve.cuh"
+#include "solve_rule.h"
 
 #include <algorithm>
+#include <cstdlib>
 
 namespace b3g {
 
@@ -87,15 +89,44 @@ cudaError_t launch_team(void (*kernel)(Args...), const Geometry& g, cudaStream_t
 	return cudaLaunchKernelEx(&cfg, kernel, args...);
 }
 
-// CTAs of the one cluster that solves a small body, 0 for a body that takes the grid team: about two
-// slices a CTA, up to eight on 16 CTAs. Measured with the grid team / 8 / 4 / 2 slices a CTA, us a step:
-// 378 vertices with three Newton iterations 823 / 723 / 657 / 628, 10^3 block 215 / 208 / 186 / 179, cloth of
-// 3721 vertices 220 / 186 / 183 / 183.
-int cluster_ctas(const DevBody& B)
+// The launch of one cluster of `cl` CTAs
+template <class... Args>
+cudaError_t cluster_config(void (*kernel)(Args...), int cl, int threads, int smem, cudaStream_t st, cudaLaunchConfig_t* cfg,
+                           cudaLaunchAttribute* attr)
 {
-	int cl = 1;
-	while (cl < kMaxTeamCtas && B.nslices > 2 * cl) cl *= 2;
-	return B.nslices <= 8 * cl ? cl : 0;
+	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, device().room);
+	if (e == cudaSuccess && cl > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+	*cfg = {};
+	cfg->gridDim = dim3((unsigned)cl, 1, 1);
+	cfg->blockDim = dim3((unsigned)threads, 1, 1);
+	cfg->dynamicSmemBytes = (size_t)smem;
+	cfg->stream = st;
+	attr->id = cudaLaunchAttributeClusterDimension;
+	attr->val.clusterDim.x = (unsigned)cl;
+	attr->val.clusterDim.y = 1;
+	attr->val.clusterDim.z = 1;
+	cfg->attrs = attr;
+	cfg->numAttrs = 1;
+	return e;
+}
+
+// The widest cluster that the device can hold, 0 if none: 16 CTAs need a GPC with as many SMs for them,
+// which a part of a device need not have. B3G_SOLVE_CLUSTER caps it (read once).
+template <class... Args>
+int widest_cluster(void (*kernel)(Args...))
+{
+	const char* cap = std::getenv("B3G_SOLVE_CLUSTER");
+	for (int cl = kMaxTeamCtas; cl > 0; cl /= 2)
+	{
+		cudaLaunchConfig_t cfg;
+		cudaLaunchAttribute attr;
+		int clusters = 0;
+		if (!(cap && cl > std::atoi(cap)) && cluster_config(kernel, cl, 256, device().room, nullptr, &cfg, &attr) == cudaSuccess &&
+		    cudaOccupancyMaxActiveClusters(&clusters, kernel, &cfg) == cudaSuccess && clusters > 0)
+			return cl;
+		cudaGetLastError();
+	}
+	return 0;
 }
 
 template <class TA, class TV, bool FF, bool FILTER>
@@ -106,28 +137,17 @@ cudaError_t launch_cluster(const DevBody& B, SolveArgs P, int cl, cudaStream_t s
 	const size_t want = (size_t)slices * (solve_vec_bytes<TV, FF>() + (size_t)B.maxw * kSlice * solve_slot_bytes<TA>());
 	P.smem = (int)(std::min(want, (size_t)device().room) & ~(size_t)127);
 	P.keep = 1024;
-	cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, device().room);
-	if (e == cudaSuccess && cl > 8) e = cudaFuncSetAttribute(kernel, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-	if (e != cudaSuccess) return e;
-	cudaLaunchConfig_t cfg = {};
-	cfg.gridDim = dim3((unsigned)cl, 1, 1);
-	cfg.blockDim = dim3((unsigned)(32 * slices), 1, 1);
-	cfg.dynamicSmemBytes = (size_t)P.smem;
-	cfg.stream = st;
-	cudaLaunchAttribute attr[1];
-	attr[0].id = cudaLaunchAttributeClusterDimension;
-	attr[0].val.clusterDim.x = (unsigned)cl;
-	attr[0].val.clusterDim.y = 1;
-	attr[0].val.clusterDim.z = 1;
-	cfg.attrs = attr;
-	cfg.numAttrs = 1;
-	return cudaLaunchKernelEx(&cfg, kernel, B, P);
+	cudaLaunchConfig_t cfg;
+	cudaLaunchAttribute attr;
+	cudaError_t e = cluster_config(kernel, cl, 32 * slices, P.smem, st, &cfg, &attr);
+	return e == cudaSuccess ? cudaLaunchKernelEx(&cfg, kernel, B, P) : e;
 }
 
 template <class TA, class TV, bool FF, bool FILTER>
 cudaError_t launch_solve(const DevBody& B, SolveArgs P, cudaStream_t st)
 {
-	const int cl = cluster_ctas(B);
+	static const int widest = widest_cluster(k_solve_cluster<TA, TV, FF, FILTER>);
+	const int cl = cluster_ctas(B.nslices, widest);
 	if (cl > 0) return launch_cluster<TA, TV, FF, FILTER>(B, P, cl, st);
 	// FP64 sweeps wait for the FP64 pipe, so they spread over every SM
 	const Geometry g = geometry(B, solve_vec_bytes<TV, FF>(), solve_slot_bytes<TA>(), sizeof(TV) == 8 ? 1 : 4);
