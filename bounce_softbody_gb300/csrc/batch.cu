@@ -9,6 +9,10 @@
 // events, restores the snapshot and keeps the fastest. Set B3G_AUTOTUNE=0 to use a fixed rule, or
 // B3G_BATCH_SCHEDULE="cluster,threshold[,lpt[,per[,helper]]]" to force a schedule (without `per`,
 // bodies of `threshold` vertices or more take a whole cluster and the others one CTA).
+//
+// The whole-step launch of more than kFlatNewton Newton iterations runs other CTAs (several an SM) on a
+// schedule of its own: bodies of at least `threshold` vertices take clusters, the others one CTA. A
+// batch keeps one schedule of each kind, made when a step first needs it.
 #include "api_internal.h"
 
 #include <algorithm>
@@ -29,6 +33,14 @@ struct Snapshot
 	size_t bytes;
 };
 
+// A schedule and the autotuner's candidates for it
+struct BatchSchedule
+{
+	bool known = false, tuned = false;
+	int cluster = 1, threshold = 1 << 30, lpt = 0, per = 0, helper = 0;
+	std::vector<std::pair<int, double>> tune_log;  // (candidate's code in b3g_batch_schedule, ms)
+};
+
 struct BatchCache
 {
 	std::vector<b3g_body*> bodies;
@@ -46,13 +58,13 @@ struct BatchCache
 	int helper = 0;              // CTAs of a cluster of the second solve launch (0: none)
 	int nbig = 0;
 	int ctas = 0;
-	bool tuned = false;
+	int whole = -1;              // kind of the schedule in force: 1 the whole-step launch's, 0 the solve launch's
+	BatchSchedule sched[2];
 	// graph of (memset queue, batch launch) for one step with the current parameters
 	cudaGraphExec_t graph = nullptr;
 	float g_h = 0.0f;
 	int g_newton = 0, g_max_iter = 0, g_refresh = 0, g_polls = 0;
 	double g_tol2 = 0.0, g_ntol2 = 0.0;
-	std::vector<std::pair<int, double>> tune_log;  // (cluster * 1e6 + threshold, ms)
 	unsigned long long* d_prof = nullptr;          // phase cycle counters when B3G_PHASE_PROFILE=1
 	unsigned* d_flat_off = nullptr;                 // flat numbering: element offsets, then slice offsets
 	unsigned nelem = 0, nslices = 0;
@@ -134,13 +146,14 @@ int team_width(const BatchCache* c, int k)
 
 // Estimated solve time of body k on a team of `width` CTAs, in units of a CTA's pass over one slice:
 // a sweep of ceil(slices / width) passes an iteration and about eleven passes' worth of team sums
-// and latency. Iteration counts come from a step already taken; before one is known every body
-// counts one iteration, so the order is by size.
+// and latency (in the whole-step launch a warp's passes, and two of them). Iteration counts come from a
+// step already taken; before one is known every body counts one iteration, so the order is by size.
 double est_time(const BatchCache* c, int k, int width)
 {
 	const double slices = std::ceil((double)c->bodies[k]->n / kSlice);
 	const double it = c->iters.empty() || c->iters[k] <= 0 ? 1.0 : (double)c->iters[k];
-	return it * (11.0 + std::ceil(slices / width));
+	constexpr int kCtaWarps = B3G_PCG_THREADS / 32;
+	return c->whole > 0 ? it * (2.0 + std::ceil(slices / (kCtaWarps * width))) : it * (11.0 + std::ceil(slices / width));
 }
 
 // The solve launch's schedule: clusters of `cluster` CTAs; with per > 0 a body's team is the part of
@@ -270,28 +283,39 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 	std::vector<Snapshot> L = snapshot_list(c, store, &total);
 	for (const Snapshot& s : L) cudaMemcpyAsync(s.dst, s.src, s.bytes, cudaMemcpyDeviceToDevice, st);
 
-	// candidates: (cluster size, slices per CTA of a team, queue order, cluster size of a helper launch)
+	// candidates: (cluster size, slices per CTA of a team, queue order, cluster size of a helper launch),
+	// or for the whole-step launch (cluster size, 0, queue order, 0, size threshold of its clusters)
 	struct Cand
 	{
-		int cl, per, lpt, helper;
+		int cl, per, lpt, helper, thr;
 	};
 	std::vector<Cand> cands;
-	const int clusters[] = {16, 8, 4};
-	const int pers[] = {2, 4, 8, 16, 32, 64};
-	for (int cl : clusters)
-		if (batch_max_clusters(c->prec, cl) > 0)  // 16-CTA clusters need hardware support
-			for (int p : pers)
-				for (int o = 0; o < 2; ++o) cands.push_back({cl, p, o, 0});
+	if (c->whole)
+	{
+		int maxn = 0;
+		for (b3g_body* b : c->bodies) maxn = std::max(maxn, (int)b->n);
+		for (int o = 0; o < 2; ++o) cands.push_back({1, 0, o, 0, 1 << 30});
+		for (int cl : {2, 4, 8, 16})
+			if (batch_max_clusters(c->prec, cl) > 0)
+				for (int t : {1, 1024, 2048, 4096, 8192, 16384, 32768})
+					for (int o = 0; t <= maxn && o < 2; ++o) cands.push_back({cl, 0, o, 0, t});
+	}
+	else
+		for (int cl : {16, 8, 4})
+			if (batch_max_clusters(c->prec, cl) > 0)  // 16-CTA clusters need hardware support
+				for (int p : {2, 4, 8, 16, 32, 64})
+					for (int o = 0; o < 2; ++o) cands.push_back({cl, p, o, 0, 0});
+	c->sched[c->whole].tune_log.clear();
 	cudaEvent_t e0, e1;
 	cudaEventCreate(&e0);
 	cudaEventCreate(&e1);
 	float best = 1e30f;
-	Cand best_c = {0, 0, 0, 0};
+	Cand best_c = {0, 0, 0, 0, 0};
 	const size_t plain = cands.size();
 	for (size_t n = 0; n < cands.size(); ++n)
 	{
 		const Cand cd = cands[n];
-		set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per, cd.helper);
+		set_schedule(c, cd.cl, cd.thr, ctx->sm_count, st, cd.lpt, cd.per, cd.helper);
 		BatchArgs A = make_args(ctx, c, h, 1, cfg);
 		if (use_side_stream(ctx, &A) != B3G_OK) e = cudaErrorUnknown;
 		if (e == cudaSuccess) e = op_batch(A, st);  // warm-up
@@ -305,7 +329,7 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 				e = cudaErrorUnknown;
 				break;
 			}
-			set_schedule(c, cd.cl, 0, ctx->sm_count, st, cd.lpt, cd.per, cd.helper);
+			set_schedule(c, cd.cl, cd.thr, ctx->sm_count, st, cd.lpt, cd.per, cd.helper);
 			A = make_args(ctx, c, h, 1, cfg);
 			use_side_stream(ctx, &A);
 		}
@@ -318,17 +342,19 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 		if (e != cudaSuccess) break;
 		float ms = 0.0f;
 		cudaEventElapsedTime(&ms, e0, e1);
-		c->tune_log.push_back({cd.lpt * 100000000 + cd.cl * 1000000 + cd.helper * 1000 + cd.per, (double)ms});
+		c->sched[c->whole].tune_log.push_back({c->whole * 1000000000 + cd.lpt * 100000000 + cd.cl * 1000000 +
+		                                           (c->whole ? std::min(cd.thr, 999999) : cd.helper * 1000 + cd.per),
+		                                       (double)ms});
 		if (ms < best)
 		{
 			best = ms;
 			best_c = cd;
 		}
-		if (n + 1 == plain && cfg.force_iterations <= (uint32_t)kFlatNewton)
+		if (n + 1 == plain && !c->whole)
 		{
 			// the best of those with a helper launch, and with wider teams for it to take from
 			for (int hw : {8, 4, 2})
-				for (int f : {1, 2, 4}) cands.push_back({best_c.cl, f * best_c.per, best_c.lpt, hw});
+				for (int f : {1, 2, 4}) cands.push_back({best_c.cl, f * best_c.per, best_c.lpt, hw, 0});
 		}
 	}
 	cudaStreamSynchronize(st);
@@ -336,8 +362,53 @@ int autotune(b3g_context* ctx, BatchCache* c, float h, const b3g_solver_config& 
 	cudaEventDestroy(e1);
 	cudaFree(store);
 	if (e != cudaSuccess) return cuda_fail(e, "batch autotune");
-	if (best_c.cl > 0) set_schedule(c, best_c.cl, 0, ctx->sm_count, st, best_c.lpt, best_c.per, best_c.helper);
-	c->tuned = true;
+	if (best_c.cl > 0) set_schedule(c, best_c.cl, best_c.thr, ctx->sm_count, st, best_c.lpt, best_c.per, best_c.helper);
+	c->sched[c->whole].tuned = true;
+	return B3G_OK;
+}
+
+// The schedule of the batch's launches of one kind in force: the one kept, or the forced, the tuned
+// or else the fixed rule's one.
+int use_schedule(b3g_context* ctx, BatchCache* c, int whole, float h, const b3g_solver_config& cfg)
+{
+	if (c->whole == whole) return B3G_OK;
+	c->whole = whole;
+	cudaStream_t st = ctx->stream;
+	BatchSchedule& S = c->sched[whole];
+	if (S.known)
+	{
+		set_schedule(c, S.cluster, S.threshold, ctx->sm_count, st, S.lpt, S.per, S.helper);
+		return B3G_OK;
+	}
+	// until the autotuner has looked (or where it may not): about 16 slices a CTA of the solve launch,
+	// clusters of 4 for bodies of 16k vertices or more in the whole-step launch
+	int maxn = 0;
+	for (b3g_body* b : c->bodies) maxn = std::max(maxn, (int)b->n);
+	if (!whole) set_schedule(c, 8, 0, ctx->sm_count, st, 0, 16);
+	else if (maxn >= 16384) set_schedule(c, 4, 16384, ctx->sm_count, st);
+	else set_schedule(c, 1, 1 << 30, ctx->sm_count, st);
+	const char* env = std::getenv("B3G_AUTOTUNE");
+	const char* forced = std::getenv("B3G_BATCH_SCHEDULE");  // "cluster,threshold[,lpt[,per[,helper]]]"
+	int fc = 0, ft = 0, fo = 0, fp = 0, fh = 0;
+	auto size = [](int x) { return x == 1 || x == 2 || x == 4 || x == 8 || x == 16; };
+	if (forced && std::sscanf(forced, "%d,%d,%d,%d,%d", &fc, &ft, &fo, &fp, &fh) >= 2 && size(fc))
+		set_schedule(c, fc, ft > 0 ? ft : (1 << 30), ctx->sm_count, st, fo ? 1 : 0, std::max(fp, 0),
+		             size(fh) && fh > 1 && fh < fc ? fh : 0);
+	else if (!(env && env[0] == '0'))
+	{
+		const int rc = autotune(ctx, c, h, cfg);
+		if (rc != B3G_OK)
+		{
+			c->whole = -1;
+			return rc;
+		}
+	}
+	S.known = true;
+	S.cluster = c->cluster;
+	S.threshold = c->threshold;
+	S.lpt = c->lpt;
+	S.per = c->per;
+	S.helper = c->helper;
 	return B3G_OK;
 }
 
@@ -423,8 +494,6 @@ int build_cache(b3g_context* ctx, b3g_body* const* bodies, uint32_t count, int p
 		if (cudaMalloc(&c->d_prof, bytes) == cudaSuccess) cudaMemset(c->d_prof, 0, bytes);
 		else cudaGetLastError();
 	}
-	// until the autotuner has looked (or where it may not): about 16 slices a CTA
-	set_schedule(c, 8, 0, ctx->sm_count, ctx->stream, 0, 16);
 	*out = c;
 	return B3G_OK;
 }
@@ -516,19 +585,9 @@ extern "C" int b3g_step_batch(b3g_context* ctx, b3g_body* const* bodies, uint32_
 		rc = build_cache(ctx, bodies, count, prec, cfg.preconditioner, filter, &c);
 		if (rc != B3G_OK) return rc;
 		ctx->batch = c;
-		const char* env = std::getenv("B3G_AUTOTUNE");
-		const char* forced = std::getenv("B3G_BATCH_SCHEDULE");  // "cluster,threshold[,lpt[,per[,helper]]]"
-		int fc = 0, ft = 0, fo = 0, fp = 0, fh = 0;
-		auto size = [](int x) { return x == 1 || x == 2 || x == 4 || x == 8 || x == 16; };
-		if (forced && std::sscanf(forced, "%d,%d,%d,%d,%d", &fc, &ft, &fo, &fp, &fh) >= 2 && size(fc))
-			set_schedule(c, fc, ft > 0 ? ft : (1 << 30), ctx->sm_count, ctx->stream, fo ? 1 : 0, std::max(fp, 0),
-			             size(fh) && fh > 1 && fh < fc ? fh : 0);
-		else if (!(env && env[0] == '0'))
-		{
-			rc = autotune(ctx, c, dt, cfg);
-			if (rc != B3G_OK) return rc;
-		}
 	}
+	rc = use_schedule(ctx, c, cfg.force_iterations > (uint32_t)kFlatNewton ? 1 : 0, dt, cfg);
+	if (rc != B3G_OK) return rc;
 	BatchArgs A = make_args(ctx, c, dt, 1, cfg);
 	rc = use_side_stream(ctx, &A);
 	if (rc != B3G_OK) return rc;
@@ -642,9 +701,10 @@ extern "C" int b3g_batch_schedule(b3g_context* ctx, int32_t* out, uint32_t capac
 	if (!ctx || !out) return fail(B3G_ERROR_INVALID_ARGUMENT, "null argument");
 	if (!ctx->batch) return fail(B3G_ERROR_INVALID_ARGUMENT, "no batch has been stepped on this context");
 	BatchCache* c = ctx->batch;
+	const BatchSchedule& S = c->sched[c->whole > 0 ? 1 : 0];
 	std::vector<int32_t> v = {c->cluster, c->threshold == (1 << 30) ? -1 : c->threshold, c->nbig, c->ctas,
-	                          c->tuned ? 1 : 0, (int32_t)c->tune_log.size(), c->lpt};
-	for (auto& t : c->tune_log)
+	                          S.tuned ? 1 : 0, (int32_t)S.tune_log.size(), c->lpt};
+	for (auto& t : S.tune_log)
 	{
 		v.push_back(t.first);
 		v.push_back((int32_t)(t.second * 1000.0));  // microseconds

@@ -281,7 +281,9 @@ B3G_API int b3g_step_batch_noalloc(b3g_context* ctx, b3g_body* const* bodies, ui
  * (-1 = none; the smallest body on more than one CTA), bodies stepped by clusters or parts of one,
  * CTAs of a whole-step launch, autotuned (0/1), number of timed candidates, queue order (0: largest first, 1:
  * longest estimated solve first), then per candidate (code = order * 1e8 + cluster * 1e6 + CTAs
- * per cluster of a second solve launch * 1e3 + row slices per CTA of a body's team, microseconds). */
+ * per cluster of a second solve launch * 1e3 + row slices per CTA of a body's team, microseconds; code =
+ * 1e9 + order * 1e8 + cluster * 1e6 + size threshold, at most 999999, for the whole-step launch of more
+ * than 16 Newton iterations, which has a schedule of its own). The schedule is that of the last step. */
 B3G_API int b3g_batch_schedule(b3g_context* ctx, int32_t* out, uint32_t capacity);
 
 /* Split assembly of the context's current batch (single Newton iteration, tetrahedra-only
