@@ -558,8 +558,8 @@ def ours(args, world, rank, local, pg):
         # the split assembly launches elements and rows twice each (two body groups)
         per_step = (3 if has_elements else 2) + (2 if b3g.batch_assembly_split(ctx)["elem_mid"] else 0)
         # the chosen schedule's second solve launch, on the SMs that the wide clusters leave free
-        best = min(sched["candidates_ms"], key=lambda c: c[3]) if sched["candidates_ms"] else None
-        if best and best[1] >= 1000:
+        best = min(sched["candidates_ms"], key=lambda c: c["ms"]) if sched["candidates_ms"] else {}
+        if best.get("second_launch_cluster"):
             per_step += 1
         launches = per_step * newton * args.steps
     line = {"metric": METRIC, "value": value, "unit": "vertex-steps/s", "n_gpus": world, "steps": args.steps,
@@ -577,8 +577,8 @@ def ours(args, world, rank, local, pg):
         line["schedule"] = {k: sched[k] for k in ("cluster", "threshold", "cluster_bodies", "ctas", "autotuned", "order")}
         line["schedule"]["candidates_timed"] = len(sched["candidates_ms"])
         # the chosen schedule per size bucket: the teams of the bucket's bodies (parts of a cluster)
-        best = min(sched["candidates_ms"], key=lambda c: c[3]) if sched["candidates_ms"] else None
-        per, helper = (best[1] % 1000, best[1] // 1000) if best else (0, 0)
+        best = min(sched["candidates_ms"], key=lambda c: c["ms"]) if sched["candidates_ms"] else {}
+        per, helper = best.get("slices_per_cta", 0), best.get("second_launch_cluster", 0)
         line["schedule"].update(slices_per_cta=per, second_launch_cluster=helper)
 
         def team(n):

@@ -529,14 +529,25 @@ def step_batch_noalloc(ctx: Context, bodies: Sequence[Body], dt: float, steps: i
     return [s.as_dict() for s in st[:len(bodies)]] if stats else None
 
 
+def _schedule_candidate(code: int, ms: float) -> dict:
+    """One of b3g_batch_schedule's candidates: teams by slices per CTA, and the cluster size of a second solve
+    launch (0: none), or, for the whole-step launch, teams by a size threshold (-1: single CTAs only)."""
+    out = {"cluster": code // 1000000 % 100, "order": "lpt" if code // 100000000 % 10 else "size", "ms": ms}
+    rest = code % 1000000
+    if code >= 1000000000:
+        out["threshold"] = rest if rest < 999999 else -1
+    else:
+        out.update(slices_per_cta=rest % 1000, second_launch_cluster=rest // 1000)
+    return out
+
+
 def batch_schedule(ctx: Context) -> dict:
-    """b3g_batch_schedule: the schedule of the context's current batch and the autotuner's timings."""
+    """b3g_batch_schedule: the schedule of the context's current batch and the autotuner's timings, fastest
+    candidate = the schedule in force (candidates_ms, empty when it was not tuned)."""
     buf = np.zeros(512, np.int32)
     _check(load_library().b3g_batch_schedule(ctx.handle, buf.ctypes.data_as(_ip), buf.size), "b3g_batch_schedule")
     n = int(buf[5])
-    cands = [((int(buf[7 + 2 * k]) // 1000000) % 100, int(buf[7 + 2 * k]) % 1000000,
-              "lpt" if int(buf[7 + 2 * k]) >= 100000000 else "size", buf[8 + 2 * k] / 1000.0)
-             for k in range(min(n, (buf.size - 7) // 2))]
+    cands = [_schedule_candidate(int(buf[7 + 2 * k]), buf[8 + 2 * k] / 1000.0) for k in range(min(n, (buf.size - 7) // 2))]
     return {"cluster": int(buf[0]), "threshold": int(buf[1]), "cluster_bodies": int(buf[2]),
             "ctas": int(buf[3]), "autotuned": bool(buf[4]), "order": "lpt" if int(buf[6]) else "size",
             "candidates_ms": cands}
