@@ -145,7 +145,8 @@ struct PhaseClock
 	{
 		if (!slot) return;
 		long long now = clock64();
-		if (threadIdx.x == 0) slot[phase] += (unsigned long long)(now - t);
+		// (atomic: a CTA of a second solve launch shares the slot of its block id)
+		if (threadIdx.x == 0) atomicAdd(slot + phase, (unsigned long long)(now - t));
 		t = now;
 	}
 };
