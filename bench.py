@@ -36,9 +36,8 @@ METRIC = "vertex-steps/s batched vs plain at resid 1e-5; p50/p99 step latency"
 DT = 1.0 / 60.0
 PCG_TOL = 1e-5
 PCG_MAX = 200
-# DRAM traffic / algorithmic bytes of the batch PCG launch, from the ncu capture of the
-# 128-body case (profiles/k_batch_solve_batch128.md): most of a body's matrix and vectors stay in
-# shared memory and L2 between its iterations
+# DRAM traffic / algorithmic bytes of the batch PCG launch, measured by ncu on the 128-body case with a
+# forced schedule: most of a body's matrix and vectors stay in shared memory and L2 between its iterations
 PCG_TRAFFIC_RATIO = 0.25
 # steps of the CPU-baseline run and of the parity check, from the bodies' initial state
 PARITY_STEPS = 3
@@ -430,11 +429,13 @@ def ours(args, world, rank, local, pg):
         ach = pcg_b / (pcg_ms / 1e3) / 1e9
         roof.update({"achieved": ach, "frac": ach / peak, "kernel": "k_batch_solve launch (PCG + final update)",
                      "algorithmic_bytes_per_launch": pcg_b, "launch_ms": pcg_ms, "launches_timed": lt["steps"]})
-        # DRAM traffic of the PCG launch: ncu on the 128-body case (PCG_TRAFFIC_RATIO); traffic
-        # grows with the work, so the ratio scales it to this launch. The algorithmic bytes count
-        # every iteration's operands, so `achieved` can pass the HBM peak
+        # The algorithmic bytes count every iteration's operands, most of which come from shared memory
+        # and L2: `frac`, their rate over the HBM's, can pass 1, and what bounds the launch is the
+        # L2-to-SM network. Traffic: an estimate, the ratio of the 128-body capture (PCG_TRAFFIC_RATIO)
         if args.precision == "fp32":
+            roof["bound"] = "l2_to_sm"
             roof["traffic"] = PCG_TRAFFIC_RATIO * pcg_b
+            roof["traffic_source"] = "estimate: DRAM / algorithmic bytes of 128 bodies on a forced schedule"
         roof["assembly_launch"] = {"achieved": asm_b / (asm_ms / 1e3) / 1e9, "frac": asm_b / (asm_ms / 1e3) / 1e9 / peak,
                                    "algorithmic_bytes_per_launch": asm_b, "launch_ms": asm_ms}
         split = b3g.batch_assembly_split(ctx)

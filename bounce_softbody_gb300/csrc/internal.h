@@ -47,22 +47,18 @@ constexpr int kMaxTeamCtas = 16;
 constexpr int kTiers = 5;                    // team widths 16, 8, 4, 2, 1
 constexpr int kQueueCounters = 2 + kTiers;   // the team launch's two, one per tier of the solve launch
 
-// Device-resident solver scalars of one body; everything the PCG decides is taken here.
+// What a body's solves and steps report, on the device.
 struct Scalars
 {
 	double delta;      // r.s of the current residual
 	double delta0;     // r0.s0
-	double tol2;       // pcg_tolerance^2
 	double newton_err, newton_err0;
-	double newton_tol2;
 	int iter;          // PCG iteration of the current solve
-	int max_iter;
 	int pending;       // rows assembled, solve not finished: set by the assembly, cleared by the solve
 	int status;        // b3g_solve_status
 	int newton_iter;
 	int newton_done;
 	int min_it, max_it;
-	int refresh;       // refresh period
 	int fault;         // a bounded device wait expired (the step's results are not valid)
 	unsigned long long total_iters;  // PCG iterations of every step since creation
 	unsigned long long total_steps;
@@ -214,7 +210,7 @@ struct DevBody
 	void* pb;
 	void* r;
 	void* d;
-	void* d2;                   // second direction buffer (persistent kernel ping-pong)
+	void* d2;                   // the BF16 mode's outer direction, where its product gathers it
 	void* q;
 	void* s;
 	void* py;

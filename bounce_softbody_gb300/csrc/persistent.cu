@@ -211,7 +211,6 @@ cudaError_t op_batch(const BatchArgs& A, cudaStream_t st)
 	P.s_begin = 0;
 	P.rows_per_sm = 0;
 	// with the flat numbering each Newton iteration is an element launch, a row launch and a PCG launch
-	// (which knows from `flat` to sum delta0 itself)
 	P.flat = (P.newton <= kFlatNewton && A.elem_off && A.slice_off && A.nslices > 0) ? 1 : 0;
 	P.k = 0;
 	cudaError_t e = launch_iteration(A, P, st);

@@ -55,8 +55,7 @@ struct BatchParams
 	int refresh;
 	double newton_tol2;
 	unsigned long long* prof;  // optional: kPhases cycle counters per CTA
-	// flat: a Newton iteration's elements and rows ran in the flat launches (their numbering below);
-	// the PCG launch then starts by summing delta0 = r.s itself
+	// flat: a Newton iteration's elements and rows run in the flat launches (their numbering below)
 	int flat;
 	const unsigned* elem_off;
 	const unsigned* slice_off;
@@ -151,48 +150,32 @@ struct PhaseClock
 	}
 };
 
-// PCG update of two rows (slices sl and sl + stride of one warp) with every load issued before
-// the first store: x += alpha d and, unless this is a refresh iteration, r -= alpha q,
-// s = M^-1 r. Returns the rows' r.s.
+// PCG update of row i: x += alpha d and, unless this is a refresh iteration, r -= alpha q, s = M^-1 r.
+// Returns the row's r.s.
 template <class TV, class LD>
-__device__ __forceinline__ double update_two(const DevBody& B, TV* __restrict__ py, const TV* __restrict__ d,
-                                             TV* __restrict__ r, const TV* __restrict__ q, TV* __restrict__ s,
-                                             int i0, int i1, bool ok1, TV alpha, bool refresh)
+__device__ __forceinline__ double update_row(const DevBody& B, TV* __restrict__ py, const TV* __restrict__ d,
+                                             TV* __restrict__ r, const TV* __restrict__ q, TV* __restrict__ s, int i,
+                                             TV alpha, bool refresh)
 {
-	const int ii[2] = {i0, i1};
-	const bool ok[2] = {true, ok1};
-	TV x[2][3], dd[2][3], rr[2][3], qq[2][3];
-#pragma unroll
-	for (int u = 0; u < 2; ++u)
-		if (ok[u])
-		{
-			vld<TV, LD>(py, ii[u], x[u]);
-			vld<TV, LD>(d, ii[u], dd[u]);
-			if (!refresh)
-			{
-				vld<TV, LD>(r, ii[u], rr[u]);
-				vld<TV, LD>(q, ii[u], qq[u]);
-			}
-		}
-	double part = 0.0;
-#pragma unroll
-	for (int u = 0; u < 2; ++u)
+	TV x[3], dd[3], rr[3], qq[3];
+	vld<TV, LD>(py, i, x);
+	vld<TV, LD>(d, i, dd);
+	if (!refresh)
 	{
-		if (!ok[u]) continue;
-		TV nx[3];
-#pragma unroll
-		for (int c = 0; c < 3; ++c) nx[c] = x[u][c] + alpha * dd[u][c];
-		vst(py, ii[u], nx);
-		if (refresh) continue;
-		TV nr[3], ss[3];
-#pragma unroll
-		for (int c = 0; c < 3; ++c) nr[c] = rr[u][c] - alpha * qq[u][c];
-		precond_row<TV, LD>(B, ii[u], nr, ss);
-		vst(r, ii[u], nr);
-		vst(s, ii[u], ss);
-		part += dot3<TV>(nr, ss);
+		vld<TV, LD>(r, i, rr);
+		vld<TV, LD>(q, i, qq);
 	}
-	return part;
+#pragma unroll
+	for (int c = 0; c < 3; ++c) x[c] += alpha * dd[c];
+	vst(py, i, x);
+	if (refresh) return 0.0;
+	TV ss[3];
+#pragma unroll
+	for (int c = 0; c < 3; ++c) rr[c] -= alpha * qq[c];
+	precond_row<TV, LD>(B, i, rr, ss);
+	vst(r, i, rr);
+	vst(s, i, ss);
+	return dot3<TV>(rr, ss);
 }
 
 // r = pb - A x, s = M^-1 r for the rows of one warp's slices (init / refresh); optionally d = s
@@ -347,7 +330,7 @@ __device__ SolveOut team_pcg(Team<CL>& T, const DevBody& B, const BatchParams& P
 		{
 			const int i0 = sl * kSlice + lane;
 			if (i0 >= B.n) continue;
-			part += update_two<TV, LD>(B, py, d, r, q, s, i0, i0, false, alpha, refresh);
+			part += update_row<TV, LD>(B, py, d, r, q, s, i0, alpha, refresh);
 		}
 		if (refresh)
 		{
@@ -515,9 +498,8 @@ __device__ void team_step(Team<CL>& T, const DevBody& B, const BatchParams& P, b
 }
 
 // Single-Newton step split in two launches so that each part runs with its own register budget
-// (the element and assembly code needs 128 registers a thread, the PCG far fewer, and more warps
-// per SM hide more of its memory latency). Part 1: elements and assembly; the PCG's delta0 goes
-// to the body's scalars.
+// (one CTA per SM for the solve, several for the assembly). Part 1: elements and assembly; k_batch_solve
+// does the rest.
 template <int CL, class TA, class TV>
 __device__ void team_step_assemble(Team<CL>& T, const DevBody& B, const BatchParams& P, bool bf16)
 {
@@ -525,8 +507,7 @@ __device__ void team_step_assemble(Team<CL>& T, const DevBody& B, const BatchPar
 	PhaseClock pc;
 	pc.start(P.prof);
 	if (T.tid() == 0) solve_pending(B, true);
-	const double delta0 = team_assemble<CL, TA, TV, LD>(T, B, P, bf16, 0, pc);
-	if (T.tid() == 0) B.sc->delta0 = delta0;
+	team_assemble<CL, TA, TV, LD>(T, B, P, bf16, 0, pc);
 }
 
 __device__ void load_body(DevBody* dst, const DevBody* src)
