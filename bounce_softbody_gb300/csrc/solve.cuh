@@ -10,18 +10,18 @@
 // runs while the second sum is on its way.
 //
 // Team sums. Every CTA stores its partial in its slot as two words, mantissa and exponent (Fixed), each
-// with two bits of the sum's number; one warp of every CTA polls all slots and adds them
-// up, so every thread holds the same bits and takes the same decisions. No fence and no atomic is on
-// that path. Above 16 CTAs the slots exist 16 times, a replica for every 16th CTA: with one copy
-// the pollers' traffic on the same lines costs 0.4 / 1.4 / 3.8 us a sum for 4 / 32 / 152 CTAs, with
-// sixteen 0.9 / 0.95 / 1.6. Two slot arrays alternate: a CTA can only overwrite its slot of sum e
-// with that of sum e + 2 after every CTA has arrived at sum e + 1, and so has read sum e. The same
-// holds for s, rewritten only after the sum that follows the sweep which gathers it.
+// with two bits of the sum's number; one warp of every CTA polls all slots and adds them up, so every
+// thread holds the same bits and takes the same decisions. No fence and no atomic is on that path. Above
+// 16 CTAs the slots exist 16 times, a replica for every 16th CTA: with one copy the pollers' traffic on
+// the same lines costs 0.4 / 1.4 / 3.8 us a sum for 4 / 32 / 152 CTAs, with sixteen 0.9 / 0.95 / 1.6
+// (slots of one word). Two slot arrays alternate: a CTA can only overwrite its slot of sum e with that
+// of sum e + 2 after every CTA has arrived at sum e + 1, and so has read sum e. The same holds for s,
+// rewritten only after the sum that follows the sweep which gathers it.
 // s itself needs no barrier in the FP32 and BF16 modes on small bodies: its fourth component carries the
 // number of its version, a vertex's 16 bytes are written and read as one access at GPU scope, and a
 // gather that meets an older version reads again. What does not fit one access (FP64 vectors, x of a
-// refresh), and the s that a large body gathers through the L1, is published by a fence of the CTA's
-// first warp and a flag behind it that the team polls with the sum's slots: the fence alone costs 900
+// refresh), and the s that a large body gathers through the L1, is published by a fence of one of the
+// CTA's warps and a flag behind it that the team polls with the sum's slots: the fence alone costs 900
 // clocks, most of them beside the sum and the update of x.
 // All polls are bounded. A wait that runs out is final for its CTA: it sets Scalars::fault, posts no
 // further partial and leaves the launch, so that its teammates' next wait runs out too. What a team
@@ -1305,7 +1305,8 @@ __global__ void __launch_bounds__(256, 1) k_solve_cluster(DevBody B, SolveArgs P
 // float-float x, preconditioned by a fixed number of Jacobi-PCG iterations with the BF16 blocks
 // from z = 0. Per outer iteration: z = P(r), p = z - (z.q_prev / p_prev.q_prev) p_prev, q = A p,
 // alpha = p.r / p.q, x += alpha p, r -= alpha q or, when a refresh is due, r = b - A x. The BF16
-// blocks, read most often, are what is kept in shared memory; the FP32 blocks stream.
+// blocks, read most often, are what is kept in shared memory; the FP32 blocks stream. With 256 threads
+// (255 registers) it spills 196 bytes.
 template <bool FILTER, int THREADS>
 __global__ void __launch_bounds__(THREADS, 1) k_solve_fcg(DevBody B, FcgVecs W, SolveArgs P, int inner)
 {
